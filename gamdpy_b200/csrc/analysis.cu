@@ -436,6 +436,7 @@ __global__ void k_cells_scatter(const float4 *pos, const int *pcell, const int *
 constexpr int SQ_TILE = 32;      // particles per shared-memory tile
 constexpr int SQ_THREADS = 256;  // q-vectors per block
 constexpr int SQ_CHUNK = 8192;   // particles per block (grid y)
+constexpr int SQ_RUN_THREADS = 640;  // most items per block (k_sq_runs): 20 warps at 96 registers
 
 struct SqArgs {
     const float4 *pos;
@@ -546,6 +547,139 @@ __global__ void __launch_bounds__(SQ_THREADS) k_sq(SqArgs a) {
             atomicAdd(&a.acc[2 * q + 1], si[k]);
         }
     }
+}
+
+// Runs of q-vectors: an item is one pair (a, b) of components along two of the
+// axes and SQ_Z consecutive components along the third (the run axis).  A
+// thread owns an item: per particle it multiplies e_a(a) e_b(b) and adds its
+// products with the run's SQ_Z factors, so a term costs two packed
+// multiply-adds and 10 bytes of shared memory, against two complex products
+// and 24 bytes in k_sq.  float32 within a tile of SQ_TILE particles, float64
+// across tiles, as k_sq.  What bounds it is the issue of those multiply-adds
+// and of the 6 shared loads a run, then the latency of a particle's loads at
+// 20 warps.  Measured on B200 with 1 000 188 particles and 3778 q-vectors in
+// an octant: a call 4.04 ms with k_sq, 1.51 here, 1.34 of it this kernel; with
+// one table and two barriers a tile 1.38, with two items a thread (320
+// threads) 1.57 to 1.85, with two blocks an SM at 48 registers 1.59.
+constexpr int SQ_Z = 8;
+struct SqRunArgs {
+    const float4 *pos;
+    const int *orig;
+    const float *ff;  // user order, may be null
+    int n, nitems;
+    int chunk;        // particles per block, a multiple of SQ_TILE
+    const int4 *items;  // table columns of a, b and of the run's first entry (even); w unused
+    int axis[3];        // coordinate of each third of the table: a, b, run axis
+    int kmin[3], klen[3];  // klen[0] + klen[1] and klen[2] even (16-byte loads of the run)
+    float invL[3];         // 1 / box length, by third of the table
+    double *acc;  // [2 SQ_Z][nitems]: re and im of entry z at rows 2 z, 2 z + 1
+};
+
+template <bool FF>
+__global__ void __launch_bounds__(SQ_RUN_THREADS, 1) k_sq_runs(SqRunArgs a) {
+    extern __shared__ __align__(16) float2 rtab[];  // two tables [SQ_TILE][klen0 + klen1 + klen2]
+    __shared__ float wsh[3][SQ_TILE];
+    __shared__ float xsh[2][3][SQ_TILE];  // coordinate / box length along a, b and the run axis
+    const int k0 = a.klen[0], k01 = a.klen[0] + a.klen[1];
+    const int row = k01 + a.klen[2];
+    const int item = blockIdx.x * blockDim.x + threadIdx.x;
+    const int4 it = a.items[min(item, a.nitems - 1)];  // threads past the end repeat the last item, unstored
+    const int ca = it.x, cb = it.y, cz = it.z;
+    // the thread's float64 sums stay in shared memory (touched once per tile):
+    // their 32 registers cost a third of the warps an SM holds
+    double *sum = reinterpret_cast<double *>(rtab + 2 * SQ_TILE * row) + threadIdx.x;
+#pragma unroll
+    for (int j = 0; j < 2 * SQ_Z; j++) sum[j * blockDim.x] = 0.0;
+    const int dpl = blockDim.x / row, dcol = blockDim.x % row;
+    const int pl0 = threadIdx.x / row, col0 = threadIdx.x % row;
+    const int p_begin = blockIdx.y * a.chunk;
+    const int p_end = min(a.n, p_begin + a.chunk);
+    const int tiles = (p_end - p_begin + SQ_TILE - 1) / SQ_TILE;
+    // particle of tile t that this thread (one of the first SQ_TILE) stages; a
+    // place past the end repeats the last particle and is not summed
+    auto fetch = [&](int t, float4 &p, float &w) {
+        const int k = min(p_begin + t * SQ_TILE + (int)threadIdx.x, p_end - 1);
+        p = a.pos[k];
+        if (FF) w = a.ff[a.orig[k]];
+    };
+    auto stage = [&](int t, float4 p, float w) {
+#pragma unroll
+        for (int d = 0; d < 3; d++)
+            xsh[t & 1][d][threadIdx.x] = (a.axis[d] == 0 ? p.x : (a.axis[d] == 1 ? p.y : p.z)) * a.invL[d];
+        if (FF) wsh[t % 3][threadIdx.x] = w;
+    };
+    auto tabulate = [&](int t) {
+        float2 *tab = rtab + (t & 1) * SQ_TILE * row;
+        for (int pl = pl0, col = col0; pl < SQ_TILE;) {
+            const int d = (col >= k0) + (col >= k01);
+            const int kk = col + (d == 0 ? a.kmin[0] : (d == 1 ? a.kmin[1] - k0 : a.kmin[2] - k01));
+            float sn, cs;
+            sincospif(2.0f * (float)kk * xsh[t & 1][d][pl], &sn, &cs);
+            tab[pl * row + col] = make_float2(cs, sn);
+            col += dcol;
+            pl += dpl;
+            if (col >= row) {
+                col -= row;
+                pl++;
+            }
+        }
+    };
+    const bool loader = threadIdx.x < SQ_TILE;
+    float4 p = make_float4(0.f, 0.f, 0.f, 0.f);
+    float w = 0.f;
+    for (int t = 0; t < 2; t++)
+        if (loader) {
+            fetch(t, p, w);
+            stage(t, p, w);
+        }
+    __syncthreads();
+    tabulate(0);
+    __syncthreads();
+    // one barrier a tile: the next tile's table is made beside this tile's
+    // sums, from the positions loaded a tile before
+    for (int t = 0; t < tiles; t++) {
+        if (loader) fetch(t + 2, p, w);
+        tabulate(t + 1);
+        const int np = min(SQ_TILE, p_end - p_begin - t * SQ_TILE);
+        const float2 *tab = rtab + (t & 1) * SQ_TILE * row;
+        // sums of x_re (z_re, z_im) and x_im (z_re, z_im), x = e_a e_b
+        f32x2 pz[SQ_Z], qz[SQ_Z];
+#pragma unroll
+        for (int z = 0; z < SQ_Z; z++) pz[z] = qz[z] = 0ull;
+#pragma unroll 2
+        for (int pl = 0; pl < np; pl++) {
+            const float2 *e = tab + pl * row;
+            const float2 ea = e[ca], eb = e[cb];
+            float re = __fmaf_rn(ea.x, eb.x, -__fmul_rn(ea.y, eb.y));
+            float im = __fmaf_rn(ea.x, eb.y, __fmul_rn(ea.y, eb.x));
+            if (FF) {
+                re *= wsh[t % 3][pl];
+                im *= wsh[t % 3][pl];
+            }
+            const f32x2 xr = pack2(re, re), xi = pack2(im, im);
+            const ulonglong2 *zr = reinterpret_cast<const ulonglong2 *>(e + cz);
+#pragma unroll
+            for (int z = 0; z < SQ_Z; z += 2) {
+                const ulonglong2 g = zr[z / 2];
+                pz[z] = fma2(xr, g.x, pz[z]);
+                qz[z] = fma2(xi, g.x, qz[z]);
+                pz[z + 1] = fma2(xr, g.y, pz[z + 1]);
+                qz[z + 1] = fma2(xi, g.y, qz[z + 1]);
+            }
+        }
+#pragma unroll
+        for (int z = 0; z < SQ_Z; z++) {
+            float pr, pi, qr, qi;
+            unpack2(pz[z], pr, pi);
+            unpack2(qz[z], qr, qi);
+            sum[(2 * z) * blockDim.x] += pr - qi;
+            sum[(2 * z + 1) * blockDim.x] += pi + qr;
+        }
+        if (loader) stage(t + 2, p, w);  // (the table of tile t, the last to use this place, is made)
+        __syncthreads();
+    }
+    if (item < a.nitems)
+        for (int j = 0; j < 2 * SQ_Z; j++) atomicAdd(&a.acc[(size_t)j * a.nitems + item], sum[j * blockDim.x]);
 }
 
 template <int QPT>
@@ -724,6 +858,118 @@ static int rdf_device(gdb_sim *h, cudaStream_t st, const float4 *pos, int n, con
     return GDB_OK;
 }
 
+// Items of k_sq_runs for a set of q-vectors, along the run axis that needs the
+// fewest; entry[q] is the q-vector's place in the accumulators, z * nitems +
+// item.
+struct SqRuns {
+    int axis[3], kmin[3], klen[3];
+    std::vector<int4> items;
+    std::vector<int> entry;
+};
+static bool sq_runs_plan(int nq, const int32_t *nvec, const int kmin[3], const int klen[3], SqRuns &best) {
+    // the plan marks the q-vectors on their bounding grid: sets much sparser
+    // than that (or wide) stay with k_sq
+    const double cells = (double)klen[0] * klen[1] * klen[2];
+    if (cells > 64.0 * nq + 65536.0) return false;
+    std::vector<int> at;
+    for (int run = 2; run >= 0; run--) {
+        // (runs along z that are half full are good enough)
+        if (!best.items.empty() && best.items.size() * SQ_Z <= 2 * (size_t)nq) break;
+        SqRuns s;
+        s.axis[0] = run == 0 ? 1 : 0;
+        s.axis[1] = run == 2 ? 1 : 2;
+        s.axis[2] = run;
+        for (int d = 0; d < 3; d++) {
+            s.kmin[d] = kmin[s.axis[d]];
+            s.klen[d] = klen[s.axis[d]];
+        }
+        const int na = s.klen[0], nb = s.klen[1], nz = s.klen[2];
+        at.assign((size_t)na * nb * nz, -1);
+        for (int q = 0; q < nq; q++) {
+            const int32_t *v = nvec + 3 * (size_t)q;
+            at[((size_t)(v[s.axis[0]] - s.kmin[0]) * nb + (v[s.axis[1]] - s.kmin[1])) * nz + (v[run] - s.kmin[2])] = 0;
+        }
+        // a run starts at the even component at or below its first one
+        for (int x = 0; x < na; x++)
+            for (int y = 0; y < nb; y++) {
+                int *col = &at[((size_t)x * nb + y) * nz];
+                for (int z = 0; z < nz;) {
+                    if (col[z] < 0) {
+                        z++;
+                        continue;
+                    }
+                    const int z0 = z & ~1;
+                    for (z = z0; z < std::min(nz, z0 + SQ_Z); z++)
+                        if (col[z] >= 0) col[z] = (int)s.items.size() * SQ_Z + (z - z0);
+                    s.items.push_back(make_int4(x, y, z0, 0));
+                }
+            }
+        if (!best.items.empty() && best.items.size() <= s.items.size()) continue;
+        // the lanes of a warp share a run (broadcast loads): items in the
+        // order of their run's start
+        std::vector<int> order(s.items.size()), place(s.items.size());
+        for (size_t k = 0; k < order.size(); k++) order[k] = (int)k;
+        std::stable_sort(order.begin(), order.end(), [&](int p, int q) { return s.items[p].z < s.items[q].z; });
+        std::vector<int4> sorted(s.items.size());
+        for (size_t k = 0; k < order.size(); k++) {
+            place[order[k]] = (int)k;
+            sorted[k] = s.items[order[k]];
+        }
+        s.items.swap(sorted);
+        s.entry.resize(nq);
+        const int nitems = (int)s.items.size();
+        for (int q = 0; q < nq; q++) {
+            const int32_t *v = nvec + 3 * (size_t)q;
+            const int e =
+                at[((size_t)(v[s.axis[0]] - s.kmin[0]) * nb + (v[s.axis[1]] - s.kmin[1])) * nz + (v[run] - s.kmin[2])];
+            s.entry[q] = (e % SQ_Z) * nitems + place[e / SQ_Z];
+        }
+        best = std::move(s);
+    }
+    // table columns: the run's section starts at an even column and holds
+    // whole runs, so that their 16-byte loads are aligned and inside a row
+    best.klen[1] += (best.klen[0] + best.klen[1]) & 1;
+    int zlen = 0;
+    for (const int4 &i : best.items) zlen = std::max(zlen, i.z + SQ_Z);
+    best.klen[2] = std::max(best.klen[2] + (best.klen[2] & 1), zlen);
+    for (int4 &i : best.items) {
+        i.y += best.klen[0];
+        i.z += best.klen[0] + best.klen[1];
+    }
+    return true;
+}
+
+// Shared memory of k_sq_runs: two tables and the threads' float64 sums.
+static size_t sq_runs_smem(const int klen[3], int threads) {
+    return (size_t)2 * SQ_TILE * (klen[0] + klen[1] + klen[2]) * sizeof(float2) +
+           (size_t)threads * 2 * SQ_Z * sizeof(double);
+}
+static cudaError_t launch_sq_runs(cudaStream_t st, SqRunArgs &r, int n) {
+    const void *fn = r.ff ? (const void *)k_sq_runs<true> : (const void *)k_sq_runs<false>;
+    // as few blocks along the items as SQ_RUN_THREADS allows (every one of
+    // them tabulates the particles again), of equal size
+    const int nbx = (r.nitems + SQ_RUN_THREADS - 1) / SQ_RUN_THREADS;
+    // (at least SQ_TILE threads: they stage the positions)
+    const int threads = ((r.nitems + nbx - 1) / nbx + 31) / 32 * 32;
+    const size_t smem = sq_runs_smem(r.klen, threads);
+    int dev = 0, sms = 0, per_sm = 0;
+    cudaError_t e;
+    if ((e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) ||
+        (e = cudaGetDevice(&dev)) || (e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) ||
+        (e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, smem)))
+        return e;
+    // four waves of blocks (an uneven last wave is an eighth of the time at
+    // most), of at least four tiles
+    const int slots = std::max(1, sms * std::max(per_sm, 1) * 4 / nbx);
+    r.chunk = std::max(4 * SQ_TILE, ((n + slots - 1) / slots + SQ_TILE - 1) / SQ_TILE * SQ_TILE);
+    const dim3 grid(nbx, (n + r.chunk - 1) / r.chunk);
+    if (r.ff)
+        k_sq_runs<true><<<grid, threads, smem, st>>>(r);
+    else
+        k_sq_runs<false><<<grid, threads, smem, st>>>(r);
+    return cudaGetLastError();
+}
+
 static int sq_device(gdb_sim *h, cudaStream_t st, const float4 *pos, const int *orig, int n, const float *ff_host,
                      const float *box, int nq, const int32_t *nvec_host, double *re, double *im) {
     if (nq < 1) return GDB_OK;
@@ -745,14 +991,22 @@ static int sq_device(gdb_sim *h, cudaStream_t st, const float4 *pos, const int *
     const int row = a.klen[0] + a.klen[1] + a.klen[2];
     const size_t smem = (size_t)SQ_TILE * row * sizeof(float2);
     if (smem > 200 * 1024) return aset(h, GDB_ERR_ARG, "sq: n_vectors span too wide");
-    int *dn = nullptr;
+    SqRuns plan;
+    bool runs = sq_runs_plan(nq, nvec_host, a.kmin, a.klen, plan);
+    // per particle a run issues 30 instructions and a q-vector of k_sq 23:
+    // runs where they hold at least two q-vectors on average
+    if (runs) runs = 2 * plan.items.size() <= (size_t)nq && sq_runs_smem(plan.klen, SQ_RUN_THREADS) <= 224 * 1024;
+    const size_t nacc = runs ? plan.items.size() * SQ_Z * 2 : (size_t)nq * 2;
+    int *dn = nullptr;  // n-vectors, or the runs' items
     float *dff = nullptr;
     double *acc = nullptr;
+    const size_t dn_bytes = runs ? plan.items.size() * sizeof(int4) : (size_t)nq * 3 * sizeof(int);
     ACK(timing_begin(h, st));
-    ACK(pool_alloc(&dn, (size_t)nq * 3 * sizeof(int), st));
-    ACK(pool_alloc(&acc, (size_t)nq * 2 * sizeof(double), st));
-    ACK(cudaMemcpyAsync(dn, nvec_host, (size_t)nq * 3 * sizeof(int), cudaMemcpyHostToDevice, st));
-    ACK(cudaMemsetAsync(acc, 0, (size_t)nq * 2 * sizeof(double), st));
+    ACK(pool_alloc(&dn, dn_bytes, st));
+    ACK(pool_alloc(&acc, nacc * sizeof(double), st));
+    ACK(cudaMemcpyAsync(dn, runs ? (const void *)plan.items.data() : (const void *)nvec_host, dn_bytes,
+                        cudaMemcpyHostToDevice, st));
+    ACK(cudaMemsetAsync(acc, 0, nacc * sizeof(double), st));
     double nf = 0.0;
     if (ff_host) {
         ACK(pool_alloc(&dff, (size_t)n * sizeof(float), st));
@@ -764,27 +1018,47 @@ static int sq_device(gdb_sim *h, cudaStream_t st, const float4 *pos, const int *
     a.nvec = dn;
     a.ff = dff;
     a.acc = acc;
-    // q-vectors per thread: up to 4, as few blocks along q as that allows,
-    // spread evenly over them (2219 q: 3 blocks of 3 x 256)
-    const int nbx = (nq + 4 * SQ_THREADS - 1) / (4 * SQ_THREADS);
-    const int qpt = (nq + nbx * SQ_THREADS - 1) / (nbx * SQ_THREADS);
-    const dim3 grid(nbx, (n + SQ_CHUNK - 1) / SQ_CHUNK);
-    const void *fn = nullptr;
-    switch (qpt) {
-        case 1: fn = a.ff ? (const void *)k_sq<1, true> : (const void *)k_sq<1, false>; break;
-        case 2: fn = a.ff ? (const void *)k_sq<2, true> : (const void *)k_sq<2, false>; break;
-        case 3: fn = a.ff ? (const void *)k_sq<3, true> : (const void *)k_sq<3, false>; break;
-        default: fn = a.ff ? (const void *)k_sq<4, true> : (const void *)k_sq<4, false>; break;
+    SqRunArgs r;
+    if (runs) {
+        r.pos = pos;
+        r.orig = orig;
+        r.ff = dff;
+        r.n = n;
+        r.nitems = (int)plan.items.size();
+        r.items = (const int4 *)dn;
+        r.acc = acc;
+        for (int d = 0; d < 3; d++) {
+            r.axis[d] = plan.axis[d];
+            r.kmin[d] = plan.kmin[d];
+            r.klen[d] = plan.klen[d];
+            r.invL[d] = a.invL[plan.axis[d]];
+        }
     }
-    ACK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    switch (qpt) {
-        case 1: launch_sq<1>(grid, smem, st, a); break;
-        case 2: launch_sq<2>(grid, smem, st, a); break;
-        case 3: launch_sq<3>(grid, smem, st, a); break;
-        default: launch_sq<4>(grid, smem, st, a); break;
+    if (runs) {
+        ACK(launch_sq_runs(st, r, n));
+    } else {
+        // q-vectors per thread: up to 4, as few blocks along q as that allows,
+        // spread evenly over them (2219 q: 3 blocks of 3 x 256)
+        const int nbx = (nq + 4 * SQ_THREADS - 1) / (4 * SQ_THREADS);
+        const int qpt = (nq + nbx * SQ_THREADS - 1) / (nbx * SQ_THREADS);
+        const dim3 grid(nbx, (n + SQ_CHUNK - 1) / SQ_CHUNK);
+        const void *fn = nullptr;
+        switch (qpt) {
+            case 1: fn = a.ff ? (const void *)k_sq<1, true> : (const void *)k_sq<1, false>; break;
+            case 2: fn = a.ff ? (const void *)k_sq<2, true> : (const void *)k_sq<2, false>; break;
+            case 3: fn = a.ff ? (const void *)k_sq<3, true> : (const void *)k_sq<3, false>; break;
+            default: fn = a.ff ? (const void *)k_sq<4, true> : (const void *)k_sq<4, false>; break;
+        }
+        ACK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        switch (qpt) {
+            case 1: launch_sq<1>(grid, smem, st, a); break;
+            case 2: launch_sq<2>(grid, smem, st, a); break;
+            case 3: launch_sq<3>(grid, smem, st, a); break;
+            default: launch_sq<4>(grid, smem, st, a); break;
+        }
     }
     ACK(cudaGetLastError());
-    std::vector<double> tmp((size_t)nq * 2);
+    std::vector<double> tmp(nacc);
     ACK(timing_end(h, st));
     ACK(cudaMemcpyAsync(tmp.data(), acc, tmp.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
     ACK(cudaFreeAsync(dn, st));
@@ -794,8 +1068,11 @@ static int sq_device(gdb_sim *h, cudaStream_t st, const float4 *pos, const int *
     timing_store(h);
     const double norm = 1.0 / sqrt(nf);
     for (int q = 0; q < nq; q++) {
-        re[q] = tmp[2 * q] * norm;
-        im[q] = tmp[2 * q + 1] * norm;
+        // runs: entry z * nitems + item, its real part at row 2 z of tmp
+        const size_t nitems = plan.items.size();
+        const size_t e = runs ? (size_t)plan.entry[q] / nitems * 2 * nitems + (size_t)plan.entry[q] % nitems : 2 * (size_t)q;
+        re[q] = tmp[e] * norm;
+        im[q] = tmp[runs ? e + nitems : e + 1] * norm;
     }
     return GDB_OK;
 }

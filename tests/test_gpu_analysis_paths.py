@@ -1,0 +1,48 @@
+"""Routes of the analyses that depend on sizes: S(q) by runs of q-vectors or one by one."""
+import numpy as np
+import pytest
+
+from gamdpy_b200 import _lib
+
+pytestmark = pytest.mark.gpu
+
+
+def _octant(m):
+    n = np.stack(np.meshgrid(*[np.arange(m)] * 3, indexing="ij"), -1).reshape(-1, 3)[1:]
+    return n[(n * n).sum(1) < m * m]
+
+
+def _sets():
+    rng = np.random.default_rng(5)
+    line = np.zeros((40, 3), int)
+    for axis, name in enumerate("xyz"):
+        one = line.copy()
+        one[:, axis] = np.arange(-20, 20)
+        yield "line_" + name, one
+    yield "octant", _octant(9)
+    yield "octant_shuffled_twice", rng.permutation(np.concatenate([_octant(7), _octant(7)]))
+    yield "slab", np.stack(np.meshgrid(np.arange(-3, 4), [2], np.arange(5, 22), indexing="ij"), -1).reshape(-1, 3)
+    yield "one", np.array([[1, -2, 3]])
+    yield "sparse", rng.integers(-12, 13, size=(300, 3))
+    yield "wide", np.stack([np.arange(600), np.zeros(600, int), np.arange(600) % 2], 1)
+    yield "more_than_a_block", _octant(24)
+
+
+@pytest.mark.parametrize("weighted", [False, True])
+@pytest.mark.parametrize("n", [1, 33, 3001])
+@pytest.mark.parametrize("name", [k for k, _ in _sets()])
+def test_sq_sets_of_q_vectors(name, n, weighted):
+    """Runs along each axis, an odd start, duplicates, single and scattered q-vectors, a particle number that
+    leaves a partial tile; against float64.  Bound: the phase of a component k is exact to 2 pi |k| 2^-24 in
+    float32 (|k| <= 600 here: 2.3e-4 at most, 1e-5 at the usual 24), and independent between particles."""
+    nv = dict(_sets())[name]
+    rng = np.random.default_rng(n)
+    box = np.array([9.0, 11.0, 14.0], np.float32)
+    r = ((rng.random((n, 3)) - 0.5) * box).astype(np.float32)
+    ff = rng.uniform(0.5, 2.0, n).astype(np.float32) if weighted else None
+    got = _lib.sq_compute(r, box, nv, ff)
+    w = np.ones(n) if ff is None else ff.astype(np.float64)
+    phase = 2 * np.pi * (r.astype(np.float64) / box.astype(np.float64)) @ nv.T.astype(np.float64)
+    ref = (w[:, None] * np.exp(1j * phase)).sum(0) / np.sqrt(w.sum())
+    k = max(24, np.abs(nv).max())
+    assert np.abs(got - ref).max() < 2 * np.pi * k * 2.0 ** -24 * 3 * max(1.0, np.abs(ref).max())
