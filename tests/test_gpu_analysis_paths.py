@@ -1,4 +1,5 @@
-"""Routes of the analyses that depend on sizes: S(q) by runs of q-vectors or one by one."""
+"""Routes of the analyses that depend on sizes: S(q) by runs of q-vectors or one by one, the RDF's rows of
+cells."""
 import numpy as np
 import pytest
 
@@ -46,3 +47,33 @@ def test_sq_sets_of_q_vectors(name, n, weighted):
     ref = (w[:, None] * np.exp(1j * phase)).sum(0) / np.sqrt(w.sum())
     k = max(24, np.abs(nv).max())
     assert np.abs(got - ref).max() < 2 * np.pi * k * 2.0 ** -24 * 3 * max(1.0, np.abs(ref).max())
+
+
+@pytest.mark.parametrize("bins,nt", [(1, 1), (12289, 1), (64, 3)])
+@pytest.mark.parametrize("n", [31, 32, 1000, 5000])
+def test_rdf_rows_of_uneven_occupation(oracle, n, bins, nt):
+    """Units of 32 slots that span many cells, one dense cell, empty rows; shared and global histograms."""
+    rng = np.random.default_rng(n + bins)
+    L = np.array([20.0, 21.0, 19.5], np.float32)
+    r = (rng.random((n, 3)) - 0.5) * L
+    r[: n // 3] = r[0] + rng.normal(0, 0.4, (n // 3, 3))  # a cluster
+    r[n // 3 : n // 2, 1:] = r[n // 3, 1:]  # a line along x
+    r = (r - L * np.round(r / L)).astype(np.float32)
+    pt = rng.integers(0, nt, n).astype(np.int32)
+    pt[:nt] = np.arange(nt)
+    got = _lib.rdf_compute(r, pt, L, nt, bins, r_max=3.1)
+    assert np.array_equal(got, oracle.rdf(r, pt, L, bins, fma=1, r_max=3.1)) and got.sum() > 0
+
+
+@pytest.mark.parametrize("axis", [0, 1, 2])
+def test_rdf_coordinates_on_the_faces(oracle, axis):
+    """Particles on the faces of the box and one float away from them, in a grid that takes plain differences."""
+    rng = np.random.default_rng(axis)
+    L = np.array([22.0, 23.0, 24.0], np.float32)
+    r = ((rng.random((4000, 3)) - 0.5) * L).astype(np.float32)
+    h = np.float32(0.5) * L[axis]
+    faces = np.array([h, -h, np.nextafter(h, np.float32(0)), np.nextafter(-h, np.float32(0))], np.float32)
+    r[:400, axis] = np.tile(faces, 100)
+    pt = rng.integers(0, 2, 4000).astype(np.int32)
+    got = _lib.rdf_compute(r, pt, L, 2, 100, r_max=3.1)
+    assert np.array_equal(got, oracle.rdf(r, pt, L, 100, fma=1, r_max=3.1)) and got.sum() > 0
