@@ -5,7 +5,7 @@
 // Forward (float32 state, float64 reductions), as integrators/NVE.py:78-97
 // with the shifted-force LJ of LJ_12_6_sigma_epsilon.py:26-36 and
 // apply_shifted_force_cutoff.py:30-37 (s -= s(rc), u += s(rc) rc (r - rc) - u(rc)):
-//   f_n     = F(r_n)                       pair sum over all j (N^2, on the fly)
+//   f_n     = F(r_n)                       pair sum over the list
 //   v_{n+1} = v_n + f_n dt / m
 //   r_{n+1} = r_n + v_{n+1} dt             (periodic wrap; derivative identity)
 //   U_n, W_n from r_n; K_n = sum m ((v_n + v_{n+1}) / 2)^2 / 2
@@ -19,25 +19,33 @@
 //   V   <- Vt + gK dK_n/dv_n
 //   dL/dtheta += (dt / m) (df/dtheta)^T Vt + gU dU_n/dtheta + gW dW_n/dtheta
 // J^T Vt is the Hessian-vector product of the pair potential: for each pair
-// (s I + s'/r d d^T)(Vt_i - Vt_j).  The sweep runs segment by segment: the
-// forward keeps checkpoints of (r, v) every `checkpoint_every` steps and the
-// backward recomputes each segment's states from its checkpoint with the
-// same kernels (bit-identical) before sweeping it in reverse, in float64.
+// (s I + s'/r d d^T)(Vt_i - Vt_j).  The states the sweep needs are all kept
+// while they fit ADJ_KEEP_BYTES; beyond that the forward keeps checkpoints of
+// (r, v) every `checkpoint_every` steps and the backward recomputes each
+// segment's states from its checkpoint with the same kernel (bit-identical)
+// before sweeping it in reverse, in float64.
 //
-// Pairs come from a neighbour list (all j within the largest cut or the RDF
-// kernel's reach plus a skin of 0.5, built N^2, rebuilt when a particle moves
-// more than half the skin); 32 lanes per particle, lane L taking its column
-// of the list, the neighbours j = L (mod 32) in ascending order.  Every per-lane sum
-// is then the same as a loop over all j (the NbList2 pair set), whatever the
-// list holds beyond the cutoff: results do not depend on when the list was
-// built, so recomputed segments are bit-identical to the forward.  Every sum
-// has a fixed order, so runs are reproducible.  Sized for the small systems
-// this is meant for (N of a few thousand; the build is N^2).
+// Forward and sweep are one cooperative kernel each, one warp per particle
+// and one grid barrier per step; every sum over the steps stays with its warp
+// until the kernel ends.
+//
+// Pairs come from a neighbour list (all j within the pair's cut plus a skin of
+// 0.5, and, apart, the other type-0 pairs within the RDF kernel's reach plus
+// the skin; built N^2 by the warp that uses it, so a rebuild costs no barrier;
+// rebuilt when a particle moves more than half the skin); 32 lanes per
+// particle, lane L taking its column of the list, the neighbours j = L (mod
+// 32) in ascending order.  Every per-lane sum of the forward is then the same
+// as a loop over all j (the NbList2 pair set), whatever the list holds beyond
+// the cutoff: results do not depend on when the list was built, so recomputed
+// segments are bit-identical to the forward.  Every sum has a fixed order, so
+// runs are reproducible.  Sized for the small systems this is meant for (N of
+// a few thousand; the build is N^2).
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stdarg.h>
 #include <stdint.h>
 #include <stdio.h>
+#include <stdlib.h>
 #include <string.h>
 
 #include <algorithm>
@@ -50,9 +58,9 @@ namespace {
 
 constexpr int ADJ_MAXT = 4;     // particle types
 constexpr int ADJ_MAXB = 128;   // RDF bins
-constexpr int ADJ_LANES = 32;   // lanes per particle
-constexpr int ADJ_BLOCK = 256;  // 8 particles per block
-constexpr int ADJ_PPB = ADJ_BLOCK / ADJ_LANES;
+constexpr int ADJ_LANES = 32;   // lanes per particle: a warp
+constexpr int ADJ_WARPS = 28;   // most warps per block: one block per SM, 4144 particles in flight on 148 SMs
+constexpr size_t ADJ_KEEP_BYTES = (size_t)1 << 30;  // states kept instead of checkpoints up to this (GDB_ADJ_KEEP_BYTES)
 constexpr int ADJ_NTH = 2 * ADJ_MAXT * ADJ_MAXT;  // d/dsigma, d/depsilon per ordered type pair
 constexpr double ADJ_FIX = 4294967296.0;          // fixed-point scale of the RDF kernel sums
 constexpr double ADJ_KW = 8.0;                    // kernel support in widths (exp(-32): smooth to 1e-14)
@@ -63,17 +71,26 @@ struct Tab32 {
 };
 // float64 parameters and cutoff values for the backward sweep
 struct Tab64 {
-    double sig, eps, cut, cut2;
+    double sig2, eps, ieps, eps_sig;  // sigma^2, epsilon, 1 / epsilon, epsilon / sigma
+    double cut;
     double s_c;    // s0(rc)
     double dsds_c; // d s0 / d sigma at rc
     double u_c;    // u0(rc)
     double duds_c; // d u0 / d sigma at rc
+    float cut2;    // the forward's cutoff test
+    float reach2;  // (cut + skin)^2: the list
 };
 
 struct Tables {
     int nt;
     Tab32 t32[ADJ_MAXT * ADJ_MAXT];
     Tab64 t64[ADJ_MAXT * ADJ_MAXT];
+};
+
+// Grid barrier words, zero at a launch.
+struct AdjBar {
+    unsigned cnt[3];  // arrivals, by barrier index mod 3
+    int abort;
 };
 
 struct AdjArgs {
@@ -84,22 +101,26 @@ struct AdjArgs {
     const float *mass;
     int nbins;
     float r_lo, dr, width;  // bin centres r_lo + (b + 1/2) dr
-    // neighbour list: all j within rl of i at the build; particle i's maxnb
-    // entries at nbl + i * maxnb as 32 columns (entry c of column L at
-    // c * 32 + L, the neighbours j = L (mod 32) ascending); nbc holds the 32
-    // column counts of each particle; rebuilt when a particle moves more than
-    // skin/2
-    const int *nbl, *nbc;
+    double step_ratio;      // exp(-dr^2 / width^2)
+    // neighbour list: particle i's maxnb entries at nbl + i * maxnb as 32
+    // columns of maxnb / 32 rows (row c of column L at c * 32 + L, the
+    // neighbours j = L (mod 32)).  From row 0 up, ascending: the pairs within
+    // cut_ab + skin at the build; from the last row down: the other type-0
+    // pairs within the RDF kernel's reach + skin.  nbc: each column's two
+    // counts, the second in the high half.  Rebuilt when a particle moves more
+    // than skin/2.
+    int *nbl, *nbc;
     int maxnb;
-    float rl2;      // (max cut or RDF reach + skin)^2
+    float far2;     // (RDF reach + skin)^2, 0 without RDF bins
     float move2;    // (skin / 2 - margin)^2
     float4 *rref;   // positions at the last build
-    int *flags;     // rebuild flags, by step parity
+    AdjBar *bar;
     unsigned *status;
 };
 
 constexpr float ADJ_SKIN = 0.5f;
 constexpr unsigned ADJ_STATUS_OVERFLOW = 1u;
+constexpr unsigned ADJ_STATUS_TIMEOUT = 2u;
 
 __device__ __forceinline__ float mic_rint(float d, float L, float iL) { return d - L * rintf(d * iL); }
 
@@ -110,343 +131,581 @@ __device__ __forceinline__ T wsum(T v) {
     return v;
 }
 
-// Forward step: forces at pos_in, integration into pos_out/vel_out, per-block
-// float64 partial sums of U, W, K; on sampled steps the A-A kernel sums into
-// gbins (fixed point, integer atomics: order-independent).
-__global__ void __launch_bounds__(ADJ_BLOCK) k_adj_step(AdjArgs a, Tables tab, const float4 *__restrict__ pos_in,
-                                                        const float4 *__restrict__ vel_in, float4 *pos_out,
-                                                        float4 *vel_out, double *partials, unsigned long long *gbins,
-                                                        int *flag_out) {
-    __shared__ Tab32 s_tab[ADJ_MAXT * ADJ_MAXT];
-    __shared__ double s_red[ADJ_PPB][3];
-    __shared__ unsigned long long s_bins[ADJ_MAXB];
-    const int nt = tab.nt;
-    for (int t = threadIdx.x; t < nt * nt; t += blockDim.x) s_tab[t] = tab.t32[t];
-    const bool rdf = gbins != nullptr;
-    if (rdf)
-        for (int b = threadIdx.x; b < a.nbins; b += blockDim.x) s_bins[b] = 0ull;
+// Barrier of the cooperative grid with a flag (a particle of some block has
+// moved beyond skin/2).  Arrivals count in the low 20 bits of one of three
+// words, flags in the high bits; a block leaves when the count reaches the
+// grid.  Block 0 then clears the word of barrier seq + 2: every block has left
+// barrier seq - 1, and block 0's next arrival orders the clear before any
+// arrival there.  A wait of about a second of SM clock gives up, sets the
+// status bit and `abort`; callers return when it fails.
+constexpr unsigned ADJ_FLAG_ONE = 1u << 20;
+__device__ __forceinline__ bool adj_barrier(const AdjArgs &a, unsigned seq, bool flag, int *any) {
+    __shared__ int s_ok;
+    const int raised_here = __syncthreads_or(flag);
+    if (threadIdx.x == 0) {
+        AdjBar *bar = a.bar;
+        int ok = *(volatile int *)&bar->abort == 0;
+        if (ok) {
+            unsigned *cnt = &bar->cnt[seq % 3u];
+            const unsigned inc = 1u | (raised_here ? ADJ_FLAG_ONE : 0u);
+            unsigned v;
+            asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], %2;" : "=r"(v) : "l"(cnt), "r"(inc) : "memory");
+            v += inc;
+            const long long t0 = clock64();
+            int polls = 0;
+            while ((v & (ADJ_FLAG_ONE - 1u)) != gridDim.x) {
+                if (*(volatile int *)&bar->abort) {
+                    ok = 0;
+                    break;
+                }
+                if ((++polls & 63) == 0 && clock64() - t0 > 2000000000LL) {
+                    atomicOr(a.status, ADJ_STATUS_TIMEOUT);
+                    *(volatile int *)&bar->abort = 1;
+                    ok = 0;
+                    break;
+                }
+                if (polls > 64) __nanosleep(32);
+                asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(cnt) : "memory");
+            }
+            *any = (v >> 20) != 0u;
+            if (ok && blockIdx.x == 0) *(volatile unsigned *)&bar->cnt[(seq + 2u) % 3u] = 0u;
+        }
+        s_ok = ok;
+    }
     __syncthreads();
-    const int lane = threadIdx.x & 31, q = threadIdx.x >> 5;
-    const int i = blockIdx.x * ADJ_PPB + q;
+    return s_ok != 0;
+}
+
+__device__ __forceinline__ int type_of(float4 p) { return __float_as_int(p.w); }
+
+// The warp's list of particle i at positions pos (AdjArgs::nbl); lane L tests
+// j = L, L + 32, ... and writes its own column, which only it reads.
+__device__ __forceinline__ void build_list(const AdjArgs &a, const Tab64 *tab, int nt, const float4 *pos, int i,
+                                           float4 pi, int lane) {
     const float iLx = 1.0f / a.Lx, iLy = 1.0f / a.Ly, iLz = 1.0f / a.Lz;
-    float fx = 0.f, fy = 0.f, fz = 0.f, u = 0.f, w = 0.f;
-    float4 pi = make_float4(0.f, 0.f, 0.f, 0.f);
-    int ti = 0;
-    if (i < a.n) {
-        pi = pos_in[i];
-        ti = a.type[i];
-        const Tab32 *row = s_tab + ti * nt;
-        const double rg_lo = (double)a.r_lo - ADJ_KW * a.width, rg_hi = (double)a.r_lo + a.nbins * (double)a.dr + ADJ_KW * a.width;
-        // lane L takes its own column of the list: the neighbours j = L
-        // (mod 32) in ascending order, the same per-lane sums as a loop over
-        // all j whatever the list holds beyond the cutoff, so results do not
-        // depend on when it was built
-        const int *lst = a.nbl + (size_t)i * a.maxnb + lane;
-        const int cnt = min(a.nbc[(size_t)i * ADJ_LANES + lane], a.maxnb / ADJ_LANES);
-        for (int c = 0; c < cnt; c++) {
-            const int j = lst[c * ADJ_LANES];
-            const float4 pj = pos_in[j];
-            const float dx = mic_rint(pj.x - pi.x, a.Lx, iLx);
-            const float dy = mic_rint(pj.y - pi.y, a.Ly, iLy);
-            const float dz = mic_rint(pj.z - pi.z, a.Lz, iLz);
-            const float d2 = dx * dx + dy * dy + dz * dz;
-            const int tj = a.type[j];
-            const Tab32 &e = row[tj];
-            if (d2 < e.cut2) {
-                const float inv2 = 1.0f / d2;
-                const float x2 = e.c * inv2;
-                const float x6 = x2 * x2 * x2;
-                const float x12 = x6 * x6;
-                const float s = (e.cs12 * x12 + e.cs6 * x6) * inv2 - e.sc;
-                fx -= dx * s;
-                fy -= dy * s;
-                fz -= dz * s;
-                const float r = sqrtf(d2);
-                u += 0.5f * (e.cu12 * x12 + e.cu6 * x6 - e.uc + e.sccut * (r - e.cut));
-                w += d2 * s * (1.0f / 6.0f);
-            }
-            if (rdf && ti == 0 && tj == 0) {
-                const double r = sqrt((double)d2);
-                if (r > rg_lo && r < rg_hi) {
-                    const double w2 = 2.0 * (double)a.width * a.width;
-                    const double kn = 1.0 / (sqrt(2.0 * M_PI) * (double)a.width);
-                    int b0 = (int)floor((r - ADJ_KW * a.width - a.r_lo) / a.dr);
-                    int b1 = (int)floor((r + ADJ_KW * a.width - a.r_lo) / a.dr);
-                    b0 = max(b0, 0);
-                    b1 = min(b1, a.nbins - 1);
-                    for (int b = b0; b <= b1; b++) {
-                        const double x = r - ((double)a.r_lo + (b + 0.5) * (double)a.dr);
-                        const double k = kn * exp(-x * x / w2);
-                        atomicAdd(&s_bins[b], (unsigned long long)(k * ADJ_FIX + 0.5));
-                    }
-                }
-            }
-        }
-    }
-    fx = wsum(fx);
-    fy = wsum(fy);
-    fz = wsum(fz);
-    u = wsum(u);
-    w = wsum(w);
-    double kin = 0.0;
-    if (lane == 0 && i < a.n) {
-        const float4 v = vel_in[i];
-        const float m = a.mass[i];
-        float vv[3] = {v.x, v.y, v.z};
-        float r[3] = {pi.x, pi.y, pi.z};
-        const float ff[3] = {fx, fy, fz};
-        const float L[3] = {a.Lx, a.Ly, a.Lz};
-        float k = 0.f;
-#pragma unroll
-        for (int c = 0; c < 3; c++) {  // integrators/NVE.py:78-97
-            float vm = vv[c];
-            vv[c] += ff[c] / m * a.dt;
-            vm += vv[c];
-            vm *= 0.5f;
-            k += 0.5f * m * vm * vm;
-            r[c] += vv[c] * a.dt;
-            if (r[c] * 2.0f > L[c]) r[c] -= L[c];
-            if (r[c] * 2.0f < -L[c]) r[c] += L[c];
-        }
-        pos_out[i] = make_float4(r[0], r[1], r[2], pi.w);
-        vel_out[i] = make_float4(vv[0], vv[1], vv[2], 0.f);
-        kin = k;
-        if (flag_out) {
-            const float4 q = a.rref[i];
-            const float ex = mic_rint(r[0] - q.x, a.Lx, iLx), ey = mic_rint(r[1] - q.y, a.Ly, iLy),
-                        ez = mic_rint(r[2] - q.z, a.Lz, iLz);
-            if (ex * ex + ey * ey + ez * ez > a.move2) atomicOr(flag_out, 1);
-        }
-    }
-    if (lane == 0) {
-        s_red[q][0] = i < a.n ? (double)u : 0.0;
-        s_red[q][1] = i < a.n ? (double)w : 0.0;
-        s_red[q][2] = kin;
-    }
-    __syncthreads();
-    if (threadIdx.x < 3) {
-        double acc = 0.0;
-        for (int p = 0; p < ADJ_PPB; p++) acc += s_red[p][threadIdx.x];
-        partials[(size_t)blockIdx.x * 3 + threadIdx.x] = acc;
-    }
-    if (rdf)
-        for (int b = threadIdx.x; b < a.nbins; b += blockDim.x)
-            if (s_bins[b]) atomicAdd(&gbins[b], s_bins[b]);
-}
-
-// Fixed-order sum of the block partials into the running time sums.
-__global__ void k_adj_reduce(const double *partials, int nblocks, double *acc) {
-    __shared__ double s[3][32];
-    double v[3] = {0.0, 0.0, 0.0};
-    for (int b = threadIdx.x; b < nblocks; b += blockDim.x)
-        for (int q = 0; q < 3; q++) v[q] += partials[(size_t)b * 3 + q];
-    for (int q = 0; q < 3; q++) v[q] = wsum(v[q]);
-    if ((threadIdx.x & 31) == 0)
-        for (int q = 0; q < 3; q++) s[q][threadIdx.x >> 5] = v[q];
-    __syncthreads();
-    if (threadIdx.x < 3) {
-        double t = 0.0;
-        for (int k = 0; k < (int)(blockDim.x >> 5); k++) t += s[threadIdx.x][k];
-        acc[threadIdx.x] += t;
-    }
-}
-
-// Vt = V + dt R + gK dK_n/dv_{n+1},  dK_n/dv_{n+1} = m (v_n + v_{n+1}) / 4
-__global__ void k_adj_vtot(int n, float dt, double gK, const float *mass, const double *R, const double *V,
-                           const float4 *vn, const float4 *vn1, double *Vt) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const double m = mass[i];
-    const float4 a = vn[i], b = vn1[i];
-    const double va[3] = {a.x, a.y, a.z}, vb[3] = {b.x, b.y, b.z};
-    for (int c = 0; c < 3; c++) Vt[3 * i + c] = V[3 * i + c] + (double)dt * R[3 * i + c] + gK * m * (va[c] + vb[c]) * 0.25;
-}
-
-// Pair derivatives of one ordered type pair at distance r (float64).
-struct PairD {
-    double s, ds_dr_over_r;  // s_SF, s0'(r)/r
-    double dsde, dsds;       // d s_SF / d eps, d s_SF / d sigma
-    double dude, duds;       // d u_SF / d eps, d u_SF / d sigma
-    double dudr_over_r;      // u_SF'(r)/r
-};
-
-__device__ __forceinline__ PairD pair_derivs(const Tab64 &e, double r2) {
-    PairD p;
-    const double r = sqrt(r2);
-    const double ir2 = 1.0 / r2;
-    const double sr2 = e.sig * e.sig * ir2;
-    const double sr6 = sr2 * sr2 * sr2, sr12 = sr6 * sr6;
-    const double s0 = e.eps * (48.0 * sr12 - 24.0 * sr6) * ir2;
-    p.s = s0 - e.s_c;
-    p.ds_dr_over_r = e.eps * (-672.0 * sr12 + 192.0 * sr6) * ir2 * ir2;
-    p.dsde = p.s / e.eps;
-    const double ds0ds = e.eps * (576.0 * sr12 - 144.0 * sr6) * ir2 / e.sig;
-    p.dsds = ds0ds - e.dsds_c;
-    const double u0 = 4.0 * e.eps * (sr12 - sr6);
-    const double uSF = u0 - e.u_c + e.s_c * e.cut * (r - e.cut);
-    p.dude = uSF / e.eps;
-    const double du0ds = 4.0 * e.eps * (12.0 * sr12 - 6.0 * sr6) / e.sig;
-    p.duds = du0ds - e.duds_c + e.dsds_c * e.cut * (r - e.cut);
-    p.dudr_over_r = -s0 + e.s_c * e.cut / r;
-    return p;
-}
-
-// Backward step at r_n: R += (dt/m) HVP(Vt) + gU dU/dr + gW dW/dr + dG/dr,
-// V = Vt + gK dK_n/dv_n, per-block parameter cotangents accumulated.
-__global__ void __launch_bounds__(ADJ_BLOCK) k_adj_back(AdjArgs a, Tables tab, const float4 *__restrict__ pos,
-                                                        const double *__restrict__ Vt, double *R, double *V,
-                                                        const float4 *vn, const float4 *vn1, double gU, double gW,
-                                                        double gK, const double *gG, double *th_part) {
-    __shared__ Tab64 s_tab[ADJ_MAXT * ADJ_MAXT];
-    __shared__ double s_th[ADJ_PPB][ADJ_NTH];
-    const int nt = tab.nt;
-    for (int t = threadIdx.x; t < nt * nt; t += blockDim.x) s_tab[t] = tab.t64[t];
-    __syncthreads();
-    const int lane = threadIdx.x & 31, q = threadIdx.x >> 5;
-    const int i = blockIdx.x * ADJ_PPB + q;
-    double h[3] = {0, 0, 0}, du[3] = {0, 0, 0}, dw[3] = {0, 0, 0}, dg[3] = {0, 0, 0};
-    double th[ADJ_NTH];
-#pragma unroll
-    for (int k = 0; k < ADJ_NTH; k++) th[k] = 0.0;
-    double mi = 1.0;
-    if (i < a.n) {
-        const float4 pi = pos[i];
-        const int ti = a.type[i];
-        mi = a.mass[i];
-        const double vi[3] = {Vt[3 * i], Vt[3 * i + 1], Vt[3 * i + 2]};
-        // input of the Hessian-vector product: the kick's cotangent (dt / m) Vt
-        const double ui[3] = {a.dt / mi * vi[0], a.dt / mi * vi[1], a.dt / mi * vi[2]};
-        const float iLx = 1.0f / a.Lx, iLy = 1.0f / a.Ly, iLz = 1.0f / a.Lz;
-        const double rg_lo = (double)a.r_lo - ADJ_KW * a.width, rg_hi = (double)a.r_lo + a.nbins * (double)a.dr + ADJ_KW * a.width;
-        const double cdt = (double)a.dt / mi;
-        const int *lst = a.nbl + (size_t)i * a.maxnb + lane;
-        const int cnt = min(a.nbc[(size_t)i * ADJ_LANES + lane], a.maxnb / ADJ_LANES);
-        for (int c = 0; c < cnt; c++) {  // lane L: the neighbours j = L (mod 32), ascending
-            const int j = lst[c * ADJ_LANES];
-            const float4 pj = pos[j];
-            // same float32 displacement and cutoff test as the forward
-            const float fdx = mic_rint(pj.x - pi.x, a.Lx, iLx);
-            const float fdy = mic_rint(pj.y - pi.y, a.Ly, iLy);
-            const float fdz = mic_rint(pj.z - pi.z, a.Lz, iLz);
-            const float fd2 = fdx * fdx + fdy * fdy + fdz * fdz;
-            const int tj = a.type[j];
-            const Tab64 &e = s_tab[ti * nt + tj];
-            // d = r_i - r_j (the forward's dx is r_j - r_i)
-            const double d[3] = {-(double)fdx, -(double)fdy, -(double)fdz};
-            const double r2 = d[0] * d[0] + d[1] * d[1] + d[2] * d[2];
-            if (fd2 < (float)e.cut2) {
-                const PairD p = pair_derivs(e, r2);
-                const double cj = (double)a.dt / (double)a.mass[j];
-                const double dv[3] = {ui[0] - cj * Vt[3 * j], ui[1] - cj * Vt[3 * j + 1], ui[2] - cj * Vt[3 * j + 2]};
-                const double dd = d[0] * dv[0] + d[1] * dv[1] + d[2] * dv[2];
-                const double vd = d[0] * vi[0] + d[1] * vi[1] + d[2] * vi[2];
-                for (int c = 0; c < 3; c++) {
-                    h[c] += p.s * dv[c] + p.ds_dr_over_r * dd * d[c];
-                    du[c] += p.dudr_over_r * d[c];
-                    dw[c] += (2.0 * p.s + r2 * p.ds_dr_over_r) * d[c] * (1.0 / 3.0);
-                }
-                const int k = ti * nt + tj;
-                // force term (dt/m) (df_i/dtheta) . Vt_i, f_i = sum_j s d
-                th[2 * k] += cdt * p.dsds * vd + gU * 0.5 * p.duds + gW * r2 * p.dsds * (1.0 / 6.0);
-                th[2 * k + 1] += cdt * p.dsde * vd + gU * 0.5 * p.dude + gW * r2 * p.dsde * (1.0 / 6.0);
-            }
-            if (gG && ti == 0 && tj == 0) {
-                const double r = sqrt(r2);
-                if (r > rg_lo && r < rg_hi) {
-                    const double w2 = (double)a.width * a.width;
-                    const double kn = 1.0 / (sqrt(2.0 * M_PI) * (double)a.width);
-                    int b0 = (int)floor((r - ADJ_KW * a.width - a.r_lo) / a.dr);
-                    int b1 = (int)floor((r + ADJ_KW * a.width - a.r_lo) / a.dr);
-                    b0 = max(b0, 0);
-                    b1 = min(b1, a.nbins - 1);
-                    double acc = 0.0;
-                    for (int b = b0; b <= b1; b++) {
-                        const double x = r - ((double)a.r_lo + (b + 0.5) * (double)a.dr);
-                        acc += gG[b] * 2.0 * (-x / w2) * kn * exp(-0.5 * x * x / w2);
-                    }
-                    for (int c = 0; c < 3; c++) dg[c] += acc * d[c] / r;
-                }
-            }
-        }
-    }
-    for (int c = 0; c < 3; c++) {
-        h[c] = wsum(h[c]);
-        du[c] = wsum(du[c]);
-        dw[c] = wsum(dw[c]);
-        dg[c] = wsum(dg[c]);
-    }
-    const int nth = 2 * nt * nt;
-    for (int k = 0; k < nth; k++) th[k] = wsum(th[k]);
-    if (lane == 0) {
-        for (int k = 0; k < nth; k++) s_th[q][k] = i < a.n ? th[k] : 0.0;
-        if (i < a.n) {
-            const float4 va = vn[i], vb = vn1[i];
-            const double sa[3] = {va.x, va.y, va.z}, sb[3] = {vb.x, vb.y, vb.z};
-            for (int c = 0; c < 3; c++) {
-                R[3 * i + c] += h[c] + gU * du[c] + gW * dw[c] + dg[c];
-                V[3 * i + c] = Vt[3 * i + c] + gK * mi * (sa[c] + sb[c]) * 0.25;
-            }
-        }
-    }
-    __syncthreads();
-    if (threadIdx.x < nth) {
-        double acc = 0.0;
-        for (int p = 0; p < ADJ_PPB; p++) acc += s_th[p][threadIdx.x];
-        th_part[(size_t)blockIdx.x * ADJ_NTH + threadIdx.x] += acc;
-    }
-}
-
-// Neighbour list (gated): rebuilt when `force` or when flags[rd] is set;
-// block 0 clears flags[clr] for the next writer.  A warp per particle; lane L
-// tests j = L, L + 32, ... and appends its hits to column L of the particle's
-// rows (entry c of column L at c * 32 + L), so each column holds the
-// neighbours j = L (mod 32) in ascending order.
-__global__ void __launch_bounds__(ADJ_BLOCK) k_adj_build(AdjArgs a, const float4 *__restrict__ pos, int *nbl, int *nbc,
-                                                         int force, int rd, int clr) {
-    const bool go = force || *(volatile int *)&a.flags[rd] != 0;
-    if (blockIdx.x == 0 && threadIdx.x == 0) a.flags[clr] = 0;
-    if (!go) return;
-    const int lane = threadIdx.x & 31;
-    const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (i >= a.n) return;
-    const float iLx = 1.0f / a.Lx, iLy = 1.0f / a.Ly, iLz = 1.0f / a.Lz;
-    const float4 pi = pos[i];
-    const int rows = a.maxnb / ADJ_LANES;
-    int *col = nbl + (size_t)i * a.maxnb + lane;
-    int count = 0;
+    const int rows = a.maxnb / ADJ_LANES, ti = type_of(pi);
+    int *col = a.nbl + (size_t)i * a.maxnb + lane;
+    int near = 0, far = 0;
+#pragma unroll 4
     for (int j = lane; j < a.n; j += ADJ_LANES) {
-        if (j == i) continue;
         const float4 pj = pos[j];
         const float dx = mic_rint(pj.x - pi.x, a.Lx, iLx);
         const float dy = mic_rint(pj.y - pi.y, a.Ly, iLy);
         const float dz = mic_rint(pj.z - pi.z, a.Lz, iLz);
-        if (dx * dx + dy * dy + dz * dz < a.rl2) {
-            if (count < rows) col[count * ADJ_LANES] = j;
-            count++;
+        const float d2 = dx * dx + dy * dy + dz * dz;
+        const int tj = type_of(pj);
+        if (j == i) continue;
+        if (d2 < tab[ti * nt + tj].reach2) {
+            if (near + far < rows) col[near * ADJ_LANES] = j;
+            near++;
+        } else if (d2 < a.far2 && ti == 0 && tj == 0) {
+            if (near + far < rows) col[(rows - 1 - far) * ADJ_LANES] = j;
+            far++;
         }
     }
-    nbc[(size_t)i * ADJ_LANES + lane] = count;
-    if (count > rows) atomicOr(a.status, ADJ_STATUS_OVERFLOW);
+    if (near + far > rows) {
+        atomicOr(a.status, ADJ_STATUS_OVERFLOW);
+        near = min(near, rows);
+        far = min(far, rows - near);
+    }
+    a.nbc[(size_t)i * ADJ_LANES + lane] = near | (far << 16);
     if (lane == 0) a.rref[i] = pi;
 }
 
-// Sets flags[wr] when a particle of pos has moved more than skin/2 since the
-// last build (the backward sweep's positions come from a stored segment).
-__global__ void k_adj_check(AdjArgs a, const float4 *__restrict__ pos, int wr) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= a.n) return;
-    const float4 p = pos[i], q = a.rref[i];
+__device__ __forceinline__ bool moved_far(const AdjArgs &a, float4 p, float4 q) {
     const float ex = mic_rint(p.x - q.x, a.Lx, 1.0f / a.Lx), ey = mic_rint(p.y - q.y, a.Ly, 1.0f / a.Ly),
                 ez = mic_rint(p.z - q.z, a.Lz, 1.0f / a.Lz);
-    if (ex * ex + ey * ey + ez * ez > a.move2) atomicOr(&a.flags[wr], 1);
+    return ex * ex + ey * ey + ez * ez > a.move2;
+}
+
+// Gaussian bins around distance r: calls f(b, x, exp(-x^2 / (2 w^2))) for
+// every bin b within the kernel's support, x = r - centre_b.  From one bin to
+// the next the exponent grows by (2 x dr - dr^2) / (2 w^2): two exponentials
+// for the first bin, two products for each further one (relative error 1e-16
+// per bin); bins wider than four widths take one exponential each.
+template <typename F>
+__device__ __forceinline__ void rdf_bins(const AdjArgs &a, double r, F f) {
+    const double w = a.width, dr = a.dr, iw2 = 0.5 / (w * w);
+    int b0 = (int)floor((r - ADJ_KW * w - a.r_lo) / dr);
+    int b1 = (int)floor((r + ADJ_KW * w - a.r_lo) / dr);
+    b0 = max(b0, 0);
+    b1 = min(b1, a.nbins - 1);
+    double x = r - ((double)a.r_lo + (b0 + 0.5) * dr);
+    double e = exp(-x * x * iw2);
+    if (dr <= 4.0 * w) {
+        double g = exp((2.0 * x * dr - dr * dr) * iw2);
+        const double k = a.step_ratio;
+        for (int b = b0; b <= b1; b++) {
+            f(b, x, e);
+            x -= dr;
+            e *= g;
+            g *= k;
+        }
+    } else {
+        for (int b = b0; b <= b1; b++) {
+            x = r - ((double)a.r_lo + (b + 0.5) * dr);
+            f(b, x, exp(-x * x * iw2));
+        }
+    }
+}
+
+// The states of a run of steps: state k at p + ((k - k0) % mod) * n.
+struct States {
+    float4 *p, *v;
+    int k0, mod;
+    __device__ __forceinline__ size_t at(int k, int n) const { return (size_t)((k - k0) % mod) * n; }
+};
+
+// Forward: steps [s0, s0 + nsteps) from state s0, one warp per particle.
+// acc (observables wanted): float64 sums of U, W, K per block into acc[block][3]
+// and, on sampled steps, the A-A kernel sums into gbins (fixed point, integer
+// atomics: order-independent).
+//
+// A step is a serial chain: list chunk, position gathers, warp sums, the new
+// position, the grid barrier.  Measured on B200, KA N 4096, 50 steps with 40
+// RDF bins sampled every 10: 1.0 ms, and observables and gradient together
+// 2.23 ms, against 7.35 ms with eight launches a step (gated N^2 rebuild
+// kernels, segments recomputed from checkpoints).
+struct ForwardArgs {
+    States st;
+    int s0, nsteps;
+    double *acc;
+    unsigned long long *gbins;
+    int rdf_every, copies;  // copies of the bins in shared memory, 32 columns each
+    float4 *ck_pos, *ck_vel;
+    int ckpt;
+};
+__global__ void __launch_bounds__(ADJ_WARPS * 32, 1) k_adj_forward(AdjArgs a, const __grid_constant__ Tables tab,
+                                                                   ForwardArgs f) {
+    extern __shared__ unsigned long long s_bins[];  // [copies][nbins][32]
+    __shared__ Tab32 s_tab[ADJ_MAXT * ADJ_MAXT];
+    __shared__ Tab64 s_tab64[ADJ_MAXT * ADJ_MAXT];
+    __shared__ double s_red[ADJ_WARPS][3];
+    __shared__ int s_any;
+    const int nt = tab.nt;
+    for (int t = threadIdx.x; t < nt * nt; t += blockDim.x) {
+        s_tab[t] = tab.t32[t];
+        s_tab64[t] = tab.t64[t];
+    }
+    const bool bins = f.gbins != nullptr;
+    if (bins)
+        for (int b = threadIdx.x; b < f.copies * a.nbins * 32; b += blockDim.x) s_bins[b] = 0ull;
+    __syncthreads();
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, wpb = blockDim.x >> 5;
+    const int first = blockIdx.x * wpb + w, nwarps = gridDim.x * wpb;
+    const float iLx = 1.0f / a.Lx, iLy = 1.0f / a.Ly, iLz = 1.0f / a.Lz;
+    const int rows = a.maxnb / ADJ_LANES;
+    double sum_u = 0.0, sum_w = 0.0, sum_k = 0.0;  // lane 0: of the warp's particles, all steps
+    for (int s = 0; s < f.nsteps; s++) {
+        const int step = f.s0 + s;
+        const float4 *pos_in = f.st.p + f.st.at(step, a.n), *vel_in = f.st.v + f.st.at(step, a.n);
+        float4 *pos_out = f.st.p + f.st.at(step + 1, a.n), *vel_out = f.st.v + f.st.at(step + 1, a.n);
+        const bool rebuild = s == 0 || s_any != 0;
+        const bool rdf = bins && step % f.rdf_every == 0;
+        bool moved = false;
+        for (int i = first; i < a.n; i += nwarps) {
+            const float4 pi = pos_in[i];
+            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+            float m = 1.f;
+            if (lane == 0) {
+                v = vel_in[i];
+                m = a.mass[i];
+            }
+            const int ti = type_of(pi);
+            if (rebuild) build_list(a, s_tab64, nt, pos_in, i, pi, lane);
+            const Tab32 *row = s_tab + ti * nt;
+            const int *lst = a.nbl + (size_t)i * a.maxnb + lane;
+            const int both = a.nbc[(size_t)i * ADJ_LANES + lane];
+            const int cnt = both & 0xffff;
+            float fx = 0.f, fy = 0.f, fz = 0.f, u = 0.f, wv = 0.f;
+            // four entries' loads in flight; the sums in ascending j
+            for (int c0 = 0; c0 < cnt; c0 += 4) {
+                int j[4];
+                float4 p[4];
+#pragma unroll
+                for (int k = 0; k < 4; k++) j[k] = c0 + k < cnt ? lst[(c0 + k) * ADJ_LANES] : i;
+#pragma unroll
+                for (int k = 0; k < 4; k++) p[k] = pos_in[j[k]];
+#pragma unroll
+                for (int k = 0; k < 4; k++) {
+                    if (c0 + k >= cnt) break;
+                    const float dx = mic_rint(p[k].x - pi.x, a.Lx, iLx);
+                    const float dy = mic_rint(p[k].y - pi.y, a.Ly, iLy);
+                    const float dz = mic_rint(p[k].z - pi.z, a.Lz, iLz);
+                    const float d2 = dx * dx + dy * dy + dz * dz;
+                    const Tab32 &e = row[type_of(p[k])];
+                    if (d2 < e.cut2) {
+                        const float inv2 = 1.0f / d2;
+                        const float x2 = e.c * inv2;
+                        const float x6 = x2 * x2 * x2;
+                        const float x12 = x6 * x6;
+                        const float sp = (e.cs12 * x12 + e.cs6 * x6) * inv2 - e.sc;
+                        fx -= dx * sp;
+                        fy -= dy * sp;
+                        fz -= dz * sp;
+                        const float r = sqrtf(d2);
+                        u += 0.5f * (e.cu12 * x12 + e.cu6 * x6 - e.uc + e.sccut * (r - e.cut));
+                        wv += d2 * sp * (1.0f / 6.0f);
+                    }
+                }
+            }
+            if (rdf && ti == 0) {
+                const double rg_lo = (double)a.r_lo - ADJ_KW * a.width,
+                             rg_hi = (double)a.r_lo + a.nbins * (double)a.dr + ADJ_KW * a.width;
+                const double kn = ADJ_FIX / (sqrt(2.0 * M_PI) * (double)a.width);
+                unsigned long long *mine = s_bins + (size_t)(w % f.copies) * a.nbins * 32 + lane;
+                const int all = cnt + (both >> 16);
+                for (int c = 0; c < all; c++) {
+                    const int j = lst[(c < cnt ? c : rows - 1 - (c - cnt)) * ADJ_LANES];
+                    const float4 p = pos_in[j];
+                    if (type_of(p) != 0) continue;
+                    const float dx = mic_rint(p.x - pi.x, a.Lx, iLx);
+                    const float dy = mic_rint(p.y - pi.y, a.Ly, iLy);
+                    const float dz = mic_rint(p.z - pi.z, a.Lz, iLz);
+                    const double r = sqrt((double)(dx * dx + dy * dy + dz * dz));
+                    if (r > rg_lo && r < rg_hi)
+                        rdf_bins(a, r, [&](int b, double, double e) {
+                            atomicAdd(&mine[b * 32], (unsigned long long)(kn * e + 0.5));
+                        });
+                }
+                __syncwarp();
+            }
+            fx = wsum(fx);
+            fy = wsum(fy);
+            fz = wsum(fz);
+            u = wsum(u);
+            wv = wsum(wv);
+            if (lane == 0) {
+                float vv[3] = {v.x, v.y, v.z};
+                float r[3] = {pi.x, pi.y, pi.z};
+                const float ff[3] = {fx, fy, fz};
+                const float L[3] = {a.Lx, a.Ly, a.Lz};
+                float k = 0.f;
+#pragma unroll
+                for (int c = 0; c < 3; c++) {  // integrators/NVE.py:78-97
+                    float vm = vv[c];
+                    vv[c] += ff[c] / m * a.dt;
+                    vm += vv[c];
+                    vm *= 0.5f;
+                    k += 0.5f * m * vm * vm;
+                    r[c] += vv[c] * a.dt;
+                    if (r[c] * 2.0f > L[c]) r[c] -= L[c];
+                    if (r[c] * 2.0f < -L[c]) r[c] += L[c];
+                }
+                if (f.ck_pos && step % f.ckpt == 0) {
+                    const size_t o = (size_t)(step / f.ckpt) * a.n + i;
+                    f.ck_pos[o] = pi;
+                    f.ck_vel[o] = v;
+                }
+                const float4 pn = make_float4(r[0], r[1], r[2], pi.w);
+                pos_out[i] = pn;
+                vel_out[i] = make_float4(vv[0], vv[1], vv[2], 0.f);
+                moved |= moved_far(a, pn, a.rref[i]);
+                sum_u += u;
+                sum_w += wv;
+                sum_k += k;
+            }
+        }
+        if (s + 1 < f.nsteps && !adj_barrier(a, (unsigned)s, moved, &s_any)) return;
+    }
+    if (!f.acc) return;
+    if (lane == 0) {
+        s_red[w][0] = sum_u;
+        s_red[w][1] = sum_w;
+        s_red[w][2] = sum_k;
+    }
+    __syncthreads();
+    if (threadIdx.x < 3) {
+        double t = 0.0;
+        for (int k = 0; k < wpb; k++) t += s_red[k][threadIdx.x];
+        f.acc[(size_t)blockIdx.x * 3 + threadIdx.x] = t;
+    }
+    if (bins)
+        for (int b = threadIdx.x; b < a.nbins; b += blockDim.x) {
+            unsigned long long t = 0ull;
+            for (int c = 0; c < f.copies; c++)
+                for (int l = 0; l < 32; l++) t += s_bins[((size_t)c * a.nbins + b) * 32 + l];
+            if (t) atomicAdd(&f.gbins[b], t);
+        }
+}
+
+// Reverse sweep over the steps s0 + len - 1 .. s0, one warp per particle.
+// Per step: R += (dt/m) HVP(Vt) + gU dU/dr + gW dW/dr + dG/dr, V = Vt + gK
+// dK_n/dv_n, parameter cotangents added to the warp's sums; then, for the step
+// before, Vt = V + dt R + gK dK/dv and the kick's cotangent U = (dt / m) Vt,
+// which the other particles read after the barrier (double-buffered by step
+// parity).  Between the steps of a sweep V holds Vt.
+struct SweepArgs {
+    States st;
+    int s0, len;
+    double gU, gW, gK;
+    const double *gG;  // 2 grad_g_b norm_b (-1 / w^2) kn by bin, NULL without RDF cotangents
+    int rdf_every, window;
+    double *R, *V;
+    double4 *U;       // 2 n
+    // parameter cotangents: the warps' running sums between the segments of a
+    // sweep (the same additions in the same order however it is cut), then
+    // the blocks' sums of the last one
+    double *th_warp;  // [blocks][warps][ADJ_NTH]
+    double *th_part;  // [blocks][ADJ_NTH]
+    int first_segment, last_segment;
+};
+// Pairs inside the cutoff wait here until 32 of them are pending, so that
+// the float64 derivatives run with every lane busy (a column holds about 1.5
+// pairs beyond the cutoff for each inside it, and the columns' lengths differ).
+// A warp's ring takes a round's hits beside 31 pending ones.  Measured on
+// B200, KA N 4096, 50 steps: the sweep takes 1.19 ms.
+constexpr int ADJ_RING = 64;
+constexpr size_t ADJ_RING_BYTES = ADJ_RING * sizeof(float4);  // displacement r_j - r_i, and j << 2 | t_j
+
+template <int NT>
+__global__ void __launch_bounds__(ADJ_WARPS * 32, 1) k_adj_sweep(AdjArgs a, const __grid_constant__ Tables tab,
+                                                                 SweepArgs f) {
+    __shared__ Tab64 s_tab[ADJ_MAXT * ADJ_MAXT];
+    __shared__ double s_th[ADJ_WARPS][ADJ_NTH];
+    __shared__ double s_gG[ADJ_MAXB];
+    extern __shared__ float4 s_ring[];  // [warps][ADJ_RING]
+    __shared__ int s_any;
+    const int nt = tab.nt;
+    for (int t = threadIdx.x; t < nt * nt; t += blockDim.x) s_tab[t] = tab.t64[t];
+    const int nth = (int)(blockDim.x >> 5) * ADJ_NTH;
+    double *th_state = f.th_warp + (size_t)blockIdx.x * nth;
+    for (int t = threadIdx.x; t < nth; t += blockDim.x) (&s_th[0][0])[t] = f.first_segment ? 0.0 : th_state[t];
+    if (f.gG)
+        for (int b = threadIdx.x; b < a.nbins; b += blockDim.x) s_gG[b] = f.gG[b];
+    __syncthreads();
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, wpb = blockDim.x >> 5;
+    const int first = blockIdx.x * wpb + w, nwarps = gridDim.x * wpb;
+    const float iLx = 1.0f / a.Lx, iLy = 1.0f / a.Ly, iLz = 1.0f / a.Lz;
+    const unsigned below = (1u << lane) - 1u;
+    const int rows = a.maxnb / ADJ_LANES;
+    const double dt = a.dt;
+    float4 *ring = s_ring + w * ADJ_RING;
+    // lane 0: Vt and U of step s from this particle's V and R after step s + 1
+    auto start_step = [&](int s, int i, double (&R)[3], double (&V)[3]) {
+        if (f.window > 0 && (s + 1) % f.window == 0) {
+            // last step of a window: nothing flows back across its end
+#pragma unroll
+            for (int c = 0; c < 3; c++) R[c] = V[c] = 0.0;
+        }
+        const double m = a.mass[i];
+        const float4 p = f.st.v[f.st.at(s, a.n) + i], q = f.st.v[f.st.at(s + 1, a.n) + i];
+        const double pv[3] = {p.x, p.y, p.z}, qv[3] = {q.x, q.y, q.z};
+#pragma unroll
+        for (int c = 0; c < 3; c++) V[c] = V[c] + dt * R[c] + f.gK * m * (pv[c] + qv[c]) * 0.25;
+        const double k = dt / m;
+        f.U[(size_t)(s & 1) * a.n + i] = make_double4(k * V[0], k * V[1], k * V[2], 0.0);
+    };
+    unsigned seq = 0;
+    for (int i = first; i < a.n; i += nwarps)
+        if (lane == 0) {
+            double R[3], V[3];
+#pragma unroll
+            for (int c = 0; c < 3; c++) R[c] = f.R[3 * (size_t)i + c], V[c] = f.V[3 * (size_t)i + c];
+            start_step(f.s0 + f.len - 1, i, R, V);
+#pragma unroll
+            for (int c = 0; c < 3; c++) f.R[3 * (size_t)i + c] = R[c], f.V[3 * (size_t)i + c] = V[c];
+        }
+    if (!adj_barrier(a, seq++, false, &s_any)) return;
+    for (int k = f.len - 1; k >= 0; k--) {
+        const int s = f.s0 + k;
+        const float4 *pos = f.st.p + f.st.at(s, a.n);
+        const double4 *U = f.U + (size_t)(s & 1) * a.n;
+        const bool rebuild = k == f.len - 1 || s_any != 0;
+        const bool rdf = f.gG && f.rdf_every > 0 && s % f.rdf_every == 0;
+        bool moved = false;
+        for (int i = first; i < a.n; i += nwarps) {
+            const float4 pi = pos[i];
+            const int ti = type_of(pi);
+            if (rebuild) build_list(a, s_tab, nt, pos, i, pi, lane);
+            const int *lst = a.nbl + (size_t)i * a.maxnb + lane;
+            const int both = a.nbc[(size_t)i * ADJ_LANES + lane];
+            const int cnt = both & 0xffff;
+            double R[3] = {0, 0, 0}, Vt[3];  // this particle's, on every lane
+#pragma unroll
+            for (int c = 0; c < 3; c++) Vt[c] = f.V[3 * (size_t)i + c];
+            const double4 ui = U[i];
+            const double cdt = dt / a.mass[i];
+            double acc[3] = {0, 0, 0};  // J^T Vt + gU dU/dr + gW dW/dr + dG/dr
+            double th[2 * NT];          // d/dsigma, d/depsilon by neighbour type
+#pragma unroll
+            for (int t = 0; t < 2 * NT; t++) th[t] = 0.0;
+            int head = 0, tail = 0;
+            auto drain = [&](int take) {
+                __syncwarp();
+                if (lane < take) {
+                    const float4 en = ring[(head + lane) & (ADJ_RING - 1)];
+                    const int code = __float_as_int(en.w), j = code >> 2, tj = code & 3;
+                    const double4 uj = U[j];
+                    const Tab64 &e = s_tab[ti * nt + tj];
+                    // d = r_i - r_j (the forward's difference is r_j - r_i)
+                    const double d[3] = {-(double)en.x, -(double)en.y, -(double)en.z};
+                    const double r2 = d[0] * d[0] + d[1] * d[1] + d[2] * d[2];
+                    const double ir = rsqrt(r2), ir2 = ir * ir, r = r2 * ir;
+                    const double sr2 = e.sig2 * ir2;
+                    const double sr6 = sr2 * sr2 * sr2, sr12 = sr6 * sr6;
+                    const double s0 = e.eps * (48.0 * sr12 - 24.0 * sr6) * ir2;
+                    const double sp = s0 - e.s_c;
+                    const double dsr = e.eps * (-672.0 * sr12 + 192.0 * sr6) * ir2 * ir2;  // s0'(r) / r
+                    const double dv[3] = {ui.x - uj.x, ui.y - uj.y, ui.z - uj.z};
+                    const double dd = d[0] * dv[0] + d[1] * dv[1] + d[2] * dv[2];
+                    // along d: the HVP's second part, gU u'/r, gW (d (r2 s) / dr) / (3 r)
+                    const double along = dsr * dd + f.gU * (e.s_c * e.cut * ir - s0) +
+                                         f.gW * (2.0 * sp + r2 * dsr) * (1.0 / 3.0);
+#pragma unroll
+                    for (int c = 0; c < 3; c++) acc[c] += sp * dv[c] + along * d[c];
+                    const double vd = d[0] * Vt[0] + d[1] * Vt[1] + d[2] * Vt[2];
+                    const double dsde = sp * e.ieps;
+                    const double dsds = e.eps_sig * (576.0 * sr12 - 144.0 * sr6) * ir2 - e.dsds_c;
+                    const double usf = 4.0 * e.eps * (sr12 - sr6) - e.u_c + e.s_c * e.cut * (r - e.cut);
+                    const double dude = usf * e.ieps;
+                    const double duds = 4.0 * e.eps_sig * (12.0 * sr12 - 6.0 * sr6) - e.duds_c +
+                                        e.dsds_c * e.cut * (r - e.cut);
+                    // force term (dt/m) (df_i/dtheta) . Vt_i, f_i = sum_j s d
+                    const double ks = cdt * vd + f.gW * r2 * (1.0 / 6.0);
+                    const double ts = ks * dsds + f.gU * 0.5 * duds, te = ks * dsde + f.gU * 0.5 * dude;
+#pragma unroll
+                    for (int t = 0; t < NT; t++)
+                        if (t == tj) {
+                            th[2 * t] += ts;
+                            th[2 * t + 1] += te;
+                        }
+                }
+                head += take;
+                __syncwarp();
+            };
+            // 64 rows of the columns at a time: first the lanes' hits as bits
+            // (same float32 displacement and cutoff test as the forward), then
+            // round by round every lane's next hit into the ring, so the order
+            // of the sums does not depend on what the list holds beyond the
+            // cutoff, nor on when it was built
+            auto pair = [&](int j, float4 p, float &dx, float &dy, float &dz) {
+                dx = mic_rint(p.x - pi.x, a.Lx, iLx);
+                dy = mic_rint(p.y - pi.y, a.Ly, iLy);
+                dz = mic_rint(p.z - pi.z, a.Lz, iLz);
+                return dx * dx + dy * dy + dz * dz;
+            };
+            for (int c00 = 0; __any_sync(0xffffffffu, c00 < cnt); c00 += 64) {
+                unsigned long long hits = 0ull;
+                const int end = min(cnt, c00 + 64);
+                for (int c0 = c00; c0 < end; c0 += 4) {
+                    int j[4];
+                    float4 p[4];
+#pragma unroll
+                    for (int q = 0; q < 4; q++) j[q] = c0 + q < end ? lst[(c0 + q) * ADJ_LANES] : i;
+#pragma unroll
+                    for (int q = 0; q < 4; q++) p[q] = pos[j[q]];
+                    unsigned bits = 0;
+#pragma unroll
+                    for (int q = 0; q < 4; q++) {
+                        float dx, dy, dz;
+                        const float d2 = pair(j[q], p[q], dx, dy, dz);
+                        if (c0 + q < end && d2 < s_tab[ti * nt + type_of(p[q])].cut2) bits |= 1u << q;
+                    }
+                    hits |= (unsigned long long)bits << (c0 - c00);
+                }
+                while (__any_sync(0xffffffffu, hits != 0ull) || tail > head) {
+                    const bool hit = hits != 0ull;
+                    const unsigned m = __ballot_sync(0xffffffffu, hit);
+                    if (hit) {
+                        const int j = lst[(c00 + __ffsll(hits) - 1) * ADJ_LANES];
+                        hits &= hits - 1ull;
+                        const float4 p = pos[j];
+                        float dx, dy, dz;
+                        pair(j, p, dx, dy, dz);
+                        ring[(tail + __popc(m & below)) & (ADJ_RING - 1)] =
+                            make_float4(dx, dy, dz, __int_as_float((j << 2) | type_of(p)));
+                    }
+                    tail += __popc(m);
+                    // a full round, or after the last hits what is left
+                    if (tail - head >= 32 || (m == 0u && !__any_sync(0xffffffffu, end < cnt)))
+                        drain(min(32, tail - head));
+                    else if (m == 0u)
+                        break;
+                }
+            }
+            if (rdf && ti == 0) {
+                const double rg_lo = (double)a.r_lo - ADJ_KW * a.width,
+                             rg_hi = (double)a.r_lo + a.nbins * (double)a.dr + ADJ_KW * a.width;
+                // the column's two lists merged: ascending j, wherever the
+                // build put a pair
+                int near = 0, far = 0;
+                const int nfar = both >> 16;
+                int jn = near < cnt ? lst[0] : a.n, jf = far < nfar ? lst[(rows - 1) * ADJ_LANES] : a.n;
+                while (jn < a.n || jf < a.n) {
+                    const int j = min(jn, jf);
+                    if (jn < jf) {
+                        near++;
+                        jn = near < cnt ? lst[near * ADJ_LANES] : a.n;
+                    } else {
+                        far++;
+                        jf = far < nfar ? lst[(rows - 1 - far) * ADJ_LANES] : a.n;
+                    }
+                    const float4 p = pos[j];
+                    if (type_of(p) != 0) continue;
+                    float dx, dy, dz;
+                    pair(j, p, dx, dy, dz);
+                    const double d[3] = {-(double)dx, -(double)dy, -(double)dz};
+                    const double r = sqrt(d[0] * d[0] + d[1] * d[1] + d[2] * d[2]);
+                    if (r > rg_lo && r < rg_hi) {
+                        double g = 0.0;
+                        rdf_bins(a, r, [&](int b, double x, double e) { g += s_gG[b] * x * e; });
+                        g /= r;
+#pragma unroll
+                        for (int q = 0; q < 3; q++) acc[q] += g * d[q];
+                    }
+                }
+                __syncwarp();
+            }
+#pragma unroll
+            for (int c = 0; c < 3; c++) acc[c] = wsum(acc[c]);
+#pragma unroll
+            for (int t = 0; t < NT; t++)
+                if (t < nt) {
+                    th[2 * t] = wsum(th[2 * t]);
+                    th[2 * t + 1] = wsum(th[2 * t + 1]);
+                }
+            if (lane == 0) {
+#pragma unroll
+                for (int t = 0; t < NT; t++)
+                    if (t < nt) {
+                        s_th[w][2 * (ti * nt + t)] += th[2 * t];
+                        s_th[w][2 * (ti * nt + t) + 1] += th[2 * t + 1];
+                    }
+                const double m = a.mass[i];
+                const float4 va = f.st.v[f.st.at(s, a.n) + i], vb = f.st.v[f.st.at(s + 1, a.n) + i];
+                const double sa[3] = {va.x, va.y, va.z}, sb[3] = {vb.x, vb.y, vb.z};
+#pragma unroll
+                for (int c = 0; c < 3; c++) {
+                    R[c] = f.R[3 * (size_t)i + c] + acc[c];
+                    Vt[c] += f.gK * m * (sa[c] + sb[c]) * 0.25;
+                }
+                if (k > 0) {
+                    start_step(s - 1, i, R, Vt);
+                    moved |= moved_far(a, f.st.p[f.st.at(s - 1, a.n) + i], a.rref[i]);
+                }
+#pragma unroll
+                for (int c = 0; c < 3; c++) f.R[3 * (size_t)i + c] = R[c], f.V[3 * (size_t)i + c] = Vt[c];
+            }
+            __syncwarp();
+        }
+        if (k > 0 && !adj_barrier(a, seq++, moved, &s_any)) return;
+    }
+    __syncthreads();
+    if (!f.last_segment) {
+        for (int t = threadIdx.x; t < nth; t += blockDim.x) th_state[t] = (&s_th[0][0])[t];
+    } else if (threadIdx.x < ADJ_NTH) {
+        double t = 0.0;
+        for (int p = 0; p < wpb; p++) t += s_th[p][threadIdx.x];
+        f.th_part[(size_t)blockIdx.x * ADJ_NTH + threadIdx.x] = t;
+    }
 }
 
 __global__ void k_adj_pack(int n, const float *r, const float *v, const int *type, float4 *pos, float4 *vel) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    pos[i] = make_float4(r[3 * i], r[3 * i + 1], r[3 * i + 2], 0.f);
+    pos[i] = make_float4(r[3 * i], r[3 * i + 1], r[3 * i + 2], __int_as_float(type[i]));
     vel[i] = make_float4(v[3 * i], v[3 * i + 1], v[3 * i + 2], 0.f);
-    (void)type;
 }
 
 char g_adj_error[512] = "";
@@ -465,13 +724,18 @@ struct gdb_adj {
     Tables tab{};
     int *d_type = nullptr;
     float *d_mass = nullptr;
-    float4 *d_pos[2] = {nullptr, nullptr}, *d_vel[2] = {nullptr, nullptr};
+    bool keep_all = false;                      // every state is kept (d_seg_*), no checkpoints
+    float4 *d_pos = nullptr, *d_vel = nullptr;  // two states, the forward's when it keeps checkpoints
     float4 *d_ck_pos = nullptr, *d_ck_vel = nullptr;  // checkpoints
-    float4 *d_seg_pos = nullptr, *d_seg_vel = nullptr;  // one recomputed segment
-    double *d_part = nullptr, *d_acc = nullptr;
+    float4 *d_seg_pos = nullptr, *d_seg_vel = nullptr;  // every state, or one recomputed segment
+    int blocks = 0, threads = 0;  // launch shape of the two kernels
+    double n_type0 = 0.0;         // particles of type 0
+    double *d_acc = nullptr;      // [blocks][3]
     unsigned long long *d_bins = nullptr;
-    double *d_R = nullptr, *d_V = nullptr, *d_Vt = nullptr, *d_th = nullptr, *d_gG = nullptr;
-    int *d_nbl = nullptr, *d_nbc = nullptr, *d_flags = nullptr;
+    double *d_R = nullptr, *d_V = nullptr, *d_th = nullptr, *d_gG = nullptr;
+    double4 *d_U = nullptr;
+    int *d_nbl = nullptr, *d_nbc = nullptr;
+    AdjBar *d_bar = nullptr;
     float4 *d_rref = nullptr;
     unsigned *d_status = nullptr;
     int maxnb = 0;
@@ -505,12 +769,11 @@ void adj_free(gdb_adj *h) {
     if (!h) return;
     cudaSetDevice(h->dev);
     if (h->st) cudaStreamSynchronize(h->st);
-    void *ptrs[] = {h->d_type, h->d_mass, h->d_pos[0], h->d_pos[1], h->d_vel[0], h->d_vel[1], h->d_ck_pos,
-                    h->d_ck_vel, h->d_seg_pos, h->d_seg_vel, h->d_part, h->d_acc, h->d_bins, h->d_R,
-                    h->d_V, h->d_Vt, h->d_th, h->d_gG, h->d_nbl, h->d_nbc, h->d_flags, h->d_rref,
-                    h->d_status};
+    void *ptrs[] = {h->d_type, h->d_mass, h->d_pos, h->d_vel, h->d_ck_pos, h->d_ck_vel, h->d_seg_pos, h->d_seg_vel,
+                    h->d_acc, h->d_bins, h->d_R, h->d_V, h->d_U, h->d_th, h->d_gG, h->d_nbl, h->d_nbc, h->d_bar,
+                    h->d_rref, h->d_status};
     for (void *p : ptrs)
-        if (p) cudaFree(p);
+        if (p) cudaFreeAsync(p, h->st);
     if (h->st) cudaStreamDestroy(h->st);
 }
 
@@ -531,36 +794,78 @@ AdjArgs adj_args(const gdb_adj *h) {
     a.nbl = h->d_nbl;
     a.nbc = h->d_nbc;
     a.maxnb = h->maxnb;
-    a.rl2 = h->rl * h->rl;
+    const double ratio = (double)a.dr / (double)a.width;
+    a.step_ratio = exp(-ratio * ratio);
+    const float far = (float)((double)h->r_hi + ADJ_KW * h->width) + ADJ_SKIN;
+    a.far2 = h->nbins > 0 ? far * far : 0.f;
     const float mv = 0.5f * ADJ_SKIN - 0.01f;
     a.move2 = mv * mv;
     a.rref = h->d_rref;
-    a.flags = h->d_flags;
+    a.bar = h->d_bar;
     a.status = h->d_status;
     return a;
 }
 
-int nblocks_of(const gdb_adj *h) { return (h->n + ADJ_PPB - 1) / ADJ_PPB; }
+// Shared copies of the RDF bins: at most 8, within 96 KB.
+int rdf_copies(const gdb_adj *h) {
+    return std::max(1, std::min(8, (int)(96 * 1024 / ((size_t)std::max(h->nbins, 1) * 32 * 8))));
+}
 
-int build_blocks(const gdb_adj *h) { return (h->n * 32 + ADJ_BLOCK - 1) / ADJ_BLOCK; }
+const void *sweep_kernel(const gdb_adj *h) {
+    return h->nt == 1   ? (const void *)k_adj_sweep<1>
+           : h->nt == 2 ? (const void *)k_adj_sweep<2>
+                        : (const void *)k_adj_sweep<ADJ_MAXT>;
+}
 
-// One forward step from buffers (pin, vin) into (pout, vout); step index s.
-// The list is rebuilt first when the previous step flagged it (or `force`);
-// step s flags into slot s & 1, which the build before it clears.
-int forward_step(gdb_adj *h, const float4 *pin, const float4 *vin, float4 *pout, float4 *vout, int s,
-                 bool accumulate, bool force) {
-    const AdjArgs a = adj_args(h);
-    k_adj_build<<<build_blocks(h), ADJ_BLOCK, 0, h->st>>>(a, pin, h->d_nbl, h->d_nbc, force ? 1 : 0, (s + 1) & 1,
-                                                           s & 1);
-    ACK(cudaGetLastError());
-    const bool rdf = accumulate && h->nbins > 0 && h->rdf_every > 0 && s % h->rdf_every == 0;
-    k_adj_step<<<nblocks_of(h), ADJ_BLOCK, 0, h->st>>>(a, h->tab, pin, vin, pout, vout, h->d_part,
-                                                        rdf ? h->d_bins : nullptr, h->d_flags + (s & 1));
-    ACK(cudaGetLastError());
-    if (accumulate) {
-        k_adj_reduce<<<1, 256, 0, h->st>>>(h->d_part, nblocks_of(h), h->d_acc);
-        ACK(cudaGetLastError());
-    }
+// One block per SM at most, of as few warps as give every particle one (more
+// particles than that are taken in turn).
+cudaError_t launch_shape(gdb_adj *h) {
+    int sms = 0;
+    cudaError_t e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->dev);
+    if (e != cudaSuccess) return e;
+    const int warps = std::min(ADJ_WARPS, (h->n + sms - 1) / sms);
+    h->threads = warps * 32;
+    h->blocks = std::min(sms, (h->n + warps - 1) / warps);
+    const int most = 96 * 1024 + ADJ_MAXB * 32 * 8;
+    if ((e = cudaFuncSetAttribute(k_adj_forward, cudaFuncAttributeMaxDynamicSharedMemorySize, most))) return e;
+    return cudaFuncSetAttribute(sweep_kernel(h), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)(ADJ_WARPS * ADJ_RING_BYTES));
+}
+
+// Zero the barrier words and launch one cooperative kernel.
+template <class Args>
+int launch(gdb_adj *h, const void *fn, Args f, size_t smem) {
+    AdjArgs a = adj_args(h);
+    ACK(cudaMemsetAsync(h->d_bar, 0, sizeof(AdjBar), h->st));
+    void *args[] = {&a, &h->tab, &f};
+    ACK(cudaLaunchCooperativeKernel(fn, dim3(h->blocks), dim3(h->threads), args, smem, h->st));
+    return GDB_OK;
+}
+
+// Steps [s0, s0 + n) from state s0 of st; observables into d_acc and d_bins
+// when wanted.
+int run_forward(gdb_adj *h, States st, int s0, int n, bool observe, bool checkpoints) {
+    ForwardArgs f{};
+    f.st = st;
+    f.s0 = s0;
+    f.nsteps = n;
+    f.acc = observe ? h->d_acc : nullptr;
+    f.gbins = observe && h->nbins > 0 && h->rdf_every > 0 ? h->d_bins : nullptr;
+    f.rdf_every = h->rdf_every;
+    f.copies = rdf_copies(h);
+    f.ck_pos = checkpoints ? h->d_ck_pos : nullptr;
+    f.ck_vel = h->d_ck_vel;
+    f.ckpt = h->ckpt;
+    return launch(h, (const void *)k_adj_forward, f,
+                  f.gbins ? (size_t)f.copies * h->nbins * 32 * sizeof(unsigned long long) : 0);
+}
+
+int check_status(gdb_adj *h, const char *who, unsigned status) {
+    if (status & ADJ_STATUS_TIMEOUT)
+        return aset(h, GDB_ERR_TIMEOUT, "%s: a grid barrier wait ran out", who);
+    if (status & ADJ_STATUS_OVERFLOW)
+        return aset(h, GDB_ERR_NBLIST, "%s: a list column outgrew %d entries (reach %.3f)", who,
+                    h->maxnb / ADJ_LANES, h->rl);
     return GDB_OK;
 }
 
@@ -578,18 +883,17 @@ int ensure_list(gdb_adj *h) {
     const int rows = std::min((int)(2.0 * mean / ADJ_LANES) + 8, (h->n + ADJ_LANES - 1) / ADJ_LANES);
     const int want = rows * ADJ_LANES;
     if (want > h->maxnb || !h->d_nbl) {
-        if (h->d_nbl) cudaFree(h->d_nbl);
+        if (h->d_nbl) ACK(cudaFreeAsync(h->d_nbl, h->st));
         h->d_nbl = nullptr;
-        ACK(cudaMalloc(&h->d_nbl, (size_t)h->n * want * sizeof(int)));
+        ACK(gdb::pool_alloc(&h->d_nbl, (size_t)h->n * want * sizeof(int), h->st));
         h->maxnb = want;
     }
     if (!h->d_nbc) {
-        ACK(cudaMalloc(&h->d_nbc, (size_t)h->n * ADJ_LANES * sizeof(int)));
-        ACK(cudaMalloc(&h->d_rref, h->n * sizeof(float4)));
-        ACK(cudaMalloc(&h->d_flags, 2 * sizeof(int)));
-        ACK(cudaMalloc(&h->d_status, sizeof(unsigned)));
+        ACK(gdb::pool_alloc(&h->d_nbc, (size_t)h->n * ADJ_LANES * sizeof(int), h->st));
+        ACK(gdb::pool_alloc(&h->d_rref, h->n * sizeof(float4), h->st));
+        ACK(gdb::pool_alloc(&h->d_bar, sizeof(AdjBar), h->st));
+        ACK(gdb::pool_alloc(&h->d_status, sizeof(unsigned), h->st));
     }
-    ACK(cudaMemsetAsync(h->d_flags, 0, 2 * sizeof(int), h->st));
     ACK(cudaMemsetAsync(h->d_status, 0, sizeof(unsigned), h->st));
     return GDB_OK;
 }
@@ -614,10 +918,13 @@ void build_tables(gdb_adj *h, const double *params) {
         e.cut = (float)cut;
         e.cut2 = (float)cut * (float)cut;
         Tab64 &d = T.t64[k];
-        d.sig = sig;
+        d.sig2 = sig * sig;
         d.eps = eps;
+        d.ieps = 1.0 / eps;
+        d.eps_sig = eps / sig;
         d.cut = cut;
-        d.cut2 = (double)e.cut2;
+        d.cut2 = e.cut2;
+        d.reach2 = ((float)cut + ADJ_SKIN) * ((float)cut + ADJ_SKIN);
         d.s_c = sc;
         d.dsds_c = eps * (576.0 * sr12 - 144.0 * sr6) / (cut * cut) / sig;
         d.u_c = uc;
@@ -638,19 +945,21 @@ int gdb_adj_create(int n, int ntypes, int device, gdb_adj **out) {
     h->n = n;
     h->nt = ntypes;
     h->dev = device;
+    // device memory comes from the library's stream-ordered pool: mapping the
+    // kept states anew for every handle took 3.6 ms (N 4096, 51 states)
     cudaError_t e;
     if ((e = cudaSetDevice(device)) != cudaSuccess || (e = cudaStreamCreateWithFlags(&h->st, cudaStreamNonBlocking)) ||
-        (e = cudaMalloc(&h->d_type, n * sizeof(int))) || (e = cudaMalloc(&h->d_mass, n * sizeof(float))) ||
-        (e = cudaMalloc(&h->d_pos[0], n * sizeof(float4))) || (e = cudaMalloc(&h->d_pos[1], n * sizeof(float4))) ||
-        (e = cudaMalloc(&h->d_vel[0], n * sizeof(float4))) || (e = cudaMalloc(&h->d_vel[1], n * sizeof(float4))) ||
-        (e = cudaMalloc(&h->d_part, (size_t)((n + ADJ_PPB - 1) / ADJ_PPB) * 3 * sizeof(double))) ||
-        (e = cudaMalloc(&h->d_acc, 3 * sizeof(double))) ||
-        (e = cudaMalloc(&h->d_bins, ADJ_MAXB * sizeof(unsigned long long))) ||
-        (e = cudaMalloc(&h->d_R, (size_t)n * 3 * sizeof(double))) ||
-        (e = cudaMalloc(&h->d_V, (size_t)n * 3 * sizeof(double))) ||
-        (e = cudaMalloc(&h->d_Vt, (size_t)n * 3 * sizeof(double))) ||
-        (e = cudaMalloc(&h->d_th, (size_t)((n + ADJ_PPB - 1) / ADJ_PPB) * ADJ_NTH * sizeof(double))) ||
-        (e = cudaMalloc(&h->d_gG, ADJ_MAXB * sizeof(double)))) {
+        (e = gdb::pool_alloc(&h->d_type, n * sizeof(int), h->st)) ||
+        (e = gdb::pool_alloc(&h->d_mass, n * sizeof(float), h->st)) ||
+        (e = launch_shape(h)) || (e = gdb::pool_alloc(&h->d_pos, (size_t)2 * n * sizeof(float4), h->st)) ||
+        (e = gdb::pool_alloc(&h->d_vel, (size_t)2 * n * sizeof(float4), h->st)) ||
+        (e = gdb::pool_alloc(&h->d_acc, (size_t)h->blocks * 3 * sizeof(double), h->st)) ||
+        (e = gdb::pool_alloc(&h->d_bins, ADJ_MAXB * sizeof(unsigned long long), h->st)) ||
+        (e = gdb::pool_alloc(&h->d_R, (size_t)n * 3 * sizeof(double), h->st)) ||
+        (e = gdb::pool_alloc(&h->d_V, (size_t)n * 3 * sizeof(double), h->st)) ||
+        (e = gdb::pool_alloc(&h->d_U, (size_t)2 * n * sizeof(double4), h->st)) ||
+        (e = gdb::pool_alloc(&h->d_th, (size_t)h->blocks * (1 + h->threads / 32) * ADJ_NTH * sizeof(double), h->st)) ||
+        (e = gdb::pool_alloc(&h->d_gG, ADJ_MAXB * sizeof(double), h->st))) {
         adj_free(h);
         delete h;
         return aset(nullptr, GDB_ERR_CUDA, "gdb_adj_create: %s", cudaGetErrorString(e));
@@ -689,16 +998,30 @@ int gdb_adj_setup(gdb_adj *h, const float box[3], const int32_t *ptype, const fl
     h->rdf_every = rdf_every;
     ACK(cudaMemcpyAsync(h->d_type, ptype, h->n * sizeof(int), cudaMemcpyHostToDevice, h->st));
     ACK(cudaMemcpyAsync(h->d_mass, mass, h->n * sizeof(float), cudaMemcpyHostToDevice, h->st));
-    const int nck = (steps + checkpoint_every - 1) / checkpoint_every;
-    if (h->d_ck_pos) cudaFree(h->d_ck_pos);
-    if (h->d_ck_vel) cudaFree(h->d_ck_vel);
-    if (h->d_seg_pos) cudaFree(h->d_seg_pos);
-    if (h->d_seg_vel) cudaFree(h->d_seg_vel);
-    h->d_ck_pos = h->d_ck_vel = h->d_seg_pos = h->d_seg_vel = nullptr;
-    ACK(cudaMalloc(&h->d_ck_pos, (size_t)nck * h->n * sizeof(float4)));
-    ACK(cudaMalloc(&h->d_ck_vel, (size_t)nck * h->n * sizeof(float4)));
-    ACK(cudaMalloc(&h->d_seg_pos, (size_t)(checkpoint_every + 1) * h->n * sizeof(float4)));
-    ACK(cudaMalloc(&h->d_seg_vel, (size_t)(checkpoint_every + 1) * h->n * sizeof(float4)));
+    h->n_type0 = (double)std::count(ptype, ptype + h->n, 0);
+    for (float4 **p : {&h->d_ck_pos, &h->d_ck_vel, &h->d_seg_pos, &h->d_seg_vel}) {
+        if (*p) ACK(cudaFreeAsync(*p, h->st));
+        *p = nullptr;
+    }
+    // every state, or checkpoints and one segment where they would need more
+    // than ADJ_KEEP_BYTES (or the memory is not there)
+    const size_t all = (size_t)(steps + 1) * h->n * sizeof(float4);
+    const char *keep = getenv("GDB_ADJ_KEEP_BYTES");
+    h->keep_all = 2 * all <= (keep && *keep ? (size_t)std::max(0LL, atoll(keep)) : ADJ_KEEP_BYTES);
+    if (h->keep_all && (gdb::pool_alloc(&h->d_seg_pos, all, h->st) != cudaSuccess ||
+                        gdb::pool_alloc(&h->d_seg_vel, all, h->st) != cudaSuccess)) {
+        (void)cudaGetLastError();
+        if (h->d_seg_pos) cudaFreeAsync(h->d_seg_pos, h->st);
+        h->d_seg_pos = h->d_seg_vel = nullptr;
+        h->keep_all = false;
+    }
+    if (!h->keep_all) {
+        const int nck = (steps + checkpoint_every - 1) / checkpoint_every;
+        ACK(gdb::pool_alloc(&h->d_ck_pos, (size_t)nck * h->n * sizeof(float4), h->st));
+        ACK(gdb::pool_alloc(&h->d_ck_vel, (size_t)nck * h->n * sizeof(float4), h->st));
+        ACK(gdb::pool_alloc(&h->d_seg_pos, (size_t)(checkpoint_every + 1) * h->n * sizeof(float4), h->st));
+        ACK(gdb::pool_alloc(&h->d_seg_vel, (size_t)(checkpoint_every + 1) * h->n * sizeof(float4), h->st));
+    }
     ACK(cudaStreamSynchronize(h->st));
     h->setup = true;
     h->forward_done = false;
@@ -725,42 +1048,30 @@ int gdb_adj_forward(gdb_adj *h, const double *params, const float *r0, const flo
     ACK(gdb::pool_alloc(&dv, (size_t)n * 3 * sizeof(float), h->st));
     ACK(cudaMemcpyAsync(dr, r0, (size_t)n * 3 * sizeof(float), cudaMemcpyHostToDevice, h->st));
     ACK(cudaMemcpyAsync(dv, v0, (size_t)n * 3 * sizeof(float), cudaMemcpyHostToDevice, h->st));
-    k_adj_pack<<<(n + 255) / 256, 256, 0, h->st>>>(n, dr, dv, h->d_type, h->d_pos[0], h->d_vel[0]);
+    float4 *p0 = h->keep_all ? h->d_seg_pos : h->d_pos, *v0d = h->keep_all ? h->d_seg_vel : h->d_vel;
+    k_adj_pack<<<(n + 255) / 256, 256, 0, h->st>>>(n, dr, dv, h->d_type, p0, v0d);
     ACK(cudaGetLastError());
     ACK(cudaFreeAsync(dr, h->st));
     ACK(cudaFreeAsync(dv, h->st));
-    ACK(cudaMemsetAsync(h->d_acc, 0, 3 * sizeof(double), h->st));
     ACK(cudaMemsetAsync(h->d_bins, 0, ADJ_MAXB * sizeof(unsigned long long), h->st));
-    int cur = 0;
-    h->nsamples = 0;
-    for (int s = 0; s < h->steps; s++) {
-        if (s % h->ckpt == 0) {
-            const size_t off = (size_t)(s / h->ckpt) * n;
-            ACK(cudaMemcpyAsync(h->d_ck_pos + off, h->d_pos[cur], n * sizeof(float4), cudaMemcpyDeviceToDevice, h->st));
-            ACK(cudaMemcpyAsync(h->d_ck_vel + off, h->d_vel[cur], n * sizeof(float4), cudaMemcpyDeviceToDevice, h->st));
-        }
-        rc = forward_step(h, h->d_pos[cur], h->d_vel[cur], h->d_pos[cur ^ 1], h->d_vel[cur ^ 1], s, true, s == 0);
-        if (rc) return rc;
-        if (h->nbins > 0 && h->rdf_every > 0 && s % h->rdf_every == 0) h->nsamples++;
-        cur ^= 1;
-    }
-    double acc[3];
+    rc = run_forward(h, States{p0, v0d, 0, h->keep_all ? h->steps + 1 : 2}, 0, h->steps, true, !h->keep_all);
+    if (rc) return rc;
+    h->nsamples = h->nbins > 0 && h->rdf_every > 0 ? (h->steps + h->rdf_every - 1) / h->rdf_every : 0;
+    std::vector<double> acc((size_t)h->blocks * 3);
     std::vector<unsigned long long> bins(ADJ_MAXB);
-    ACK(cudaMemcpyAsync(acc, h->d_acc, sizeof(acc), cudaMemcpyDeviceToHost, h->st));
+    ACK(cudaMemcpyAsync(acc.data(), h->d_acc, acc.size() * sizeof(double), cudaMemcpyDeviceToHost, h->st));
     ACK(cudaMemcpyAsync(bins.data(), h->d_bins, ADJ_MAXB * sizeof(unsigned long long), cudaMemcpyDeviceToHost, h->st));
     unsigned status = 0;
     ACK(cudaMemcpyAsync(&status, h->d_status, sizeof(unsigned), cudaMemcpyDeviceToHost, h->st));
     ACK(cudaStreamSynchronize(h->st));
-    if (status & ADJ_STATUS_OVERFLOW)
-        return aset(h, GDB_ERR_NBLIST, "gdb_adj_forward: a list column outgrew %d entries (reach %.3f)",
-                    h->maxnb / ADJ_LANES, h->rl);
+    if ((rc = check_status(h, "gdb_adj_forward", status))) return rc;
     h->obs.assign(3 + h->nbins, 0.0);
-    for (int q = 0; q < 3; q++) h->obs[q] = acc[q] / h->steps;
+    for (int b = 0; b < h->blocks; b++)
+        for (int q = 0; q < 3; q++) h->obs[q] += acc[(size_t)b * 3 + q];
+    for (int q = 0; q < 3; q++) h->obs[q] /= h->steps;
     if (h->nbins > 0 && h->nsamples > 0) {
         // g_b = sum K / (samples * N_A * rho_A * 4 pi r_b^2)
-        std::vector<int> types(n);
-        ACK(cudaMemcpy(types.data(), h->d_type, n * sizeof(int), cudaMemcpyDeviceToHost));
-        const double na = (double)std::count(types.begin(), types.end(), 0);
+        const double na = h->n_type0;
         const double vol = (double)h->box[0] * h->box[1] * h->box[2];
         const double dr_ = (double)(h->r_hi - h->r_lo) / h->nbins;
         for (int b = 0; b < h->nbins; b++) {
@@ -784,72 +1095,56 @@ int gdb_adj_backward(gdb_adj *h, const double *grad_obs, double *grad_params) {
     std::vector<double> gG(ADJ_MAXB, 0.0);
     bool any_g = false;
     if (h->nbins > 0 && h->nsamples > 0) {
-        std::vector<int> types(n);
-        ACK(cudaMemcpy(types.data(), h->d_type, n * sizeof(int), cudaMemcpyDeviceToHost));
-        const double na = (double)std::count(types.begin(), types.end(), 0);
+        const double na = h->n_type0;
         const double vol = (double)h->box[0] * h->box[1] * h->box[2];
         const double dr_ = (double)(h->r_hi - h->r_lo) / h->nbins;
+        const double w = h->width;
         for (int b = 0; b < h->nbins; b++) {
             const double rb = h->r_lo + (b + 0.5) * dr_;
-            gG[b] = grad_obs[3 + b] / (h->nsamples * na * (na / vol) * 4.0 * M_PI * rb * rb);
-            any_g |= gG[b] != 0.0;
+            const double g = grad_obs[3 + b] / (h->nsamples * na * (na / vol) * 4.0 * M_PI * rb * rb);
+            any_g |= g != 0.0;
+            gG[b] = g * 2.0 * (-1.0 / (w * w)) / (sqrt(2.0 * M_PI) * w);
         }
         ACK(cudaMemcpyAsync(h->d_gG, gG.data(), ADJ_MAXB * sizeof(double), cudaMemcpyHostToDevice, h->st));
     }
-    const int nb = nblocks_of(h);
+    const int nb = h->blocks;
     ACK(cudaMemsetAsync(h->d_R, 0, (size_t)n * 3 * sizeof(double), h->st));
     ACK(cudaMemsetAsync(h->d_V, 0, (size_t)n * 3 * sizeof(double), h->st));
-    ACK(cudaMemsetAsync(h->d_th, 0, (size_t)nb * ADJ_NTH * sizeof(double), h->st));
-    const AdjArgs a = adj_args(h);
-    const int nseg = (T + h->ckpt - 1) / h->ckpt;
-    for (int sg = nseg - 1; sg >= 0; sg--) {
-        const int s0 = sg * h->ckpt, len = std::min(h->ckpt, T - s0);
-        // recompute the segment's states (bit-identical to the forward)
-        const size_t off = (size_t)sg * n;
-        ACK(cudaMemcpyAsync(h->d_seg_pos, h->d_ck_pos + off, n * sizeof(float4), cudaMemcpyDeviceToDevice, h->st));
-        ACK(cudaMemcpyAsync(h->d_seg_vel, h->d_ck_vel + off, n * sizeof(float4), cudaMemcpyDeviceToDevice, h->st));
-        for (int k = 0; k < len; k++) {
-            int rc = forward_step(h, h->d_seg_pos + (size_t)k * n, h->d_seg_vel + (size_t)k * n,
-                                  h->d_seg_pos + (size_t)(k + 1) * n, h->d_seg_vel + (size_t)(k + 1) * n, s0 + k,
-                                  false, k == 0);
-            if (rc) return rc;
+    SweepArgs f{};
+    f.gU = gU;
+    f.gW = gW;
+    f.gK = gK;
+    f.gG = any_g ? h->d_gG : nullptr;
+    f.rdf_every = h->rdf_every;
+    f.window = h->window;
+    f.R = h->d_R;
+    f.V = h->d_V;
+    f.U = h->d_U;
+    f.th_part = h->d_th;
+    f.th_warp = h->d_th + (size_t)nb * ADJ_NTH;
+    const int seg = h->keep_all ? T : h->ckpt;
+    for (int sg = (T + seg - 1) / seg - 1; sg >= 0; sg--) {
+        const int s0 = sg * seg, len = std::min(seg, T - s0);
+        f.st = States{h->d_seg_pos, h->d_seg_vel, s0, len + 1};
+        f.s0 = s0;
+        f.len = len;
+        f.first_segment = s0 + len == T;
+        f.last_segment = sg == 0;
+        int rc;
+        if (!h->keep_all) {  // recompute the segment's states (bit-identical to the forward)
+            const size_t off = (size_t)sg * n;
+            ACK(cudaMemcpyAsync(h->d_seg_pos, h->d_ck_pos + off, n * sizeof(float4), cudaMemcpyDeviceToDevice, h->st));
+            ACK(cudaMemcpyAsync(h->d_seg_vel, h->d_ck_vel + off, n * sizeof(float4), cudaMemcpyDeviceToDevice, h->st));
+            if ((rc = run_forward(h, f.st, s0, len, false, false))) return rc;
         }
-        // reverse sweep of the segment; the list follows the positions
-        // backwards (check -> gated build), slots by step parity
-        ACK(cudaMemsetAsync(h->d_flags, 0, 2 * sizeof(int), h->st));
-        for (int k = len - 1; k >= 0; k--) {
-            const int s = s0 + k;
-            {
-                const float4 *pk = h->d_seg_pos + (size_t)k * n;
-                k_adj_check<<<(n + 255) / 256, 256, 0, h->st>>>(a, pk, s & 1);
-                ACK(cudaGetLastError());
-                k_adj_build<<<build_blocks(h), ADJ_BLOCK, 0, h->st>>>(a, pk, h->d_nbl, h->d_nbc, k == len - 1 ? 1 : 0,
-                                                                       s & 1, (s + 1) & 1);
-                ACK(cudaGetLastError());
-            }
-            if (h->window > 0 && (s + 1) % h->window == 0) {
-                // last step of a window: nothing flows back across its end
-                ACK(cudaMemsetAsync(h->d_R, 0, (size_t)n * 3 * sizeof(double), h->st));
-                ACK(cudaMemsetAsync(h->d_V, 0, (size_t)n * 3 * sizeof(double), h->st));
-            }
-            const float4 *pn = h->d_seg_pos + (size_t)k * n;
-            const float4 *vn = h->d_seg_vel + (size_t)k * n, *vn1 = h->d_seg_vel + (size_t)(k + 1) * n;
-            k_adj_vtot<<<(n + 255) / 256, 256, 0, h->st>>>(n, h->dt, gK, h->d_mass, h->d_R, h->d_V, vn, vn1, h->d_Vt);
-            ACK(cudaGetLastError());
-            const bool rdf = any_g && h->rdf_every > 0 && s % h->rdf_every == 0;
-            k_adj_back<<<nb, ADJ_BLOCK, 0, h->st>>>(a, h->tab, pn, h->d_Vt, h->d_R, h->d_V, vn, vn1, gU, gW, gK,
-                                                     rdf ? h->d_gG : nullptr, h->d_th);
-            ACK(cudaGetLastError());
-        }
+        if ((rc = launch(h, sweep_kernel(h), f, h->threads / 32 * ADJ_RING_BYTES))) return rc;
     }
     std::vector<double> th((size_t)nb * ADJ_NTH);
     unsigned status = 0;
     ACK(cudaMemcpyAsync(th.data(), h->d_th, th.size() * sizeof(double), cudaMemcpyDeviceToHost, h->st));
     ACK(cudaMemcpyAsync(&status, h->d_status, sizeof(unsigned), cudaMemcpyDeviceToHost, h->st));
     ACK(cudaStreamSynchronize(h->st));
-    if (status & ADJ_STATUS_OVERFLOW)
-        return aset(h, GDB_ERR_NBLIST, "gdb_adj_backward: a list column outgrew %d entries (reach %.3f)",
-                    h->maxnb / ADJ_LANES, h->rl);
+    if (int rc = check_status(h, "gdb_adj_backward", status)) return rc;
     // fixed-order sum over blocks; a parameter of the unordered pair {a, b}
     // collects the (a, b) and (b, a) entries
     const int nt = h->nt;
@@ -877,10 +1172,10 @@ int gdb_adj_set_window(gdb_adj *h, int window) {
 int gdb_adj_final_state(gdb_adj *h, float *r, float *v) {
     if (!h || !h->forward_done) return aset(h, GDB_ERR_STATE, "gdb_adj_final_state: no forward run");
     ACK(cudaSetDevice(h->dev));
-    const int cur = h->steps & 1;
+    const size_t last = (size_t)(h->keep_all ? h->steps : h->steps & 1) * h->n;
     std::vector<float4> p(h->n), q(h->n);
-    ACK(cudaMemcpy(p.data(), h->d_pos[cur], h->n * sizeof(float4), cudaMemcpyDeviceToHost));
-    ACK(cudaMemcpy(q.data(), h->d_vel[cur], h->n * sizeof(float4), cudaMemcpyDeviceToHost));
+    ACK(cudaMemcpy(p.data(), (h->keep_all ? h->d_seg_pos : h->d_pos) + last, h->n * sizeof(float4), cudaMemcpyDeviceToHost));
+    ACK(cudaMemcpy(q.data(), (h->keep_all ? h->d_seg_vel : h->d_vel) + last, h->n * sizeof(float4), cudaMemcpyDeviceToHost));
     for (int i = 0; i < h->n; i++) {
         if (r) {
             r[3 * i] = p[i].x;

@@ -1,9 +1,9 @@
-"""Routes of the analyses that depend on sizes: S(q) by runs of q-vectors or one by one, the RDF's rows of
-cells."""
+"""Routes of the analyses and the adjoint that depend on sizes or memory: S(q) by runs of q-vectors or one by
+one, the RDF's rows of cells, the adjoint with every state kept or recomputed from checkpoints."""
 import numpy as np
 import pytest
 
-from gamdpy_b200 import _lib
+from gamdpy_b200 import _lib, adjoint, workloads
 
 pytestmark = pytest.mark.gpu
 
@@ -77,3 +77,21 @@ def test_rdf_coordinates_on_the_faces(oracle, axis):
     pt = rng.integers(0, 2, 4000).astype(np.int32)
     got = _lib.rdf_compute(r, pt, L, 2, 100, r_max=3.1)
     assert np.array_equal(got, oracle.rdf(r, pt, L, 100, fma=1, r_max=3.1)) and got.sum() > 0
+
+
+@pytest.mark.parametrize("n,every", [(256, 7), (301, 40), (700, 1)])
+def test_adjoint_kept_states_equal_checkpoints(monkeypatch, n, every):
+    """Every state kept against segments recomputed from checkpoints: the same numbers, bit for bit."""
+    conf = workloads.ka_configuration(n, rho=1.2 if n > 256 else 0.4, temperature=0.6, seed=n)
+    cut = np.minimum(workloads.KA_CUT, 0.49 * float(conf.simbox.lengths.min()))
+    rdf = {"bins": 12, "r_lo": 0.7, "r_hi": 1.9, "width": 0.1, "every": 3}
+    theta = adjoint.theta_from_tables(workloads.KA_SIGMA, workloads.KA_EPSILON)
+    out = []
+    for keep in (None, "0"):
+        if keep is not None:
+            monkeypatch.setenv("GDB_ADJ_KEEP_BYTES", keep)
+        eng = adjoint.AdjointNVE(conf, cut, dt=0.004, steps=23, checkpoint_every=every, rdf=rdf)
+        obs = eng.forward(theta)
+        out.append((obs, eng.backward(np.linspace(0.5, 1.5, len(obs))), *eng.final_state()))
+    for a, b in zip(*out):
+        assert np.isfinite(a).all() and np.array_equal(a, b)
