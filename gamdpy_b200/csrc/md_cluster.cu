@@ -105,7 +105,7 @@ __global__ void __launch_bounds__(CL_THREADS, 1) k_cluster_run(const ClusterJob 
     }
     int maxcount = 0, nbuild = 0;
     const float Lx = a.Lx, Ly = a.Ly, Lz = a.Lz;
-    const float ilx = 1.0f / Lx, ily = 1.0f / Ly, ilz = 1.0f / Lz;
+    const PairBox box(Lx, Ly, Lz);
     // cluster-wide maximum of a per-thread value (called by every thread)
     auto cluster_max = [&](int val) -> int {
         val = __reduce_max_sync(0xffffffffu, val);
@@ -381,15 +381,15 @@ __global__ void __launch_bounds__(CL_THREADS, 1) k_cluster_run(const ClusterJob 
                 const float4 q2 = spos[v2 ? jj.z : i];
                 const float4 q3 = spos[v3 ? jj.w : i];
                 if (rec) {
-                    pair_force<true, NT>(pr, pi, q0, true, Lx, Ly, Lz, ilx, ily, ilz, fx, fy, fz, u, w, l);
-                    pair_force<true, NT>(pr, pi, q1, v1, Lx, Ly, Lz, ilx, ily, ilz, fx, fy, fz, u, w, l);
-                    pair_force<true, NT>(pr, pi, q2, v2, Lx, Ly, Lz, ilx, ily, ilz, fx, fy, fz, u, w, l);
-                    pair_force<true, NT>(pr, pi, q3, v3, Lx, Ly, Lz, ilx, ily, ilz, fx, fy, fz, u, w, l);
+                    pair_force<true, NT>(pr, box, pi, q0, true, fx, fy, fz, u, w, l);
+                    pair_force<true, NT>(pr, box, pi, q1, v1, fx, fy, fz, u, w, l);
+                    pair_force<true, NT>(pr, box, pi, q2, v2, fx, fy, fz, u, w, l);
+                    pair_force<true, NT>(pr, box, pi, q3, v3, fx, fy, fz, u, w, l);
                 } else {
-                    pair_force<false, NT>(pr, pi, q0, true, Lx, Ly, Lz, ilx, ily, ilz, fx, fy, fz, u, w, l);
-                    pair_force<false, NT>(pr, pi, q1, v1, Lx, Ly, Lz, ilx, ily, ilz, fx, fy, fz, u, w, l);
-                    pair_force<false, NT>(pr, pi, q2, v2, Lx, Ly, Lz, ilx, ily, ilz, fx, fy, fz, u, w, l);
-                    pair_force<false, NT>(pr, pi, q3, v3, Lx, Ly, Lz, ilx, ily, ilz, fx, fy, fz, u, w, l);
+                    pair_force<false, NT>(pr, box, pi, q0, true, fx, fy, fz, u, w, l);
+                    pair_force<false, NT>(pr, box, pi, q1, v1, fx, fy, fz, u, w, l);
+                    pair_force<false, NT>(pr, box, pi, q2, v2, fx, fy, fz, u, w, l);
+                    pair_force<false, NT>(pr, box, pi, q3, v3, fx, fy, fz, u, w, l);
                 }
             }
         }
