@@ -12,9 +12,9 @@
 //   * steps are separated by hardware cluster barriers -- one per step when
 //     two position copies fit (new positions go straight into every CTA's
 //     other copy), two otherwise; the per-CTA float64 partial sums (only
-//     those a step needs) are read by every CTA from the others' shared
-//     memory in a fixed order, so every CTA computes the same thermostat
-//     update, flags and sums without another round trip.
+//     those a step needs) are sent to every CTA's shared memory before the
+//     barrier and added there in a fixed order, so every CTA computes the same
+//     thermostat update, flags and sums without another round trip.
 // Global memory is read at the start of a timeblock and written at its end
 // (plus ScalarSaver rows and ConfigurationSaver frames).  Lists are built in
 // shared memory over the cell grid of the global cell build (counting sort of
@@ -43,15 +43,20 @@ __global__ void __launch_bounds__(CL_THREADS, 1) k_cluster_run(const ClusterJob 
     __shared__ double s_red[NQ * 32];
     __shared__ int s_flag[4];
     __shared__ double s_lmax;
-    __shared__ double s_gather[16][CL_NQ];
+    __shared__ int s_max[16];
+    __shared__ double s_gather[2][16][CL_NQ];  // every CTA's partial sums, by step parity
+    __shared__ SimArgs s_a;                    // the arguments of this cluster's system
     __shared__ int s_seg_lo[CL_THREADS / 32][64];
     __shared__ int s_seg_pre[CL_THREADS / 32][64];
     cg::cluster_group cl = cg::this_cluster();
     const int C = (int)cl.num_blocks();
     const int rank = (int)cl.block_rank();
     const ClusterJob &job = jobs[blockIdx.x / C];
-    const SimArgs &a = job.a;
+    if (threadIdx.x == 0) s_a = job.a;
+    __syncthreads();
+    const SimArgs &a = s_a;
     DevCtrl *ctrl = a.ctrl;
+    const double time_zero = ctrl->time_zero;
     const int n = a.n;
     const int P = (n + C - 1) / C;
     const int ncx = a.ncx, ncy = a.ncy, ncz = a.ncz;
@@ -72,7 +77,6 @@ __global__ void __launch_bounds__(CL_THREADS, 1) k_cluster_run(const ClusterJob 
     float4 *ssort = reinterpret_cast<float4 *>(smem + L.sorted);
     unsigned short *snbl = reinterpret_cast<unsigned short *>(smem + L.nbl);
     int *snbc = reinterpret_cast<int *>(smem + L.nbc);
-    double *spart = reinterpret_cast<double *>(smem + L.part);
     double *stot = reinterpret_cast<double *>(smem + L.tot);
     const int tid = threadIdx.x, lane = tid & 31;
     const int p0 = rank * P;
@@ -115,11 +119,11 @@ __global__ void __launch_bounds__(CL_THREADS, 1) k_cluster_run(const ClusterJob 
         __syncthreads();
         if (tid == 0) s_lmax = (double)s_flag[0];
         cl.sync();
-        if (tid < C) s_gather[tid][0] = *cl.map_shared_rank(&s_lmax, tid);
+        if (tid < C) s_max[tid] = (int)*cl.map_shared_rank(&s_lmax, tid);
         __syncthreads();
         if (tid == 0) {
             int m = 0;
-            for (int r = 0; r < C; r++) m = max(m, (int)s_gather[r][0]);
+            for (int r = 0; r < C; r++) m = max(m, s_max[r]);
             s_flag[1] = m;
         }
         __syncthreads();
@@ -310,24 +314,43 @@ __global__ void __launch_bounds__(CL_THREADS, 1) k_cluster_run(const ClusterJob 
                     lmax = max(lmax, count);
                 }
             } else {
+                // N^2: lane L tests j = 32 r + L and sets bit r of its mask;
+                // n <= CL_NSQ_MAX < 1024 candidates fit the masks, or they
+                // are filled again (sparse grids); then the lanes' hits are
+                // appended lane by lane
+                const float cps2 = a.cps2;
+                const bool fma = a.fma != 0;
                 for (int q = tid >> 5; q < np; q += CL_THREADS / 32) {
                     const int ii = p0 + q;
                     const float4 pi = spos[ii];
                     int count = 0;
-                    for (int j0 = 0; j0 < n; j0 += 32) {
-                        const int j = j0 + lane;
-                        bool hit = false;
-                        if (j < n && j != ii) {
-                            const float d2 = a.fma ? dist_sq_exact<true>(spos[j], pi, Lx, Ly, Lz)
-                                                   : dist_sq_exact<false>(spos[j], pi, Lx, Ly, Lz);
-                            hit = d2 < a.cps2;
+                    for (int j0 = 0; j0 < n; j0 += 1024) {
+                        unsigned mask = 0;
+                        const int own = min(32, max(0, (n - j0 - lane + 31) >> 5));  // this lane's candidates
+#pragma unroll 4
+                        for (int r = 0; r < own; r++) {
+                            const float4 pj = spos[j0 + 32 * r + lane];
+                            const float d2 = fma ? dist_sq_exact<true>(pj, pi, Lx, Ly, Lz)
+                                                 : dist_sq_exact<false>(pj, pi, Lx, Ly, Lz);
+                            if (d2 < cps2) mask |= 1u << r;
                         }
-                        const unsigned m = __ballot_sync(0xffffffffu, hit);
-                        if (hit) {
-                            const int k = count + __popc(m & ((1u << lane) - 1u));
+                        __syncwarp();
+                        if ((unsigned)(ii - j0) < 1024u && ((ii - j0) & 31) == lane) mask &= ~(1u << ((ii - j0) >> 5));
+                        const int mine = __popc(mask);
+                        int incl = mine;
+#pragma unroll
+                        for (int o = 1; o < 32; o <<= 1) {
+                            const int y = __shfl_up_sync(0xffffffffu, incl, o);
+                            if (lane >= o) incl += y;
+                        }
+                        int k = count + incl - mine;
+                        while (mask) {
+                            const int j = j0 + 32 * (__ffs(mask) - 1) + lane;
+                            mask &= mask - 1u;
                             if (k < cap && k < a.max_nbs) snbl[cl_nbl_index(q, k, P)] = (unsigned short)j;
+                            k++;
                         }
-                        count += __popc(m);
+                        count += __shfl_sync(0xffffffffu, incl, 31);
                     }
                     if (lane == 0) snbc[q] = count;
                     lmax = max(lmax, count);
@@ -489,7 +512,6 @@ __global__ void __launch_bounds__(CL_THREADS, 1) k_cluster_run(const ClusterJob 
         // thermostat (NVT) otherwise, and always the rebuild flag
         const bool full = rec || reset;
         const bool needk = full || INTEG == GDB_INTEGRATOR_NVT;
-        double *slot = spart + (pp ? (s & 1) : 0) * CL_NQ;
         const int any_moved = __syncthreads_or(moved);  // also orders snew before the copies below
         if (full) {
             block_sum<NQ>(red, s_red);
@@ -498,14 +520,21 @@ __global__ void __launch_bounds__(CL_THREADS, 1) k_cluster_run(const ClusterJob 
             block_sum<1>(rk, s_red);
             red[0] = rk[0];
         }
-        if (tid == 0) {
+        // lane r of the first warp (every lane of which holds the sums) sends
+        // them to CTA r, so that after the barrier they are local (measured on
+        // B200, KA N 512, us per step: 7.1 with remote reads after the
+        // barrier, the arguments in global memory and a ballot per round of
+        // the list build, 5.5 here)
+        double (*gather)[CL_NQ] = s_gather[s & 1];
+        if (tid < C) {
+            double *dst = cl.map_shared_rank(&gather[rank][0], tid);
             if (full) {
 #pragma unroll
-                for (int q = 0; q < NQ; q++) slot[q] = red[q];
+                for (int q = 0; q < NQ; q++) dst[q] = red[q];
             } else if (needk) {
-                slot[0] = red[0];
+                dst[0] = red[0];
             }
-            slot[NQ] = any_moved ? 1.0 : 0.0;
+            dst[NQ] = any_moved ? 1.0 : 0.0;
         }
         // with two position copies, the new positions go straight into every
         // CTA's other copy, read only after the barrier below
@@ -523,26 +552,27 @@ __global__ void __launch_bounds__(CL_THREADS, 1) k_cluster_run(const ClusterJob 
                 cl.map_shared_rank(spos, r)[p0 + q] = snew[q];
             }
         }
-        // the needed partials of every CTA, one remote load per thread, then
-        // a fixed-order local sum
-        const int ng = full ? NQ + 1 : (needk ? 2 : 1);
-        if (tid < C * ng) {
-            const int r = tid / ng, g = tid - r * ng;
-            const int q = full ? g : (g == ng - 1 ? NQ : 0);
-            s_gather[r][q] = cl.map_shared_rank(slot, r)[q];
+        // fixed-order sums over the CTAs: every thread takes the kinetic energy
+        // and the flag itself; the other columns (saved and reset steps) are
+        // summed by a thread each
+        double sum_k = 0.0, sum_moved = 0.0;
+        for (int r = 0; r < C; r++) {
+            if (needk) sum_k += gather[r][0];
+            sum_moved += gather[r][NQ];
         }
-        __syncthreads();
-        if (tid < NQ + 1 && (full || tid == NQ || (needk && tid == 0))) {
-            double acc = 0.0;
-            for (int r = 0; r < C; r++) acc += s_gather[r][tid];
-            stot[tid] = acc;
+        if (full) {
+            if (tid < NQ) {
+                double acc = 0.0;
+                for (int r = 0; r < C; r++) acc += gather[r][tid];
+                stot[tid] = acc;
+            }
+            __syncthreads();
         }
-        __syncthreads();
         if (!eval) {
-            const double time = ctrl->time_zero + (double)step * (double)a.dt;
+            const double time = time_zero + (double)step * (double)a.dt;
             if (INTEG == GDB_INTEGRATOR_NVT) {  // NVT.py:113-124
                 const double T = target_temperature(a, time);
-                const double dev = 2.0 * stot[0] / ((double)a.dof * T) - 1.0;
+                const double dev = 2.0 * sum_k / ((double)a.dof * T) - 1.0;
                 xi = (float)((double)xi + (double)(a.dt * a.omega2) * dev);
             }
             if (rank == 0 && tid == 0 && rec && step / a.every < a.nrows) {  // scalar_saver.py:165-179
@@ -550,7 +580,7 @@ __global__ void __launch_bounds__(CL_THREADS, 1) k_cluster_run(const ClusterJob 
                 row[GDB_SCALAR_U] = stot[1];
                 row[GDB_SCALAR_W] = stot[2];
                 row[GDB_SCALAR_LAPU] = stot[3];
-                row[GDB_SCALAR_K] = stot[0];
+                row[GDB_SCALAR_K] = sum_k;
                 row[GDB_SCALAR_FSQ] = stot[4];
             }
             if (reset && owner) {  // momentum_reset.py:64-78
@@ -558,8 +588,8 @@ __global__ void __launch_bounds__(CL_THREADS, 1) k_cluster_run(const ClusterJob 
                 v.y -= (float)(stot[6] / stot[8]);
                 v.z -= (float)(stot[7] / stot[8]);
             }
-            rebuild = stot[NQ] > 0.0;
-            if (rank == 0 && tid == 0 && needk) ctrl->sumK = (float)stot[0];
+            rebuild = sum_moved > 0.0;
+            if (rank == 0 && tid == 0 && needk) ctrl->sumK = (float)sum_k;
         } else if (rank == 0 && tid == 0) {
             ctrl->evalU = stot[1];
             ctrl->evalW = stot[2];

@@ -12,7 +12,7 @@ constexpr int CL_CAP_MAX = 1024;    // neighbour slots per particle: upper bound
 constexpr int CL_MAX_CELLS = 8192;  // shared cell table; sparser grids build N^2
 constexpr int CL_NSQ_MAX = 768;     // up to this size the list build is N^2 (measured: 2x faster at 512, 1.5x slower at 2048)
 constexpr int CL_NQ = 11;           // NQ sums + moved flag + max list length
-constexpr size_t CL_SMEM_LIMIT = 208 * 1024;  // dynamic; the kernel's static arrays take under 16 KB
+constexpr size_t CL_SMEM_LIMIT = 208 * 1024;  // dynamic; the kernel's static arrays take under 18 KB
 
 struct ClusterJob {
     SimArgs a;
@@ -25,7 +25,7 @@ struct ClusterJob {
 };
 
 struct ClusterSmem {
-    size_t pos, pos2, sorted, nbl, nbc, newp, part, tot, cstart, cell, crank, cperm, total;
+    size_t pos, pos2, sorted, nbl, nbc, newp, tot, cstart, cell, crank, cperm, total;
 };
 
 __host__ __device__ inline ClusterSmem cluster_smem_layout(int n, int P, int ncell, int cap, int pingpong,
@@ -46,8 +46,6 @@ __host__ __device__ inline ClusterSmem cluster_smem_layout(int n, int P, int nce
     s.nbc = o;
     o += (size_t)P * sizeof(int);
     o = (o + 15) & ~(size_t)15;
-    s.part = o;  // two slots (by step parity when pingpong)
-    o += 2 * CL_NQ * sizeof(double);
     s.tot = o;
     o += CL_NQ * sizeof(double);
     s.cstart = o;  // cell counts, then exclusive starts (ncell + 1)
