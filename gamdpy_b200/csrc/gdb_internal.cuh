@@ -75,6 +75,7 @@ struct DevCtrl {
     unsigned bar_all[3];  // step barrier where every block keeps the books: arrivals, by barrier index mod 3
     int abort;            // set when a barrier wait timed out
     unsigned work[2];     // persistent step: next round to hand out, by step parity
+    unsigned nbl_work;    // cell build: next chunk to hand out
     long long bar_timeout;  // grid-barrier wait limit in SM clock cycles (0: the default, ~1 s)
     unsigned long long *trace;  // optional phase trace: (tag << 56) | globaltimer ns
     int trace_cap;

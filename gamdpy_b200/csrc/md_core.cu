@@ -218,19 +218,15 @@ __global__ void __launch_bounds__(GDB_BLOCK) k_scatter(SimArgs a) {
     if (!a.ctrl->rebuild) return;
     phase_scatter(a);
 }
-__global__ void __launch_bounds__(GDB_BLOCK) k_sort_cells(SimArgs a) {
+__global__ void __launch_bounds__(GDB_BLOCK) k_place(SimArgs a, int cur) {
     if (!a.ctrl->rebuild) return;
-    phase_sort_cells(a);
-}
-__global__ void __launch_bounds__(GDB_BLOCK) k_gather(SimArgs a, int cur) {
-    if (!a.ctrl->rebuild) return;
-    phase_gather(a, cur);
+    phase_place(a, cur);
 }
 template <bool FMA>
 __global__ void __launch_bounds__(GDB_BLOCK) k_nbl_cells(SimArgs a) {
     if (!a.ctrl->rebuild) return;
-    __shared__ NbScratch<GDB_BLOCK / 32> scr;
-    phase_nbl_cells<FMA>(a, grid_span(), scr);
+    __shared__ __align__(16) unsigned char rings[GDB_BLOCK / 32 * NB_RING_BYTES];
+    phase_nbl_cells<FMA>(a, grid_span(), rings);
 }
 __global__ void __launch_bounds__(GDB_BLOCK) k_finish_cells(SimArgs a, int cur) {
     if (!a.ctrl->rebuild) return;
@@ -409,11 +405,13 @@ static void free_graphs(gdb_sim *h) {
 
 static int choose_tp(const gdb_sim *h) {
     if (h->tp_req > 0) return h->tp_req;
-    // about 131k lanes in flight (measured on B200: 1 lane per particle at
-    // N = 1M, 2 at 65k; at 2k, 32 lanes on 256 blocks 100 k TPS against 93 k
-    // with 16 lanes, once grids up to 320 blocks take the one-level barrier)
+    // as many lanes as one block of RUN_THREADS threads per SM gives every
+    // particle, at most 16 (measured on B200, KA, us per step: N 4096 12.0 at
+    // 16 lanes and 13.8 at 32; N 10 007 15.7 at 8 lanes, 17.3 at 4, and 27.6
+    // at 16, which take two rounds; N 65 536 35.9 at 2, 44.0 at 1, 52.3 at 4)
+    const long long even = (h->n + h->num_sms - 1) / h->num_sms;
     int tp = 1;
-    while (tp < 32 && (long long)h->n * tp < 131072) tp *= 2;
+    while (tp < 16 && even * tp * 2 <= RUN_THREADS) tp *= 2;
     return tp;
 }
 
@@ -497,6 +495,7 @@ static int ensure_partials(gdb_sim *h, int nblocks) {
 static SimArgs make_args(gdb_sim *h) {
     SimArgs a;
     a.nsq_smem = 0;
+    a.per_round = 0;
     a.bar_all = h->step_bar_all ? 1 : 0;
     a.pos0 = h->pos[0];
     a.pos1 = h->pos[1];
@@ -610,11 +609,12 @@ static int enqueue_rebuild(gdb_sim *h) {
         k_scan_top<<<1, GDB_BLOCK, 0, h->st>>>(a);
         k_scan_final<<<a.nchunks, GDB_BLOCK, 0, h->st>>>(a);
         k_scatter<<<g, GDB_BLOCK, 0, h->st>>>(a);
-        k_sort_cells<<<grid_for(a.ncell), GDB_BLOCK, 0, h->st>>>(a);
-        k_gather<<<g, GDB_BLOCK, 0, h->st>>>(a, cur);
-        // a warp per cell, or a thread per particle for large systems (the
-        // build picks by threads per particle)
-        const int gw = n >= 131072 ? grid_for(n) : grid_for((long long)a.ncell * 32);
+        k_place<<<g, GDB_BLOCK, 0, h->st>>>(a, cur);
+        // lanes per particle until the GPU is full (the build derives them
+        // from its threads)
+        int lanes = 1;
+        while (lanes < 32 && (long long)n * lanes < (long long)h->num_sms * 1024) lanes *= 2;
+        const int gw = grid_for((long long)n * lanes);
         if (h->fma)
             k_nbl_cells<true><<<gw, GDB_BLOCK, 0, h->st>>>(a);
         else
@@ -627,30 +627,64 @@ static int enqueue_rebuild(gdb_sim *h) {
     return GDB_OK;
 }
 
+// Lanes per particle of the standalone step: its blocks are not bound to an
+// SM, so it wants about 131k lanes in flight (measured on B200: 2 at 65k).
+static int step_lanes(const gdb_sim *h) {
+    if (h->tp_req > 0) return h->tp_req;
+    int tp = 1;
+    while (tp < 32 && (long long)h->n * tp < 131072) tp *= 2;
+    return tp;
+}
+
 static int enqueue_step(gdb_sim *h, int mode) {
-    const int grid = grid_for((long long)h->n * h->tp);
+    const int tp = step_lanes(h);
+    const int grid = grid_for((long long)h->n * tp);
     int rc = ensure_partials(h, grid);
     if (rc) return rc;
     const SimArgs a = make_args(h);
     if (h->ntypes == 1)
-        launch_step_nt1(a, h->table, h->st, h->tp, h->integ, mode, grid, h->cur);
+        launch_step_nt1(a, h->table, h->st, tp, h->integ, mode, grid, h->cur);
     else if (h->ntypes == 2)
-        launch_step_nt2(a, h->table, h->st, h->tp, h->integ, mode, grid, h->cur);
+        launch_step_nt2(a, h->table, h->st, tp, h->integ, mode, grid, h->cur);
     else
-        launch_step_ntg(a, h->table, h->st, h->tp, h->integ, mode, grid, h->cur);
+        launch_step_ntg(a, h->table, h->st, tp, h->integ, mode, grid, h->cur);
     CKL();
     if (mode == MODE_STEP) h->cur ^= 1;
     return GDB_OK;
 }
 
-// Grid of the persistent kernel: every block resident (cooperative launch).
-static int run_grid(gdb_sim *h, const void *fn, int *grid, size_t dsmem = 0) {
+// Shape of the persistent kernel, every block resident (cooperative launch):
+// one block per SM with the particles spread evenly (one round each, as many
+// threads as its particles have lanes) while that fits RUN_THREADS, else
+// blocks of GDB_BLOCK threads that take rounds until none is left.  Measured
+// on B200, KA, us per step, spread against rounds of GDB_BLOCK threads over
+// three blocks an SM: N 65 536 35.9 and 54.6, N 20 000 19.8 and 27.8, N 10 007
+// 15.9 and 25.9 (some blocks had two rounds, others one, and the last of 320
+// to 444 blocks kept the books of all).  Above RUN_THREADS per SM the rounds
+// balance better than even shares taken in turn (N 1 048 576: the force phase
+// 242 us against 320).
+struct RunShape {
+    int grid, block, per_round;
+};
+constexpr int RUN_DSMEM_MAX =
+    std::max(NSQ_SMEM_MAX * (int)sizeof(float4), RUN_THREADS / 32 * NB_RING_BYTES);
+static int run_shape(gdb_sim *h, const void *fn, const SimArgs &a, RunShape *s, size_t *dsmem) {
+    const int tp = h->tp;
+    const int even = (h->n + h->num_sms - 1) / h->num_sms;
+    const bool spread = h->grid_cap == 0 && (long long)even * tp <= RUN_THREADS;
+    s->per_round = spread ? even : GDB_BLOCK / tp;
+    // (the list build's scan wants GDB_BLOCK threads, and its walk uses them)
+    s->block = spread ? std::max(GDB_BLOCK, (even * tp + 31) / 32 * 32) : GDB_BLOCK;
+    *dsmem = a.nsq_smem ? (size_t)h->n * sizeof(float4)
+                        : (a.nb_kind == GDB_NBLIST_CELLS ? (size_t)s->block / 32 * NB_RING_BYTES : 0);
     int occ = 0;
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, GDB_BLOCK, dsmem));
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, s->block, *dsmem));
     if (occ < 1) return set_err(h, GDB_ERR_CUDA, "persistent kernel cannot be resident");
-    const int needed = grid_for((long long)h->n * h->tp);
-    *grid = std::min(std::min(needed, occ * h->num_sms), 64 * BAR_GROUP);
-    if (h->grid_cap > 0) *grid = std::min(*grid, h->grid_cap);
+    s->grid = (h->n + s->per_round - 1) / s->per_round;
+    if (!spread) {
+        s->grid = std::min(std::min(s->grid, occ * h->num_sms), 64 * BAR_GROUP);
+        if (h->grid_cap > 0) s->grid = std::min(s->grid, h->grid_cap);
+    }
     return GDB_OK;
 }
 
@@ -691,20 +725,22 @@ static int launch_run(gdb_sim *h, int steps, int do_eval) {
         a.nbx = a.nby = a.nbz = 0;
     }
     // small N^2 systems: every block stages the positions for the list build
-    const size_t dsmem =
-        (a.nb_kind == GDB_NBLIST_NSQ && h->n <= NSQ_SMEM_MAX && h->nsq_stage) ? (size_t)h->n * sizeof(float4) : 0;
-    a.nsq_smem = dsmem > 0;
-    // static plus dynamic shared memory above 48 KiB needs the opt-in
-    if (dsmem > 0) CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dsmem));
-    int grid = 0;
-    int rc = run_grid(h, fn, &grid, dsmem);
+    a.nsq_smem = a.nb_kind == GDB_NBLIST_NSQ && h->n <= NSQ_SMEM_MAX && h->nsq_stage;
+    // static plus dynamic shared memory above 48 KiB needs the opt-in; one
+    // value for every launch of the function
+    CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, RUN_DSMEM_MAX));
+    RunShape shape{};
+    size_t dsmem = 0;
+    int rc = run_shape(h, fn, a, &shape, &dsmem);
     if (rc) return rc;
+    a.per_round = shape.per_round;
     // a row per round, two steps' rows where every block keeps the books
-    if ((rc = ensure_partials(h, std::max(grid, 2 * grid_for((long long)h->n * h->tp))))) return rc;
+    const int rounds = (h->n + shape.per_round - 1) / shape.per_round;
+    if ((rc = ensure_partials(h, std::max(shape.grid, 2 * rounds)))) return rc;
     a.partials = h->partials;
     int cur0 = h->cur, ns = steps, ev = do_eval;
     void *args[] = {(void *)&a, (void *)&h->table, (void *)&cur0, (void *)&ns, (void *)&ev};
-    CK(cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(GDB_BLOCK), args, dsmem, h->st));
+    CK(cudaLaunchCooperativeKernel(fn, dim3(shape.grid), dim3(shape.block), args, dsmem, h->st));
     h->cur ^= (steps & 1);
     return GDB_OK;
 }
@@ -926,7 +962,7 @@ int gdb_sim_create(int n, int ntypes, int device, gdb_sim **out) {
     AL(h->vel, N * sizeof(float4));
     AL(h->frc, N * sizeof(float4));
     AL(h->rref, N * sizeof(float4));
-    AL(h->pos_tmp, N * sizeof(float4));
+    AL(h->pos_tmp, (N + NB_PAD) * sizeof(float4));
     AL(h->vel_tmp, N * sizeof(float4));
     AL(h->img, N * sizeof(int4));
     AL(h->img_tmp, N * sizeof(int4));
@@ -1930,14 +1966,17 @@ static gdb_batch::Group *batch_group(gdb_batch *b, int kind, int C, int tp) {
 
 static cudaError_t launch_run_clusters(const void *fn, const ClusterRunJob *d_jobs, int count, int C, int nsteps,
                                        int do_eval, cudaStream_t st) {
+    constexpr int dsmem = CLG_BLOCK / 32 * NB_RING_BYTES;  // the cell build's rings
+    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, dsmem);
+    if (e != cudaSuccess) return e;
     if (C > 8) {
-        cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        e = cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
         if (e != cudaSuccess) return e;
     }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(count * C);
     cfg.blockDim = dim3(CLG_BLOCK);
-    cfg.dynamicSmemBytes = 0;
+    cfg.dynamicSmemBytes = dsmem;
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;

@@ -17,13 +17,11 @@ __device__ __forceinline__ void load_table(const PairTable &tab, PairEntry *s_ta
 // one step (or the force-only evaluation); the last block to finish does
 // the float64 bookkeeping
 // register budget: 64 per thread (4 blocks/SM) for one lane per particle,
-// 80 (3 blocks/SM) when lanes share a particle (measured best on B200); the
-// persistent kernel also holds the list-build phase
+// 80 (3 blocks/SM) when lanes share a particle (measured best on B200)
 #define GDB_STEP_MINBLOCKS(TP) ((TP) == 1 ? 4 : 3)
-#ifndef GDB_RUN_MINBLOCKS_TP1
-#define GDB_RUN_MINBLOCKS_TP1 4
-#endif
-#define GDB_RUN_MINBLOCKS(TP) ((TP) == 1 ? GDB_RUN_MINBLOCKS_TP1 : 3)
+// the persistent kernel: 64 as well, for one block of up to RUN_THREADS
+// threads per SM or four of GDB_BLOCK
+constexpr int RUN_THREADS = 1024;
 
 template <int TP, int NT, int INTEG, int MODE>
 __global__ void __launch_bounds__(GDB_BLOCK, GDB_STEP_MINBLOCKS(TP)) k_step(SimArgs a, PairTable tab, int cur) {
@@ -83,13 +81,14 @@ struct ClusterSync {
 
 // Neighbour-list rebuild by the blocks of span g: the phases of the
 // standalone chain with a synchronisation between them.
-template <bool FMA, int WPB, class Sync>
-__device__ inline bool rebuild_phases(const SimArgs &a, int cur, Span g, const Sync &sync, NbScratch<WPB> &scr,
-                                      float4 *spos) {
+// dsm: the kernel's dynamic shared memory, for the N^2 build's copy of the
+// positions (a.nsq_smem) or the cell build's rings.
+template <bool FMA, class Sync>
+__device__ inline bool rebuild_phases(const SimArgs &a, int cur, Span g, const Sync &sync, unsigned char *dsm) {
     DevCtrl *c = a.ctrl;
     auto none = [] {};
     if (a.nb_kind == GDB_NBLIST_NSQ) {
-        phase_nbl_nsq<FMA, false>(a, cur, g, spos);
+        phase_nbl_nsq<FMA, false>(a, cur, g, a.nsq_smem ? reinterpret_cast<float4 *>(dsm) : nullptr);
         trace_mark(c, TR_REBUILD_PHASE);
         const bool ok = sync(c, [&] {
             if (threadIdx.x == 0) rebuild_done(c);
@@ -100,20 +99,21 @@ __device__ inline bool rebuild_phases(const SimArgs &a, int cur, Span g, const S
     phase_cell_assign<false>(a, cur, g);
     if (!sync(c, none)) return false;
     trace_mark(c, TR_REBUILD_PHASE);
-    phase_scan_partial(a, g);
-    if (!sync(c, [&] { block_scan_chunks(a); })) return false;
-    phase_scan_final(a, g);
+    if (a.nchunks <= SCAN_DIRECT_CHUNKS) {
+        phase_scan_direct(a, g);
+    } else {
+        phase_scan_partial(a, g);
+        if (!sync(c, [&] { block_scan_chunks(a); })) return false;
+        phase_scan_final(a, g);
+    }
     if (!sync(c, none)) return false;
     phase_scatter(a, g);
     if (!sync(c, none)) return false;
     trace_mark(c, TR_REBUILD_PHASE);
-    phase_sort_cells(a, g);
-    if (!sync(c, none)) return false;
-    phase_gather(a, cur, g);
+    phase_place(a, cur, g);
     if (!sync(c, none)) return false;
     trace_mark(c, TR_REBUILD_PHASE);
-    phase_nbl_cells<FMA>(a, g, scr);
-    if (!sync(c, none)) return false;
+    phase_nbl_cells<FMA>(a, g, dsm);
     trace_mark(c, TR_REBUILD_PHASE);
     phase_finish_cells(a, cur, g);
     const bool ok = sync(c, [&] {
@@ -126,15 +126,9 @@ __device__ inline bool rebuild_phases(const SimArgs &a, int cur, Span g, const S
 // `nsteps` steps starting from pos[cur0], then (if do_eval) the force-only
 // evaluation of the final state -- one timeblock of
 // simulation/Simulation.py:306-328 -- by the blocks of span g.
-// NPT_Atomic changes the box every step: the box of the step (ctrl->box,
-// written by the previous step's bookkeeping), and at a list build the cell
-// grid of that box as nblist_linked_lists.py:36-39 computes it, within the
-// allocated grid.
-__device__ __forceinline__ void npt_refresh_box(SimArgs &a) {
-    a.Lx = *(volatile float *)&a.ctrl->box[0];
-    a.Ly = *(volatile float *)&a.ctrl->box[1];
-    a.Lz = *(volatile float *)&a.ctrl->box[2];
-}
+// NPT_Atomic changes the box every step; at a list build the cell grid of
+// that box as nblist_linked_lists.py:36-39 computes it, within the allocated
+// grid.
 __device__ __forceinline__ void npt_cell_grid(SimArgs &a) {
     if (a.nb_kind != GDB_NBLIST_CELLS) return;
     a.ncx = min(a.ncx_max, max(1, (int)(a.Lx / a.min_cell)));
@@ -144,17 +138,20 @@ __device__ __forceinline__ void npt_cell_grid(SimArgs &a) {
     a.nchunks = (a.ncell + SCAN_CHUNK - 1) / SCAN_CHUNK;
 }
 
-template <int TP, int NT, int INTEG, int WPB, class Sync>
+template <int TP, int NT, int INTEG, class Sync>
 __device__ inline void run_steps(const SimArgs &a0, const PairEntry *s_tab, int nt, int cur0, int nsteps, int do_eval,
-                                 Span g, const Sync &sync, double *s_red, float4 *spos = nullptr) {
-    __shared__ NbScratch<WPB> scr;
-    // NPT_Atomic: a copy of the arguments follows the box
-    SimArgs a_npt;
-    if (INTEG == GDB_INTEGRATOR_NPT) a_npt = a0;
-    const SimArgs &a = INTEG == GDB_INTEGRATOR_NPT ? a_npt : a0;
+                                 Span g, const Sync &sync, double *s_red, unsigned char *dsm) {
+    // NPT_Atomic: the block's copy of the arguments follows the box
+    __shared__ SimArgs s_npt;
+    if (INTEG == GDB_INTEGRATOR_NPT) {
+        if (threadIdx.x == 0) s_npt = a0;
+        __syncthreads();
+    }
+    const SimArgs &a = INTEG == GDB_INTEGRATOR_NPT ? s_npt : a0;
     DevCtrl *ctrl = a.ctrl;
     int cur = cur0;
-    const int rounds = (a.n + (int)blockDim.x / TP - 1) / ((int)blockDim.x / TP);  // partial rows per step
+    const int per_round = a.per_round > 0 ? a.per_round : (int)blockDim.x / TP;
+    const int rounds = (a.n + per_round - 1) / per_round;  // partial rows per step
     trace_mark(ctrl, TR_START);
     __shared__ StepCtl s_ctl;
     __shared__ int s_any;  // a particle moved beyond skin/2 (the block running `last`, or every block)
@@ -162,22 +159,30 @@ __device__ inline void run_steps(const SimArgs &a0, const PairEntry *s_tab, int 
     // step (step_barrier_all, finalize_step_all), on rows double-buffered by
     // step parity, as a block may write the next step's rows while another
     // still sums this step's
-    const bool all = Sync::kGrid && INTEG != GDB_INTEGRATOR_NPT && a.bar_all && (int)gridDim.x <= BAR_FLAT_MAX;
+    const bool all = Sync::kGrid && a.bar_all && (int)gridDim.x <= BAR_FLAT_MAX;
     unsigned seq = 0;  // step barriers of this launch
     for (int s = 0; s < nsteps + do_eval; s++) {
-        if (INTEG == GDB_INTEGRATOR_NPT) npt_refresh_box(a_npt);
         // the rebuild flag, the step index and the state the step reads
         // (momentum shift, thermostat), loaded together by one thread: none
         // of them changes across a rebuild.  Where every block keeps the
         // books, its own copy is current after the first step.
-        if (threadIdx.x == 0 && (!all || s == 0)) load_step_ctl(ctrl, &s_ctl);
+        if (threadIdx.x == 0) {
+            if (!all || s == 0) load_step_ctl(ctrl, &s_ctl);
+            if (INTEG == GDB_INTEGRATOR_NPT) {  // the step's box, constants and (for a build) cell grid
+                if (!all || s == 0) load_npt_state(ctrl, &s_ctl.npt);
+                s_npt.Lx = s_ctl.npt.box[0];
+                s_npt.Ly = s_ctl.npt.box[1];
+                s_npt.Lz = s_ctl.npt.box[2];
+                s_ctl.ns = npt_step_consts(s_npt, s_ctl.npt);
+                if (s_ctl.rebuild) npt_cell_grid(s_npt);
+            }
+        }
         __syncthreads();
         const int rebuild = s_ctl.rebuild;
         const int step = s_ctl.step;
         if (rebuild) {
-            if (INTEG == GDB_INTEGRATOR_NPT) npt_cell_grid(a_npt);
-            const bool ok = a.fma ? rebuild_phases<true>(a, cur, g, sync, scr, spos)
-                                  : rebuild_phases<false>(a, cur, g, sync, scr, spos);
+            const bool ok = a.fma ? rebuild_phases<true>(a, cur, g, sync, dsm)
+                                  : rebuild_phases<false>(a, cur, g, sync, dsm);
             if (!ok) return;
         }
         bool ok;
@@ -230,9 +235,7 @@ __device__ inline bool rebuild_phases_bricks(const SimArgs &a, int cur, Span g, 
     phase_scatter(a, g);
     if (!sync(c, none)) return false;
     trace_mark(c, TR_REBUILD_PHASE);
-    phase_sort_cells(a, g);
-    if (!sync(c, none)) return false;
-    phase_gather(a, cur, g);
+    phase_place(a, cur, g);
     if (!sync(c, none)) return false;
     trace_mark(c, TR_REBUILD_PHASE);
     if (!phase_nbl_bricks<FMA>(a, bs, pp, g)) return false;
@@ -323,18 +326,17 @@ __global__ void __launch_bounds__(BRICK_THREADS, 2) k_step_bricks(SimArgs a, Pai
 }
 
 // Persistent cooperative kernel: one timeblock of one system per launch.
-// Small N^2-list systems stage their positions for the list build in dynamic
-// shared memory (a.nsq_smem, n float4 per block).
+// The list builds use dynamic shared memory: n float4 for small N^2-list
+// systems (a.nsq_smem), the rings of the cell build otherwise.
 template <int TP, int NT, int INTEG>
-__global__ void __launch_bounds__(GDB_BLOCK, GDB_RUN_MINBLOCKS(TP)) k_run(SimArgs a, PairTable tab, int cur0, int nsteps, int do_eval) {
-    extern __shared__ float4 run_dsm[];
+__global__ void __launch_bounds__(RUN_THREADS, 1) k_run(SimArgs a, PairTable tab, int cur0, int nsteps, int do_eval) {
+    extern __shared__ __align__(16) unsigned char run_dsm[];
     __shared__ PairEntry s_tab[GDB_MAX_TYPES * GDB_MAX_TYPES];
     __shared__ double s_red[NQ * 32];
     load_table(tab, s_tab);
     // a block that starts after others abandoned a barrier does no work
     if (*(volatile int *)&a.ctrl->abort) return;
-    run_steps<TP, NT, INTEG, GDB_BLOCK / 32>(a, s_tab, tab.nt, cur0, nsteps, do_eval, grid_span(), GridSync{}, s_red,
-                                             a.nsq_smem ? run_dsm : nullptr);
+    run_steps<TP, NT, INTEG>(a, s_tab, tab.nt, cur0, nsteps, do_eval, grid_span(), GridSync{}, s_red, run_dsm);
 }
 
 // One system per thread-block cluster, state in global memory: a batch of
@@ -353,6 +355,7 @@ __global__ void __launch_bounds__(CLG_BLOCK, 1)
     k_run_clusters(const ClusterRunJob *__restrict__ jobs, int nsteps, int do_eval) {
     __shared__ PairEntry s_tab[GDB_MAX_TYPES * GDB_MAX_TYPES];
     __shared__ double s_red[NQ * 32];
+    extern __shared__ __align__(16) unsigned char clg_dsm[];  // NB_RING_BYTES per warp
     __shared__ SimArgs s_a;
     unsigned rank, nrank;
     asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
@@ -360,8 +363,8 @@ __global__ void __launch_bounds__(CLG_BLOCK, 1)
     const ClusterRunJob &job = jobs[blockIdx.x / nrank];
     if (threadIdx.x == 0) s_a = job.a;
     load_table(job.tab, s_tab);  // ends with __syncthreads
-    run_steps<TP, NT, INTEG, CLG_BLOCK / 32>(s_a, s_tab, job.tab.nt, job.cur, nsteps, do_eval,
-                                             Span{(int)rank, (int)nrank}, ClusterSync{(int)rank}, s_red);
+    run_steps<TP, NT, INTEG>(s_a, s_tab, job.tab.nt, job.cur, nsteps, do_eval, Span{(int)rank, (int)nrank},
+                             ClusterSync{(int)rank}, s_red, clg_dsm);
 }
 
 // Entry points each instantiation unit exports to the host code.

@@ -24,6 +24,7 @@ constexpr int SCAN_CHUNK = 2048;
 constexpr int MODE_STEP = 0;
 constexpr int MODE_EVAL = 1;
 constexpr int NB_CHUNK = 4;  // neighbour indices stored and loaded 4 at a time (int4)
+constexpr int NB_PAD = 4;    // slots of pos_tmp that may be read past the last particle
 
 // Neighbour list layout: entry k of particle i at
 //   (k / 4) * (stride * 4) + i * 4 + (k % 4)
@@ -55,6 +56,7 @@ struct SimArgs {
     int brick_hcap;     // staged positions a brick's halo may hold (<= BRICK_HCAP)
     int nb_kind, fma;
     int nsq_smem;  // persistent N^2 build stages all positions in dynamic shared memory
+    int per_round;  // particles per round of the force phase (0: blockDim / lanes)
     int bar_all;   // persistent grid: every block keeps the step's books (grids of <= BAR_FLAT_MAX blocks)
     float Lx, Ly, Lz;
     float cps2;    // (max_cut + skin)^2, nblist.py:152
@@ -268,76 +270,45 @@ __device__ __forceinline__ bool step_barrier_all(DevCtrl *c, unsigned seq, bool 
 // ---------------------------------------------------------------------------
 // neighbour-list phases
 // ---------------------------------------------------------------------------
-
-// One pass of the N^2 candidate walk of a warp: lanes test candidates
-// j0 + 32u + lane (u < 4, loaded before they are tested) against particle i0
-// and, with TWO, i1; hits are appended in ascending j by ballot + popc.  CHECK
-// (the last, partial pass only) masks candidates j >= n.  The tests are
-// combined without short-circuit branches: the distance is cheap and pure.
 template <bool B>
 struct BoolTag {
     static constexpr bool value = B;
 };
 
-struct NsqWalk {
-    const float4 *pos, *src;
-    int n, max_nbs;
-    size_t cstride;  // stride * NB_CHUNK: entries k and k + 4 of a particle
-    float Lx, Ly, Lz, cps2;
-    const int *excl, *orig;
-    int *nbl;
-    int lane;
-    unsigned below;
-};
-template <bool FMA, bool NC, bool TWO, bool CHECK>
-__device__ __forceinline__ void nsq_pass(const SimArgs &a, const NsqWalk &w, int j0, int i0, int i1, float4 p0,
-                                         float4 p1, int u0, int u1, int &c0, int &c1) {
-    float4 q[4];
+
+// Hits of a warp's particle i, set bits of the lanes' masks, appended to its
+// list: the lanes' hits follow one another in lane order, bit q of lane L is
+// index(L, q).  Returns the number of hits (all lanes).
+template <class Index>
+__device__ __forceinline__ int warp_append(unsigned mask, int cnt, int max_nbs, int *base, size_t cstride, int lane,
+                                           Index index) {
+    const int mine = __popc(mask);
+    int incl = mine;
 #pragma unroll
-    for (int u = 0; u < 4; u++) {
-        const int j = j0 + 32 * u + w.lane;
-        // one load kind per instantiation: the read-only path for the
-        // standalone kernel (never staged), plain loads from the staged copy
-        // or the coherent buffer otherwise
-        q[u] = (!CHECK || j < w.n) ? (NC ? load<true>(w.pos + j) : w.src[j]) : p0;
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += y;
     }
-#pragma unroll
-    for (int u = 0; u < 4; u++) {
-        const int j = j0 + 32 * u + w.lane;
-        const bool in = !CHECK || j < w.n;
-        bool h0 = in & (j != i0) & (dist_sq_exact<FMA>(q[u], p0, w.Lx, w.Ly, w.Lz) < w.cps2);
-        bool h1 = false;
-        if (TWO) h1 = in & (j != i1) & (dist_sq_exact<FMA>(q[u], p1, w.Lx, w.Ly, w.Lz) < w.cps2);
-        if (w.excl) {
-            if (h0) h0 = !excluded(a, u0, w.orig[j]);
-            if (TWO && h1) h1 = !excluded(a, u1, w.orig[j]);
-        }
-        const unsigned m0 = __ballot_sync(0xffffffffu, h0);
-        if (h0) {
-            const int k = c0 + __popc(m0 & w.below);
-            if (k < w.max_nbs) w.nbl[(size_t)(k >> 2) * w.cstride + (size_t)i0 * NB_CHUNK + (k & 3)] = j;
-        }
-        c0 += __popc(m0);
-        if (TWO) {
-            const unsigned m1 = __ballot_sync(0xffffffffu, h1);
-            if (h1) {
-                const int k = c1 + __popc(m1 & w.below);
-                if (k < w.max_nbs) w.nbl[(size_t)(k >> 2) * w.cstride + (size_t)i1 * NB_CHUNK + (k & 3)] = j;
-            }
-            c1 += __popc(m1);
-        }
+    int k = cnt + incl - mine;
+    while (mask) {
+        const int j = index(__ffs(mask) - 1);
+        mask &= mask - 1u;
+        if (k < max_nbs) base[(size_t)(k >> 2) * cstride + (k & 3)] = j;
+        k++;
     }
+    return __shfl_sync(0xffffffffu, incl, 31);
 }
 
-// N^2 build (interactions/nblist.py:88-143): a warp per particle, lanes
-// stride over j, ballot + popc append hits in ascending j (deterministic).
-// A warp takes its particles two at a time (i and i + the number of warps):
-// every candidate is loaded once for both, and the two append chains are
-// independent.  Whether a warp has a second particle is uniform over the
-// warp, so the walk is instantiated for one and for two particles, and the
-// full passes skip the j < n test of the last one.  With `spos` (shared
-// memory for all n positions) the block first copies the positions there,
-// so the candidate loads are shared-memory loads.
+// N^2 build (interactions/nblist.py:88-143): a warp per particle.  Lane L
+// tests j = 32 q + L and sets bit q of its mask; after 32 rounds the lanes'
+// hits are appended lane by lane (a fixed order).  The walk over the
+// candidates is the test alone (18 instructions against 57 with a ballot and
+// an append per round); the appends run once per 1024 candidates.  A warp
+// takes its particles two at a time (i and i + the number of warps): every
+// candidate is loaded once for both.  With `spos` (shared memory for all n
+// positions) the block first copies the positions there, so the candidate
+// loads are shared-memory loads.  Measured on B200, N 2048 (KA and LJ), whole
+// rebuild: 23.6 -> 13.2 us.
 template <bool FMA, bool NC>
 __device__ inline void phase_nbl_nsq(const SimArgs &a, int cur, Span g = grid_span(), float4 *spos = nullptr) {
     const float4 *pos = cur_pos(a, cur);
@@ -360,49 +331,60 @@ __device__ inline void phase_nbl_nsq(const SimArgs &a, int cur, Span g = grid_sp
     }
     // the arguments the loop reads, in registers: the list stores could
     // otherwise force them to be reloaded after every store
-    NsqWalk w;
-    w.pos = pos;
-    w.src = src;
-    w.n = a.n;
-    w.max_nbs = a.max_nbs;
-    w.cstride = (size_t)a.stride * NB_CHUNK;
-    w.Lx = a.Lx;
-    w.Ly = a.Ly;
-    w.Lz = a.Lz;
-    w.cps2 = a.cps2;
-    w.excl = a.excl;
-    w.orig = a.orig;
-    w.nbl = a.nbl;
-    w.lane = threadIdx.x & 31;
-    w.below = (1u << w.lane) - 1u;
-    const int n = w.n;
-    const int nfull = n & ~127;  // candidates covered by full passes
+    const int n = a.n, max_nbs = a.max_nbs;
+    const size_t cstride = (size_t)a.stride * NB_CHUNK;
+    const float Lx = a.Lx, Ly = a.Ly, Lz = a.Lz, cps2 = a.cps2;
+    const int lane = threadIdx.x & 31;
     const int warps = (g.nb * (int)blockDim.x) >> 5;
+    // one load kind per instantiation: the read-only path for the standalone
+    // kernel (never staged), plain loads from the staged copy or the coherent
+    // buffer otherwise
+    auto at = [&](int j) { return NC ? load<true>(pos + j) : src[j]; };
     for (int i0 = (g.b * (int)blockDim.x + (int)threadIdx.x) >> 5; i0 < n; i0 += 2 * warps) {
         const int i1 = i0 + warps;
         const bool has1 = i1 < n;  // the same for every lane of the warp
-        const float4 p0 = NC ? load<true>(pos + i0) : src[i0];
-        const float4 p1 = has1 ? (NC ? load<true>(pos + i1) : src[i1]) : p0;
-        const int u0 = w.excl ? w.orig[i0] : 0, u1 = (w.excl && has1) ? w.orig[i1] : 0;
+        const float4 p0 = at(i0), p1 = has1 ? at(i1) : p0;
+        int *row0 = a.nbl + (size_t)i0 * NB_CHUNK, *row1 = a.nbl + (size_t)i1 * NB_CHUNK;
         int c0 = 0, c1 = 0;
-        if (has1) {
-            int j0 = 0;
-            for (; j0 < nfull; j0 += 128) nsq_pass<FMA, NC, true, false>(a, w, j0, i0, i1, p0, p1, u0, u1, c0, c1);
-            if (j0 < n) nsq_pass<FMA, NC, true, true>(a, w, j0, i0, i1, p0, p1, u0, u1, c0, c1);
-        } else {
-            int j0 = 0;
-            for (; j0 < nfull; j0 += 128) nsq_pass<FMA, NC, false, false>(a, w, j0, i0, i1, p0, p1, u0, u1, c0, c1);
-            if (j0 < n) nsq_pass<FMA, NC, false, true>(a, w, j0, i0, i1, p0, p1, u0, u1, c0, c1);
+        for (int j0 = 0; j0 < n; j0 += 1024) {
+            unsigned m0 = 0, m1 = 0;
+            const int rounds = min(32, (n - j0 + 31) >> 5);
+            for (int q = 0; q < rounds; q += 4) {  // four candidates in flight
+                float4 p[4];
+#pragma unroll
+                for (int u = 0; u < 4; u++) p[u] = at(min(j0 + 32 * (q + u) + lane, n - 1));
+                unsigned b0 = 0, b1 = 0;
+#pragma unroll
+                for (int u = 0; u < 4; u++) {
+                    if (dist_sq_exact<FMA>(p[u], p0, Lx, Ly, Lz) < cps2) b0 |= 1u << u;
+                    if (has1 && dist_sq_exact<FMA>(p[u], p1, Lx, Ly, Lz) < cps2) b1 |= 1u << u;
+                }
+                m0 |= b0 << q;
+                m1 |= b1 << q;
+            }
+            // candidates past n, and the particle itself
+            const int own = max(0, (n - j0 - lane + 31) >> 5);  // this lane's candidates
+            const unsigned in = own >= 32 ? 0xffffffffu : (1u << own) - 1u;
+            auto keep = [&](unsigned m, int i) {
+                m &= in;
+                if ((unsigned)(i - j0) < 1024u && ((i - j0) & 31) == lane) m &= ~(1u << ((i - j0) >> 5));
+                if (a.excl)
+                    for (unsigned t = m; t; t &= t - 1u)
+                        if (excluded(a, a.orig[i], a.orig[j0 + 32 * (__ffs(t) - 1) + lane])) m &= ~(t & (0u - t));
+                return m;
+            };
+            auto index = [&](int q) { return j0 + 32 * q + lane; };
+            c0 += warp_append(keep(m0, i0), c0, max_nbs, row0, cstride, lane, index);
+            if (has1) c1 += warp_append(keep(m1, i1), c1, max_nbs, row1, cstride, lane, index);
         }
-        if (w.lane == 0) {
+        if (lane == 0) {
             a.nbc[i0] = c0;
             a.rref[i0] = p0;
-            atomicMax(&a.ctrl->maxcount, c0);
             if (has1) {
                 a.nbc[i1] = c1;
                 a.rref[i1] = p1;
-                atomicMax(&a.ctrl->maxcount, c1);
             }
+            atomicMax(&a.ctrl->maxcount, max(c0, c1));
         }
     }
 }
@@ -517,6 +499,30 @@ __device__ inline void phase_scan_final(const SimArgs &a, Span g = grid_span()) 
     if (g.b == 0 && threadIdx.x == 0) a.cell_start[a.ncell] = a.n;
 }
 
+// The whole scan in one phase for grids of at most SCAN_DIRECT_CHUNKS chunks:
+// every block adds up the counts before its chunk itself (at most 120 loads a
+// thread, in flight together) instead of meeting at a barrier for the chunk
+// sums and at another for their scan (a grid barrier is 3 to 5 us; a rebuild
+// has four of them, of eight before).
+constexpr int SCAN_DIRECT_CHUNKS = 16;
+__device__ inline void phase_scan_direct(const SimArgs &a, Span g = grid_span()) {
+    __shared__ int sm[32];
+    __shared__ int s_base;
+    for (int c = g.b; c < a.nchunks; c += g.nb) {
+        int sum = 0;
+#pragma unroll 8
+        for (int k = threadIdx.x; k < c * SCAN_CHUNK; k += blockDim.x) sum += a.cell_count[k];
+        sum = warp_sum(sum);
+        if (threadIdx.x == 0) s_base = 0;
+        __syncthreads();
+        if ((threadIdx.x & 31) == 0) atomicAdd(&s_base, sum);
+        __syncthreads();
+        chunk_scan(a.cell_count, a.ncell, c * SCAN_CHUNK, a.cell_start, s_base, nullptr, sm);
+        __syncthreads();
+    }
+    if (g.b == 0 && threadIdx.x == 0) a.cell_start[a.ncell] = a.n;
+}
+
 __device__ inline void phase_scatter(const SimArgs &a, Span g = grid_span()) {
     for (int i = g.b * (int)blockDim.x + (int)threadIdx.x; i < a.n; i += g.nb * (int)blockDim.x) {
         const int slot = a.cell_start[a.pcell[i]] + a.prank[i];
@@ -527,42 +533,41 @@ __device__ inline void phase_scatter(const SimArgs &a, Span g = grid_span()) {
     }
 }
 
-// Order every cell's particles by user index: the atomics of the assignment
-// rank them arbitrarily; this makes the layout and every sum deterministic.
-__device__ inline void phase_sort_cells(const SimArgs &a, Span g = grid_span()) {
-    for (int c = g.b * (int)blockDim.x + (int)threadIdx.x; c < a.ncell; c += g.nb * (int)blockDim.x) {
-        const int lo = a.cell_start[c], hi = a.cell_start[c + 1];
-        for (int x = lo + 1; x < hi; x++) {
-            const int v = a.perm[x];
-            const int key = a.orig[v];
-            int y = x - 1;
-            while (y >= lo && a.orig[a.perm[y]] > key) {
-                a.perm[y + 1] = a.perm[y];
-                y--;
-            }
-            a.perm[y + 1] = v;
-        }
-    }
-}
-
-__device__ inline void phase_gather(const SimArgs &a, int cur, Span g = grid_span()) {
+// Every particle into its slot: its cell's particles in the order of their
+// user indices (the atomics of the assignment rank them arbitrarily; this
+// makes the layout and every sum deterministic).  A particle counts the
+// members of its cell below it, so ordering and moving take one phase.
+__device__ inline void phase_place(const SimArgs &a, int cur, Span g = grid_span()) {
+    if (g.b == 0 && threadIdx.x == 0) a.ctrl->nbl_work = 0;  // the build follows a barrier later
     const float4 *pos = cur_pos(a, cur);
     const size_t n = a.n;
-    for (int s = g.b * (int)blockDim.x + (int)threadIdx.x; s < a.n; s += g.nb * (int)blockDim.x) {
-        int i = a.perm[s];
-        if ((unsigned)i >= (unsigned)a.n) {
-            atomicOr(&a.ctrl->status, GDB_STATUS_BAD_INDEX);
-            i = s;
-        }
-        a.pos_tmp[s] = pos[i];
-        a.vel_tmp[s] = a.vel[i];
-        a.img_tmp[s] = a.img[i];
-        a.orig_tmp[s] = a.orig[i];
-        a.scell[s] = a.pcell[i];
+    for (int i = g.b * (int)blockDim.x + (int)threadIdx.x; i < a.n; i += g.nb * (int)blockDim.x) {
+        const int c = a.pcell[i], key = a.orig[i];
+        const float4 p = pos[i], v = a.vel[i];
+        const int4 im = a.img[i];
         // K and Fsq travel with the particle; U, W, lapU are rewritten by the
         // next force evaluation
-        a.pscal_tmp[3 * n + s] = a.pscal[3 * n + i];
-        a.pscal_tmp[4 * n + s] = a.pscal[4 * n + i];
+        const float kin = a.pscal[3 * n + i], fsq = a.pscal[4 * n + i];
+        const int lo = a.cell_start[c], hi = a.cell_start[c + 1];
+        int s = lo;
+        for (int x = lo; x < hi; x++) {
+            const int m = a.perm[x];
+            if ((unsigned)m < (unsigned)a.n)
+                s += a.orig[m] < key ? 1 : 0;
+            else
+                atomicOr(&a.ctrl->status, GDB_STATUS_BAD_INDEX);
+        }
+        if ((unsigned)s >= (unsigned)a.n) {
+            atomicOr(&a.ctrl->status, GDB_STATUS_BAD_INDEX);
+            continue;
+        }
+        a.pos_tmp[s] = p;
+        a.vel_tmp[s] = v;
+        a.img_tmp[s] = im;
+        a.orig_tmp[s] = key;
+        a.scell[s] = c;
+        a.pscal_tmp[3 * n + s] = kin;
+        a.pscal_tmp[4 * n + s] = fsq;
     }
 }
 
@@ -586,312 +591,267 @@ __device__ __forceinline__ float dist_sq_shifted(float4 pj, float4 pi, float sx,
     return s;
 }
 
-// Cell-list build (nblist_linked_lists.py:133-183 semantics: all particles of
-// the 5x5x5 stencil with dist_sq < (max_cut+skin)^2, j != i).  One warp per
-// cell: the cell's particles share the stencil.  Slots are sorted by cell
-// with x fastest, so the five x-cells of one (dy, dz) row are one contiguous
-// slot range (two at the x wrap); the warp lists the <= 50 ranges with their
-// prefix sums in shared memory and walks the packed candidate sequence 64 at
-// a time, testing each candidate against up to NBW particles of the cell held
-// in registers.  Ballot + popc append in candidate order: deterministic.
+// Cell-list builds (nblist_linked_lists.py:133-183 semantics: all particles of
+// the 5x5x5 stencil with dist_sq < (max_cut+skin)^2, j != i).  Slots are sorted
+// by cell with x fastest, so the x-cells of one (dy, dz) row of the stencil are
+// one contiguous slot range (two at the x wrap).  The build first sets a bit
+// per hit for up to 32 or 64 candidates, then append the set bits: the test is
+// a load, the differences, one compare and one OR, and the append's address
+// arithmetic runs once per hit (a quarter of the candidates).
 //
 // SHIFTED (every dimension >= 7 cells, no coordinate on a box face): a pair
 // in cells at most two apart is closer than 3 cell edges < L/2 without a
 // wrap and farther than L/2 with one, so the minimum-image decision of the
-// reference is fixed per range and the distance needs no comparisons.
-// Otherwise (small grids) every candidate takes the reference's full test,
-// and grids with fewer than five cells in a dimension visit each cell once.
-constexpr int NBW = 4;         // particles of a cell handled per pass
-constexpr int NB_SEG_MAX = 64; // 25 rows x at most 2 ranges
+// reference is fixed per range and the distance needs no comparisons: it is
+// ((rj - ri) + shift), bit for bit.  Otherwise (small grids) every candidate
+// takes the reference's full test, and grids with fewer than five cells in a
+// dimension visit each cell once.
 
-__device__ __forceinline__ int wrapi(int x, int n) { return ((x % n) + n) % n; }
+// Next number of a work counter, for the whole warp.
+__device__ __forceinline__ int warp_take(unsigned *counter) {
+    int k = 0;
+    if ((threadIdx.x & 31) == 0) k = (int)atomicAdd(counter, 1u);
+    return __shfl_sync(0xffffffffu, k, 0);
+}
+
 // x within two cells of [0, n), n >= 5: one compare each way, no division
 __device__ __forceinline__ int wrap_near(int x, int n) { return x < 0 ? x + n : (x >= n ? x - n : x); }
 
-// s_lo, s_pre, s_sh: per-warp segment tables in shared memory (block warp w
-// uses entries [w * NB_SEG_MAX, ...), s_pre one more).
-template <bool FMA, bool SHIFTED>
-__device__ inline void phase_nbl_cells_t(const SimArgs &a, Span g, int *s_lo, int *s_pre, float3 *s_sh) {
-    const float4 *pos = a.pos_tmp;
-    const int ncx = a.ncx, ncy = a.ncy, ncz = a.ncz;
-    const float Lx = a.Lx, Ly = a.Ly, Lz = a.Lz;
-    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    int *lo_s = s_lo + wib * NB_SEG_MAX, *pre_s = s_pre + wib * (NB_SEG_MAX + 1);
-    float3 *sh_s = s_sh + wib * NB_SEG_MAX;
-    const int nwarps = (g.nb * (int)blockDim.x) >> 5;
-    const int ry = ncy < 5 ? ncy : 5, rz = ncz < 5 ? ncz : 5;
-    const int nrows = ry * rz;
-    for (int c = (g.b * (int)blockDim.x + (int)threadIdx.x) >> 5; c < a.ncell; c += nwarps) {
-        const int cs = a.cell_start[c], ce = a.cell_start[c + 1];
-        if (cs == ce) continue;
-        const int cx = c % ncx, cy = (c / ncx) % ncy, cz = c / (ncx * ncy);
-        // lane r < nrows builds the x-range(s) of stencil row r
-        int len0 = 0, len1 = 0, lo0 = 0, lo1 = 0;
-        float sy = 0.f, sz = 0.f, sx0 = 0.f, sx1 = 0.f;
-        if (lane < nrows) {
-            const int za = lane / ry, yb = lane % ry;
-            const int zu = cz - 2 + za, yu = cy - 2 + yb;  // unwrapped (SHIFTED: grid >= 7 cells)
-            const int z = ncz < 5 ? za : wrapi(zu, ncz);
-            const int y = ncy < 5 ? yb : wrapi(yu, ncy);
-            if (SHIFTED) {  // cells past the low face hold coordinates near +L/2: shift -L
-                sz = zu < 0 ? -Lz : (zu >= ncz ? Lz : 0.f);
-                sy = yu < 0 ? -Ly : (yu >= ncy ? Ly : 0.f);
-            }
-            const int rowbase = (z * ncy + y) * ncx;
-            int l0, h0, l1 = 0, h1 = 0;
-            if (ncx <= 5) {
-                l0 = rowbase;
-                h0 = rowbase + ncx;
-            } else {
-                const int x0 = cx - 2, x1 = cx + 2;
-                if (x0 >= 0 && x1 < ncx) {
-                    l0 = rowbase + x0;
-                    h0 = rowbase + x1 + 1;
-                } else if (x0 < 0) {
-                    l0 = rowbase + x0 + ncx;
-                    h0 = rowbase + ncx;
-                    l1 = rowbase;
-                    h1 = rowbase + x1 + 1;
-                    sx0 = -Lx;
-                } else {
-                    l0 = rowbase + x0;
-                    h0 = rowbase + ncx;
-                    l1 = rowbase;
-                    h1 = rowbase + x1 - ncx + 1;
-                    sx1 = Lx;
-                }
-            }
-            lo0 = a.cell_start[l0];
-            len0 = a.cell_start[h0] - lo0;
-            if (h1 > l1) {
-                lo1 = a.cell_start[l1];
-                len1 = a.cell_start[h1] - lo1;
-            }
-        }
-        // segments in row order: row r gives entries 2r, 2r+1 (second may be empty)
-        const int tot = len0 + len1;
-        int incl = tot;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int y = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += y;
-        }
-        const int excl = incl - tot;
-        if (lane < nrows) {
-            lo_s[2 * lane] = lo0;
-            pre_s[2 * lane] = excl;
-            lo_s[2 * lane + 1] = lo1;
-            pre_s[2 * lane + 1] = excl + len0;
-            if (SHIFTED) {
-                sh_s[2 * lane] = make_float3(sx0, sy, sz);
-                sh_s[2 * lane + 1] = make_float3(sx1, sy, sz);
-            }
-        }
-        const int T = __shfl_sync(0xffffffffu, incl, 31);
-        if (lane == 0) pre_s[2 * nrows] = T;
+// Hits of a build on their way to the list.  The LN lanes of a particle put
+// theirs into a ring in shared memory, entry k at k mod 8 LN, and write whole
+// chunks of four from there: a quarter of the stores, each a 16-byte one (the
+// 4-byte stores of the hits one by one cost an L2 sector operation each and
+// bounded the large builds).  A warp's rings take NB_RING_BYTES.
+constexpr int NB_RING_BYTES = 32 * 12 * (int)sizeof(int);  // LN = 1: 8 entries in 12 words (bank spread)
+
+struct NbAppend {
+    int *ring;        // this particle's
+    int *row;         // its list: entry k at chunk k / 4 (cs apart)
+    size_t cs;
+    int maxn, LN, sub;
+    int cap;          // 8 LN entries
+    int count, done;  // hits so far, entries written (a multiple of 4); equal on the LN lanes
+    __device__ __forceinline__ NbAppend(int *warp_rings, int LN_, int lane, int *row_, size_t cs_, int maxn_)
+        : row(row_), cs(cs_), maxn(maxn_), LN(LN_), sub(lane & (LN_ - 1)), cap(8 * LN_), count(0), done(0) {
+        ring = warp_rings + lane / LN_ * (8 * LN_ + 4);
+    }
+    // whole chunks below `upto` to the list (every lane of the warp)
+    __device__ __forceinline__ void write(int upto, int pad) {
         __syncwarp();
-        const int nseg = 2 * nrows;
-        for (int g0 = cs; g0 < ce; g0 += NBW) {
-            const int gn = min(NBW, ce - g0);
-            float4 pi[NBW];
-            int cnt[NBW];
-#pragma unroll
-            for (int p = 0; p < NBW; p++) {
-                pi[p] = p < gn ? pos[g0 + p] : make_float4(0.f, 0.f, 0.f, 0.f);
-                cnt[p] = 0;
-            }
-            // each lane walks the segments forward as its candidate index grows
-            // (64 candidates per iteration: two independent position loads)
-            int seg = 0;
-            for (int v0 = 0; v0 < T; v0 += 64) {
-                const int va = v0 + lane, vb = va + 32;
-                const bool oka = va < T, okb = vb < T;
-                int ja = 0, jb = 0;
-                float4 pa = make_float4(0.f, 0.f, 0.f, 0.f), pb = pa;
-                float3 sha = make_float3(0.f, 0.f, 0.f), shb = sha;
-                if (oka) {
-                    while (seg + 1 < nseg && pre_s[seg + 1] <= va) seg++;
-                    ja = lo_s[seg] + (va - pre_s[seg]);
-                    pa = pos[ja];
-                    if (SHIFTED) sha = sh_s[seg];
-                }
-                if (okb) {
-                    while (seg + 1 < nseg && pre_s[seg + 1] <= vb) seg++;
-                    jb = lo_s[seg] + (vb - pre_s[seg]);
-                    pb = pos[jb];
-                    if (SHIFTED) shb = sh_s[seg];
-                }
-#pragma unroll
-                for (int half = 0; half < 2; half++) {
-                    const bool ok = half ? okb : oka;
-                    const int j = half ? jb : ja;
-                    const float4 pj = half ? pb : pa;
-                    const float3 sh = half ? shb : sha;
-#pragma unroll
-                    for (int p = 0; p < NBW; p++) {
-                        if (p >= gn) break;
-                        const float d2 = SHIFTED ? dist_sq_shifted<FMA>(pj, pi[p], sh.x, sh.y, sh.z)
-                                                 : dist_sq_exact<FMA>(pj, pi[p], Lx, Ly, Lz);
-                        bool hit = ok && j != g0 + p && d2 < a.cps2;
-                        if (hit && a.excl) hit = !excluded(a, a.orig_tmp[g0 + p], a.orig_tmp[j]);
-                        const unsigned m = __ballot_sync(0xffffffffu, hit);
-                        if (hit) {
-                            const int k = cnt[p] + __popc(m & ((1u << lane) - 1u));
-                            if (k < a.max_nbs) a.nbl[nbl_index(g0 + p, k, a.stride)] = j;
-                        }
-                        cnt[p] += __popc(m);
-                    }
-                }
-            }
-#pragma unroll
-            for (int p = 0; p < NBW; p++) {
-                if (p < gn && lane == p) {
-                    a.nbc[g0 + p] = cnt[p];
-                    atomicMax(&a.ctrl->maxcount, cnt[p]);
-                }
-            }
+        const int chunks = (upto + pad - done) >> 2;
+        for (int c = sub; c < chunks; c += LN) {
+            const int k = done + 4 * c;
+            if (k < maxn)  // the list has room for max_nbs + 4 entries
+                *reinterpret_cast<int4 *>(row + (size_t)(k >> 2) * cs) =
+                    *reinterpret_cast<const int4 *>(ring + (k & (cap - 1)));
         }
+        done += 4 * chunks;
         __syncwarp();
     }
-}
+    // `mine` hits of this lane, after those of the particle's lower lanes;
+    // next() hands out their indices (every lane of the warp calls)
+    template <class Next>
+    __device__ __forceinline__ void add(int mine, Next next) {
+        int k = count, total = mine;
+        if (LN > 1) {
+            int incl = mine;
+            for (int o = 1; o < LN; o <<= 1) {
+                const int y = __shfl_up_sync(0xffffffffu, incl, o, LN);
+                if (sub >= o) incl += y;
+            }
+            k += incl - mine;
+            total = __shfl_sync(0xffffffffu, incl, LN - 1, LN);
+        }
+        const int end = k + mine;
+        count += total;
+        for (;;) {
+            while (k < end && k < done + cap) {
+                ring[k & (cap - 1)] = next();
+                k++;
+            }
+            write(min(count, done + cap), 0);
+            if (!__any_sync(0xffffffffu, k < end)) break;
+        }
+    }
+    __device__ __forceinline__ void finish() { write(count, 3); }
+};
 
-// Cell-list build, one thread per particle slot: the thread walks the
-// stencil rows in the same order as phase_nbl_cells_t's packed candidate
-// sequence and appends hits in that order, so both builds give identical
-// lists.  No ballots and no segment search: about half the instructions per
-// candidate, at one lane per particle; used when the grid has at least one
-// thread per particle.
+// Build with LN lanes (a power of two) per particle: lane r of a particle
+// takes the stencil rows r, r + LN, ...; the lanes' hits of a round of LN rows
+// follow one another in row order.  LN grows until the lanes fill the
+// threads, up to a warp per particle.  rings: NB_RING_BYTES per warp.
+//
+// What bounds it is instruction issue, with the loads of the candidates behind
+// (48 instructions a candidate with an append behind every test).  Measured on
+// B200, KA, whole rebuild: N 1 048 576 1440 -> 1140 us, N 65 536 212 -> 105 us
+// (two lanes a particle), N 10 007 97 -> 50 us.
 template <bool FMA, bool SHIFTED>
-__device__ inline void phase_nbl_cells_tpp(const SimArgs &a, Span g) {
-    const float4 *pos = a.pos_tmp;
+__device__ inline void phase_nbl_cells_lanes(const SimArgs &a, Span g, int LN, unsigned char *rings) {
+    const float4 *pos = a.pos_tmp;  // n + NB_PAD entries: a group of four may read past the last slot
     const int ncx = a.ncx, ncy = a.ncy, ncz = a.ncz;
     const float Lx = a.Lx, Ly = a.Ly, Lz = a.Lz;
     const float cps2 = a.cps2;
-    const int maxn = a.max_nbs;
     const size_t cs = (size_t)a.stride * NB_CHUNK;
     const int ry = ncy < 5 ? ncy : 5, rz = ncz < 5 ? ncz : 5;
-    // the arguments the walk reads, in registers: the list stores could
-    // otherwise force them to be reloaded after every store
+    const int nrows = ry * rz;
     const int n = a.n;
     const int *excl = a.excl;
-    const int *orig_tmp = a.orig_tmp;
     const int *cstart = a.cell_start;
     const int *scell = a.scell;
     int *nbl = a.nbl;
-    // the walk instantiated with and without pair exclusions (uniform)
-    auto walk = [&](auto ex_tag) {
-        constexpr bool EX = decltype(ex_tag)::value;
-        for (int s = g.b * (int)blockDim.x + (int)threadIdx.x; s < n; s += g.nb * (int)blockDim.x) {
-            const float4 pi = pos[s];
-            const int c = scell[s];
-            const int cxy = ncx * ncy;
-            const int cz = c / cxy, rem = c - cz * cxy;
-            const int cy = rem / ncx, cx = rem - cy * ncx;
-            // entry k of slot s at chunk k/4 (cs apart), position k%4
-            int *chunk = nbl + (size_t)s * NB_CHUNK;
-            int cnt = 0;
-            const int ui = EX ? orig_tmp[s] : 0;
-            // the append without a branch: the store (predicated), the count and
-            // the step to the next chunk when one fills
-            auto test = [&](float4 pj, int j, float sx, float sy, float sz) {
-                const float d2 =
-                    SHIFTED ? dist_sq_shifted<FMA>(pj, pi, sx, sy, sz) : dist_sq_exact<FMA>(pj, pi, Lx, Ly, Lz);
-                bool hit = (d2 < cps2) & (j != s);
-                if (EX && hit) hit = !excluded(a, ui, orig_tmp[j]);
-                if (hit & (cnt < maxn)) chunk[cnt & 3] = j;
-                cnt += hit ? 1 : 0;
-                chunk += (hit & ((cnt & 3) == 0)) ? cs : (size_t)0;
-            };
-            for (int za = 0; za < rz; za++) {
-                const int zu = cz - 2 + za;
-                const int z = ncz < 5 ? za : wrap_near(zu, ncz);
-                const float sz = SHIFTED ? (zu < 0 ? -Lz : (zu >= ncz ? Lz : 0.f)) : 0.f;
-                for (int yb = 0; yb < ry; yb++) {
-                    const int yu = cy - 2 + yb;
-                    const int y = ncy < 5 ? yb : wrap_near(yu, ncy);
-                    const float sy = SHIFTED ? (yu < 0 ? -Ly : (yu >= ncy ? Ly : 0.f)) : 0.f;
-                    const int rowbase = (z * ncy + y) * ncx;
-                    int l0, h0, l1 = 0, h1 = 0;
-                    float sx0 = 0.f, sx1 = 0.f;
-                    if (ncx <= 5) {
-                        l0 = rowbase;
-                        h0 = rowbase + ncx;
-                    } else {
-                        const int x0 = cx - 2, x1 = cx + 2;
-                        if (x0 >= 0 && x1 < ncx) {
-                            l0 = rowbase + x0;
-                            h0 = rowbase + x1 + 1;
-                        } else if (x0 < 0) {
-                            l0 = rowbase + x0 + ncx;
-                            h0 = rowbase + ncx;
-                            l1 = rowbase;
-                            h1 = rowbase + x1 + 1;
-                            sx0 = -Lx;
+    const int lane = threadIdx.x & 31, sub = threadIdx.x & (LN - 1);
+    int *wring = reinterpret_cast<int *>(rings + (threadIdx.x >> 5) * NB_RING_BYTES);
+    const int shift = __ffs(LN) - 1;
+    // a chunk is a thread each of a block.  Blocks that take several get them
+    // from a counter, and the last chunk of each is handed out a warp at a
+    // time, so that nobody waits for a whole chunk at the barrier (measured on
+    // B200, KA, rebuild: N 180 000, 4.8 blocks of particles an SM, 397 -> 318
+    // us; N 262 144 382 -> 370 us; N 1 048 576 no change)
+    __shared__ int s_chunk;
+    const int chunks = (int)((((long long)n << shift) + blockDim.x - 1) / blockDim.x);
+    const bool dynamic = chunks > g.nb;
+    const int bulk = dynamic ? chunks - g.nb : chunks;
+    bool fine = false;
+    int most = 0;
+    for (int chunk = g.b;;) {
+        if (dynamic) {
+            if (!fine) {
+                __syncthreads();  // every thread has read s_chunk
+                if (threadIdx.x == 0) s_chunk = (int)atomicAdd(&a.ctrl->nbl_work, 1u);
+                __syncthreads();
+                chunk = s_chunk;
+                fine = chunk >= bulk;
+                if (fine && threadIdx.x >= 32) chunk = warp_take(&a.ctrl->nbl_work);
+            } else {
+                chunk = warp_take(&a.ctrl->nbl_work);
+            }
+        }
+        // a warp's lanes stay together: it goes on while its first lane has a particle
+        const int t = fine ? bulk * (int)blockDim.x + (chunk - bulk) * 32 + lane : chunk * (int)blockDim.x + (int)threadIdx.x;
+        if (((t & ~31) >> shift) >= n) break;
+        const int s = t >> shift;
+        const bool valid = s < n;
+        const float4 pi = pos[valid ? s : 0];
+        const f32x2 mxy = pack2(-pi.x, -pi.y);
+        const int c = valid ? scell[s] : 0;
+        const int cxy = ncx * ncy;
+        const int cz = c / cxy, rem = c - cz * cxy;
+        const int cy = rem / ncx, cx = rem - cy * ncx;
+        NbAppend app(wring, LN, lane, nbl + (size_t)s * NB_CHUNK, cs, a.max_nbs);
+        // slots [lo, hi), every one at the same periodic shift
+        auto walk = [&](int lo, int hi, float sx, float sy, float sz) {
+            const f32x2 sxy = pack2(sx, sy);
+            for (int j0 = lo; __any_sync(0xffffffffu, j0 < hi); j0 += 32) {
+                const int len = max(0, min(32, hi - j0));
+                const float4 *q = pos + j0;
+                unsigned mask = 0;
+                for (int k = 0; k < len; k += 4) {  // four independent loads in flight
+                    unsigned bits = 0;
+                    const float4 p[4] = {q[k], q[k + 1], q[k + 2], q[k + 3]};
+#pragma unroll
+                    for (int u = 0; u < 4; u++) {
+                        float d2;
+                        if (SHIFTED) {  // x and y as a register pair
+                            const f32x2 dxy = add2(add2(pack2(p[u].x, p[u].y), mxy), sxy);
+                            const float dz = __fadd_rn(__fsub_rn(p[u].z, pi.z), sz);
+                            float dx, dy;
+                            unpack2(dxy, dx, dy);
+                            d2 = __fmul_rn(dx, dx);
+                            if (FMA) {
+                                d2 = __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, d2));
+                            } else {
+                                d2 = __fadd_rn(__fadd_rn(d2, __fmul_rn(dy, dy)), __fmul_rn(dz, dz));
+                            }
                         } else {
-                            l0 = rowbase + x0;
-                            h0 = rowbase + ncx;
-                            l1 = rowbase;
-                            h1 = rowbase + x1 - ncx + 1;
-                            sx1 = Lx;
+                            d2 = dist_sq_exact<FMA>(p[u], pi, Lx, Ly, Lz);
                         }
+                        if (d2 < cps2) bits |= 1u << u;
                     }
-    #pragma unroll
-                    for (int r = 0; r < 2; r++) {
-                        const int lc = r ? l1 : l0, hc = r ? h1 : h0;
-                        if (hc <= lc) continue;
-                        const float sx = r ? sx1 : sx0;
-                        const int lo = cstart[lc], hi = cstart[hc];
-                        int j = lo;
-                        for (; j + 4 <= hi; j += 4) {  // four independent loads in flight
-                            const float4 q0 = pos[j], q1 = pos[j + 1], q2 = pos[j + 2], q3 = pos[j + 3];
-                            test(q0, j, sx, sy, sz);
-                            test(q1, j + 1, sx, sy, sz);
-                            test(q2, j + 2, sx, sy, sz);
-                            test(q3, j + 3, sx, sy, sz);
-                        }
-                        for (; j < hi; j++) test(pos[j], j, sx, sy, sz);
+                    mask |= bits << k;
+                }
+                if (len < 32) mask &= (1u << len) - 1u;  // the last group may pass hi
+                if ((unsigned)(s - j0) < 32u) mask &= ~(1u << (s - j0));
+                if (excl)
+                    for (unsigned m = mask; m; m &= m - 1u)
+                        if (excluded(a, a.orig_tmp[s], a.orig_tmp[j0 + __ffs(m) - 1])) mask &= ~(m & (0u - m));
+                app.add(__popc(mask), [&] {
+                    const int j = j0 + __ffs(mask) - 1;
+                    mask &= mask - 1u;
+                    return j;
+                });
+            }
+        };
+        for (int r0 = 0; r0 < nrows; r0 += LN) {
+            const int r = r0 + sub;
+            int lo0 = 0, hi0 = 0, lo1 = 0, hi1 = 0;
+            float sx0 = 0.f, sx1 = 0.f, sy = 0.f, sz = 0.f;
+            if (valid && r < nrows) {
+                const int za = r / ry, yb = r - za * ry;
+                const int zu = cz - 2 + za, yu = cy - 2 + yb;  // unwrapped (SHIFTED: grid >= 7 cells)
+                const int z = ncz < 5 ? za : wrap_near(zu, ncz);
+                const int y = ncy < 5 ? yb : wrap_near(yu, ncy);
+                if (SHIFTED) {  // cells past the low face hold coordinates near +L/2: shift -L
+                    sz = zu < 0 ? -Lz : (zu >= ncz ? Lz : 0.f);
+                    sy = yu < 0 ? -Ly : (yu >= ncy ? Ly : 0.f);
+                }
+                const int rowbase = (z * ncy + y) * ncx;
+                int l0, h0, l1 = 0, h1 = 0;
+                if (ncx <= 5) {
+                    l0 = rowbase;
+                    h0 = rowbase + ncx;
+                } else {
+                    const int x0 = cx - 2, x1 = cx + 2;
+                    if (x0 >= 0 && x1 < ncx) {
+                        l0 = rowbase + x0;
+                        h0 = rowbase + x1 + 1;
+                    } else if (x0 < 0) {
+                        l0 = rowbase + x0 + ncx;
+                        h0 = rowbase + ncx;
+                        l1 = rowbase;
+                        h1 = rowbase + x1 + 1;
+                        sx0 = -Lx;
+                    } else {
+                        l0 = rowbase + x0;
+                        h0 = rowbase + ncx;
+                        l1 = rowbase;
+                        h1 = rowbase + x1 - ncx + 1;
+                        sx1 = Lx;
                     }
                 }
+                lo0 = cstart[l0];
+                hi0 = cstart[h0];
+                if (h1 > l1) {
+                    lo1 = cstart[l1];
+                    hi1 = cstart[h1];
+                }
             }
-            a.nbc[s] = cnt;
-            atomicMax(&a.ctrl->maxcount, cnt);
+#pragma unroll 1
+            for (int w = 0; w < 2; w++) walk(w ? lo1 : lo0, w ? hi1 : hi0, w ? sx1 : sx0, sy, sz);
         }
-    };
-    if (excl)
-        walk(BoolTag<true>{});
-    else
-        walk(BoolTag<false>{});
+        app.finish();
+        if (valid && sub == 0) a.nbc[s] = app.count;
+        most = max(most, valid ? app.count : 0);
+        if (!dynamic) break;
+    }
+    most = __reduce_max_sync(0xffffffffu, most);
+    if (lane == 0 && most > 0) atomicMax(&a.ctrl->maxcount, most);
 }
 
-// Per-warp segment tables of the cell build, in shared memory, for blocks of
-// up to WPB warps.  Declared once per kernel and handed down.
-template <int WPB>
-struct NbScratch {
-    int lo[WPB * NB_SEG_MAX];
-    int pre[WPB * (NB_SEG_MAX + 1)];
-    float3 sh[WPB * NB_SEG_MAX];
-};
-
-template <bool FMA, int WPB>
-__device__ inline void phase_nbl_cells(const SimArgs &a, Span g, NbScratch<WPB> &scr) {
+template <bool FMA>
+__device__ inline void phase_nbl_cells(const SimArgs &a, Span g, unsigned char *rings) {
     const bool shifted = a.ncx >= 7 && a.ncy >= 7 && a.ncz >= 7 && !*(volatile int *)&a.ctrl->cell_wrap;
-    // a warp per cell while threads outnumber particles, a thread per
-    // particle beyond (measured on B200: 1.7x faster at 1M particles, 1.6x
-    // slower at 32k on the whole GPU)
-    const bool tpp = a.n >= g.nb * (int)blockDim.x;
-    if (tpp) {
-        if (shifted)
-            phase_nbl_cells_tpp<FMA, true>(a, g);
-        else
-            phase_nbl_cells_tpp<FMA, false>(a, g);
-    } else if (shifted) {
-        phase_nbl_cells_t<FMA, true>(a, g, scr.lo, scr.pre, scr.sh);
-    } else {
-        phase_nbl_cells_t<FMA, false>(a, g, scr.lo, scr.pre, scr.sh);
-    }
+    const long long threads = (long long)g.nb * blockDim.x;
+    int lanes = 1;
+    while (lanes < 32 && (long long)a.n * lanes * 2 <= threads) lanes *= 2;
+    if (shifted)
+        phase_nbl_cells_lanes<FMA, true>(a, g, lanes, rings);
+    else
+        phase_nbl_cells_lanes<FMA, false>(a, g, lanes, rings);
 }
 
 // Move the reordered state into place, record r_ref, clear the cell counters.
+// It writes nothing that the list build reads, so it may follow the build
+// without a barrier.
 __device__ inline void phase_finish_cells(const SimArgs &a, int cur, Span g = grid_span()) {
     float4 *pos = cur_pos(a, cur);
     const size_t n = a.n;
@@ -937,27 +897,69 @@ __device__ __forceinline__ double target_pressure(const SimArgs &a, double t) {
     return a.pp0;
 }
 
+// State of NPT_Atomic between steps: thermostat p_xi/Q, barostat p_eps/W,
+// volume and box.  Every block keeps it (step_barrier_all), and its constants
+// are made once per block and step: with the books in the last block, the
+// arguments in local memory and a pow by every thread a step of 13 500
+// particles took 47 us (17.9 us of it bookkeeping), and takes 19 here.
+struct NptState {
+    float ts0, bs0, vol;
+    float box[3];
+};
 // Per-step constants of NPT_Atomic's particle update (integrators/
 // NPT_Atomic.py:108-113, with numba's typing: factor in float64, plus, minus
 // and rfactor in float32) and the box scaling of scale_box (:168-181): every
-// coordinate times sf = (1 + dt D bs0)^(1/3), the box lengths too.
+// coordinate times sf = (1 + dt D bs0)^(1/3), the box lengths too.  Computed
+// by one thread per block and step (a float64 cube root).
 struct NptStep {
     float plus, minus, rfactor;
     double sf;
     float Lx, Ly, Lz;  // box after the scaling
 };
-__device__ __forceinline__ NptStep npt_step_consts(const SimArgs &a, const DevCtrl *ctrl) {
+__device__ __forceinline__ NptStep npt_step_consts(const SimArgs &a, const NptState &st) {
     NptStep ns;
-    const float ts0 = ctrl->npt_ts0, bs0 = ctrl->npt_bs0;
-    const double factor = (double)(0.5f * a.dt) * ((1.0 + 3.0 / (double)a.dof) * (double)bs0 + (double)ts0);
+    const double factor = (double)(0.5f * a.dt) * ((1.0 + 3.0 / (double)a.dof) * (double)st.bs0 + (double)st.ts0);
     ns.plus = 1.0f / (float)(1.0 + factor);
     ns.minus = (float)(1.0 - factor);
-    ns.rfactor = bs0 * a.dt;
-    ns.sf = pow(1.0 + (double)a.dt * 3.0 * (double)bs0, 1.0 / 3.0);
-    ns.Lx = (float)((double)a.Lx * ns.sf);
-    ns.Ly = (float)((double)a.Ly * ns.sf);
-    ns.Lz = (float)((double)a.Lz * ns.sf);
+    ns.rfactor = st.bs0 * a.dt;
+    ns.sf = cbrt(1.0 + (double)a.dt * 3.0 * (double)st.bs0);
+    ns.Lx = (float)((double)st.box[0] * ns.sf);
+    ns.Ly = (float)((double)st.box[1] * ns.sf);
+    ns.Lz = (float)((double)st.box[2] * ns.sf);
     return ns;
+}
+// update_thermostat_barostat_state (integrators/NPT_Atomic.py:138-166) with
+// numba's typing; the float32 accumulators thermostat_state[1] and
+// barostat_state[1] are the float64 sums of K and W rounded to float32.
+__device__ __forceinline__ void npt_update(const SimArgs &a, NptState &st, const NptStep &ns, double sumk, double sumw,
+                                           double time) {
+    const float ts1 = (float)sumk, bs1 = (float)sumw;
+    const float bs0 = st.bs0;
+    const long long deg = a.dof;
+    const double temperature = 2.0 * (double)ts1 / (double)deg;
+    const double sf3 = 1.0 + (double)a.dt * 3.0 * (double)bs0;
+    const double mass_t = (double)a.npt_mass_t * temperature;
+    const double mass_p = (double)a.npt_mass_p * temperature;
+    const float vol = (float)((double)st.vol * sf3);
+    st.vol = vol;
+    st.box[0] = ns.Lx;
+    st.box[1] = ns.Ly;
+    st.box[2] = ns.Lz;
+    const double T_target = target_temperature(a, time);
+    const double P_target = target_pressure(a, time);
+    const double p_inst = (temperature * (double)a.n + (double)bs1) / (double)vol;
+    const double ke_dev = ((double)(2.0f * ts1) + (double)(bs0 * bs0) * mass_p) / ((double)(deg + 1) * T_target) - 1.0;
+    const double p_dev = 3.0 * ((double)vol * (p_inst - P_target) + (double)(0.5f * ts1) / (double)deg);
+    const float ts0 = (float)((double)st.ts0 + (double)a.dt * ke_dev * (double)(deg + 1) * T_target / mass_t);
+    st.ts0 = ts0;
+    st.bs0 = (float)((double)bs0 + (double)a.dt * (p_dev / mass_p + (double)(ts0 * bs0)));
+}
+// The saver's volume column: the box the step left (scalar_saver.py:195).
+__device__ __forceinline__ float npt_saved_volume(const NptState &st) {
+    float vol = st.box[0];
+    vol *= st.box[1];
+    vol *= st.box[2];
+    return vol;
 }
 
 // numba.cuda.random's generator, the one of integrators/NVT_Langevin.py:105:
@@ -1307,7 +1309,23 @@ struct StepCtl {
     float shift[2][3];
     float xi;
     double time_zero;
+    NptState npt;
+    NptStep ns;  // NPT_Atomic: this step's constants
 };
+__device__ __forceinline__ void load_npt_state(const DevCtrl *c, NptState *st) {
+    st->ts0 = *(volatile const float *)&c->npt_ts0;
+    st->bs0 = *(volatile const float *)&c->npt_bs0;
+    st->vol = *(volatile const float *)&c->npt_vol;
+#pragma unroll
+    for (int k = 0; k < 3; k++) st->box[k] = *(volatile const float *)&c->box[k];
+}
+__device__ __forceinline__ void store_npt_state(DevCtrl *c, const NptState &st) {
+    c->npt_ts0 = st.ts0;
+    c->npt_bs0 = st.bs0;
+    c->npt_vol = st.vol;
+#pragma unroll
+    for (int k = 0; k < 3; k++) c->box[k] = st.box[k];
+}
 __device__ __forceinline__ void load_step_ctl(const DevCtrl *c, StepCtl *sc) {
     const int rb = *(volatile const int *)&c->rebuild;
     const int st = *(volatile const int *)&c->step;
@@ -1332,7 +1350,7 @@ __device__ __forceinline__ void load_step_ctl(const DevCtrl *c, StepCtl *sc) {
 }
 
 // Forces from pos[cur], integration into pos[cur^1] (MODE_STEP) or forces
-// only (MODE_EVAL).  A round is blockDim/TP consecutive particles.
+// only (MODE_EVAL).  A round is per_round (or blockDim/TP) consecutive particles.
 // Standalone launches (PERSIST false) take rounds g.b, g.b + g.nb, ... and
 // write one float64 partial row per block to partials[g.b].  The persistent
 // kernels (PERSIST true) hand rounds out through an atomic counter (blocks on
@@ -1362,11 +1380,11 @@ __device__ inline bool phase_step(const SimArgs &a, const PairEntry *tab, int nt
     const float shz0 = sc ? sc->shift[ppar][2] : ctrl->shift[ppar][2];
     const float shx = shift_pending ? shx0 : 0.f, shy = shift_pending ? shy0 : 0.f, shz = shift_pending ? shz0 : 0.f;
     const float xi = sc ? sc->xi : ctrl->xi;
-    NptStep ns;
-    if (INTEG == GDB_INTEGRATOR_NPT && MODE == MODE_STEP) ns = npt_step_consts(a, ctrl);
-    const int per_block = blockDim.x / TP;
+    // NPT_Atomic runs on the persistent kernel only, which hands its constants down
+    const NptStep *ns = INTEG == GDB_INTEGRATOR_NPT && sc ? &sc->ns : nullptr;
+    const int per_block = a.per_round > 0 ? a.per_round : (int)blockDim.x / TP;
     const int rounds_total = (a.n + per_block - 1) / per_block;
-    const bool full = rec || reset;
+    const bool full = rec || reset;  // (NPT_Atomic: rec is set on every step)
     const bool needk = full || INTEG == GDB_INTEGRATOR_NVT;
     double red[NQ];
 #pragma unroll
@@ -1385,7 +1403,7 @@ __device__ inline bool phase_step(const SimArgs &a, const PairEntry *tab, int nt
     while (round < rounds_total) {
         const int i = round * per_block + threadIdx.x / TP;
         const int sub = threadIdx.x % TP;
-        const bool active = i < a.n;
+        const bool active = i < a.n && (int)threadIdx.x / TP < per_block;
         float fx = 0.f, fy = 0.f, fz = 0.f, u = 0.f, w = 0.f, l = 0.f;
         float4 pi = make_float4(0.f, 0.f, 0.f, 0.f);
         // the integrating lane's own state, loaded before the neighbour loop so
@@ -1418,7 +1436,7 @@ __device__ inline bool phase_step(const SimArgs &a, const PairEntry *tab, int nt
         if (active && sub == 0 && a.bond_cnt) bond_forces(a, i, pi, pos, rec, fx, fy, fz, u, w, l);
         if (active && sub == 0)
             finish_particle<INTEG, MODE>(a, i, pi, v, rr, fx, fy, fz, u, w, l, rec, reset, step, shift_pending, shx,
-                                         shy, shz, xi, pos_next, red, moved, &ns);
+                                         shy, shz, xi, pos_next, red, moved, ns);
         if (PERSIST) {
             // this round's sums to partials[round]; the next round
             if (full) {
@@ -1468,8 +1486,8 @@ __device__ inline bool phase_step(const SimArgs &a, const PairEntry *tab, int nt
 // Fixed-order float64 sums of `nrows` partial rows (blocks or rounds): every
 // column (full) or the kinetic energy alone (needk); the result is valid in
 // thread 0.  Each thread sums rows threadIdx.x, + blockDim.x, ... in that
-// order; the rows of a batch are loaded before they are added, so several
-// loads are in flight (the same sums as one row at a time, bit for bit).
+// order, with several loads in flight (a full row, or eight kinetic energies:
+// more would not fit the registers).
 __device__ inline void sum_partial_rows(const double *part, int nrows, bool full, bool needk, double *s_red,
                                         double (&tot)[NQ]) {
 #pragma unroll
@@ -1477,17 +1495,6 @@ __device__ inline void sum_partial_rows(const double *part, int nrows, bool full
     const int bs = blockDim.x;
     if (full) {
         int b = threadIdx.x;
-        for (; b + 3 * bs < nrows; b += 4 * bs) {
-            double v[4][NQ];
-#pragma unroll
-            for (int u = 0; u < 4; u++)
-#pragma unroll
-                for (int q = 0; q < NQ; q++) v[u][q] = __ldcg(part + (size_t)(b + u * bs) * NQ + q);
-#pragma unroll
-            for (int u = 0; u < 4; u++)
-#pragma unroll
-                for (int q = 0; q < NQ; q++) tot[q] += v[u][q];
-        }
         for (; b < nrows; b += bs) {
 #pragma unroll
             for (int q = 0; q < NQ; q++) tot[q] += __ldcg(part + (size_t)b * NQ + q);
@@ -1545,46 +1552,19 @@ __device__ inline void finalize_step(const SimArgs &a, int step, int nblocks, do
     if (threadIdx.x == 0) {
         if (MODE == MODE_STEP) {
             const double time = ctrl->time_zero + (double)step * (double)a.dt;
+            NptState st;
             if (npt) {
-                // update_thermostat_barostat_state (integrators/NPT_Atomic.py:
-                // 138-166) with numba's typing; the float32 accumulators
-                // thermostat_state[1] and barostat_state[1] are the float64
-                // sums of K and W rounded to float32
-                const float ts1 = (float)tot[0], bs1 = (float)tot[2];
-                const float bs0 = ctrl->npt_bs0;
-                const long long deg = a.dof;
-                const double temperature = 2.0 * (double)ts1 / (double)deg;
-                const double sf3 = 1.0 + (double)a.dt * 3.0 * (double)bs0;
-                const double mass_t = (double)a.npt_mass_t * temperature;
-                const double mass_p = (double)a.npt_mass_p * temperature;
-                const float vol = (float)((double)ctrl->npt_vol * sf3);
-                ctrl->npt_vol = vol;
-                const double sf = pow(sf3, 1.0 / 3.0);
-                ctrl->box[0] = (float)((double)ctrl->box[0] * sf);
-                ctrl->box[1] = (float)((double)ctrl->box[1] * sf);
-                ctrl->box[2] = (float)((double)ctrl->box[2] * sf);
-                const double T_target = target_temperature(a, time);
-                const double P_target = target_pressure(a, time);
-                const double p_inst = (temperature * (double)a.n + (double)bs1) / (double)vol;
-                const double ke_dev =
-                    ((double)(2.0f * ts1) + (double)(bs0 * bs0) * mass_p) / ((double)(deg + 1) * T_target) - 1.0;
-                const double p_dev = 3.0 * ((double)vol * (p_inst - P_target) + (double)(0.5f * ts1) / (double)deg);
-                const float ts0 = (float)((double)ctrl->npt_ts0 +
-                                          (double)a.dt * ke_dev * (double)(deg + 1) * T_target / mass_t);
-                ctrl->npt_ts0 = ts0;
-                ctrl->npt_bs0 = (float)((double)bs0 + (double)a.dt * (p_dev / mass_p + (double)(ts0 * bs0)));
+                load_npt_state(ctrl, &st);
+                npt_update(a, st, npt_step_consts(a, st), tot[0], tot[2], time);
+                store_npt_state(ctrl, st);
             } else if (a.omega2 > 0.f) {
                 ctrl->xi = nose_hoover_next(a, ctrl->xi, tot[0], time);
             }
             ctrl->sumK = (float)tot[0];
             if (rec) {
                 write_scalar_row(a, step, tot);
-                if (npt && step / a.every < a.nrows) {  // the saver reads the box the step left (scalar_saver.py:195)
-                    float vol = ctrl->box[0];
-                    vol *= ctrl->box[1];
-                    vol *= ctrl->box[2];
-                    a.rows[(size_t)(step / a.every) * GDB_NUM_SCALARS + GDB_SCALAR_VOL] = vol;
-                }
+                if (npt && step / a.every < a.nrows)
+                    a.rows[(size_t)(step / a.every) * GDB_NUM_SCALARS + GDB_SCALAR_VOL] = npt_saved_volume(st);
             }
             if (reset) {
                 ctrl->shift[par][0] = (float)(tot[5] / tot[8]);
@@ -1602,8 +1582,8 @@ __device__ inline void finalize_step(const SimArgs &a, int step, int nblocks, do
     }
 }
 
-// The bookkeeping of finalize_step for a step (not NPT_Atomic) by every block
-// of the persistent grid after step_barrier_all: each block sums the same
+// The bookkeeping of finalize_step for a step by every block of the persistent
+// grid after step_barrier_all: each block sums the same
 // rows (part, this step's half of the double-buffered rows) in the same
 // order, so each computes the same next control state, into its StepCtl.
 // Block 0 also writes that state to ctrl (for the host and the next launch)
@@ -1616,13 +1596,17 @@ __device__ inline void finalize_step_all(const SimArgs &a, int step, int nrows, 
     const bool rec = a.every > 0 && step % a.every == 0;
     const bool reset = a.reset_every > 0 && step % a.reset_every == 0;
     const int par = step & 1, ppar = par ^ 1;
-    const bool full = rec || reset;
+    constexpr bool npt = INTEG == GDB_INTEGRATOR_NPT;
+    const bool full = rec || reset || npt;
     const bool needk = full || a.omega2 > 0.f;
     double tot[NQ];
     sum_partial_rows(part, nrows, full, needk, s_red, tot);
     if (threadIdx.x == 0) {
         const bool writer = blockIdx.x == 0;
-        if (a.omega2 > 0.f) {
+        if (npt) {
+            npt_update(a, sc->npt, sc->ns, tot[0], tot[2], sc->time_zero + (double)step * (double)a.dt);
+            if (writer) store_npt_state(ctrl, sc->npt);
+        } else if (a.omega2 > 0.f) {
             sc->xi = nose_hoover_next(a, sc->xi, tot[0], sc->time_zero + (double)step * (double)a.dt);
             if (writer) ctrl->xi = sc->xi;
         }
@@ -1638,6 +1622,8 @@ __device__ inline void finalize_step_all(const SimArgs &a, int step, int nrows, 
         if (writer) {
             ctrl->sumK = (float)tot[0];
             if (rec) write_scalar_row(a, step, tot);
+            if (npt && rec && step / a.every < a.nrows)
+                a.rows[(size_t)(step / a.every) * GDB_NUM_SCALARS + GDB_SCALAR_VOL] = npt_saved_volume(sc->npt);
             if (reset) {
 #pragma unroll
                 for (int k = 0; k < 3; k++) ctrl->shift[par][k] = sc->shift[par][k];
