@@ -30,8 +30,8 @@ class SimulationBatch:
     most 256, up to 16 CTAs per system; 0 = the single-system default, so
     every system gives the same bits as alone); ``clg_particles_per_cta`` and
     ``clg_tp`` the global-memory clusters of larger systems (particles per
-    1024-thread CTA, 0 = fit one wave; lanes per particle, 0 = 1).
-    ``autotune`` picks all three by timing.
+    1024-thread CTA, 0 = fit one wave; lanes per particle, 0 = as many as its
+    threads give every particle).  ``autotune`` picks all three by timing.
     """
 
     def __init__(self, simulations, particles_per_cta=0, clg_particles_per_cta=0, clg_tp=0):
