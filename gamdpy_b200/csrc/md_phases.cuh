@@ -1035,8 +1035,11 @@ struct PairBox {
 // adding and subtracting 1.5 2^23 (|d/L| is far below 2^22): the rounding
 // instruction runs at an eighth of the add's rate and three of them a pair
 // bound the force loop.  x and y take one packed instruction per operation.
-// Only the additions depend on the pair being in range (predicated, no branch),
-// so the reciprocals of the pairs in flight overlap.  Measured on B200, KA
+// Only the additions depend on the pair being in range, so the reciprocals of
+// the pairs in flight overlap; a particle without a position (NaN) adds nothing
+// to its neighbours (measured: with one type as products with zero, LJ N 2048
+// 8.1 us a step against 8.4 with the condition; with two types as the
+// condition, KA N 65 536 35.4 us against 36.6).  Measured on B200, KA
 // N 1 048 576: the force phase of a step 300 us with rintf (46 instructions a
 // pair) and a branch, 243 here, bound by the gathers of the positions.
 template <bool REC, int NT>
@@ -1058,8 +1061,13 @@ __device__ __forceinline__ void pair_force(const PairRow<NT> &pr, const PairBox 
     const float x2 = c * inv2;
     const float x6 = x2 * x2 * x2;
     const float x12 = x6 * x6;
-    const float s = (cs12 * x12 + cs6 * x6) * inv2 - sc;
-    if (in) {
+    float s = (cs12 * x12 + cs6 * x6) * inv2 - sc;
+    if (NT == 1) {  // (one type: s = 0 out of range, and the minimum turns a NaN into a number for 0 to multiply)
+        if (!in) s = 0.f;
+        fx -= fminf(dx, 3e38f) * s;
+        fy -= fminf(dy, 3e38f) * s;
+        fz -= fminf(dz, 3e38f) * s;
+    } else if (in) {
         fx -= dx * s;
         fy -= dy * s;
         fz -= dz * s;
