@@ -362,8 +362,8 @@ __device__ __forceinline__ int rdf_cell(float r, float L, int nc) {
 // minimum image leaves unchanged.  When any position lies outside [-L/2, L/2]
 // (*outside set by the binning) every unit takes the minimum image.
 //
-// What bounds it is instruction issue: about 9 instructions a candidate in
-// the first pass and 20 a hit in the second.  Measured on B200, LJ, 1 000 188
+// What bounds it is instruction issue (69 % of the slots), then the shared
+// memory that the two passes go through (59 % of its rate).  Measured on B200, LJ, 1 000 188
 // particles, r_max 5, 1000 bins: a call 3.80 ms with a warp per cell and hits
 // compacted into a ring for a float64 bin, 1.41 ms here.
 template <bool FMA>
@@ -635,9 +635,8 @@ __global__ void __launch_bounds__(SQ_THREADS) k_sq(SqArgs a) {
 // products with the run's SQ_Z factors, so a term costs two packed
 // multiply-adds and 10 bytes of shared memory, against two complex products
 // and 24 bytes in k_sq.  float32 within a tile of SQ_TILE particles, float64
-// across tiles, as k_sq.  What bounds it is the issue of those multiply-adds
-// and of the 6 shared loads a run, then the latency of a particle's loads at
-// 20 warps.  Measured on B200 with 1 000 188 particles and 3778 q-vectors in
+// across tiles, as k_sq.  What bounds it is the 6 shared loads a run (76 % of
+// the shared memory's rate; 60 % of the issue slots).  Measured on B200 with 1 000 188 particles and 3778 q-vectors in
 // an octant: a call 4.04 ms with k_sq, 1.51 here, 1.34 of it this kernel; with
 // one table and two barriers a tile 1.38, with two items a thread (320
 // threads) 1.57 to 1.85, with two blocks an SM at 48 registers 1.59.
