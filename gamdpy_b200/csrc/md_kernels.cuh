@@ -37,7 +37,7 @@ __global__ void __launch_bounds__(GDB_BLOCK, GDB_STEP_MINBLOCKS(TP)) k_step(SimA
     if (threadIdx.x == 0) s_last = atomicAdd(&ctrl->ticket, 1u) == gridDim.x - 1;
     __syncthreads();
     if (!s_last) return;
-    finalize_step<MODE>(a, step, gridDim.x, s_red);
+    finalize_step<MODE>(a, step, a.partials, gridDim.x, s_red);
     if (threadIdx.x == 0) ctrl->ticket = 0;
 }
 
@@ -157,8 +157,8 @@ __device__ inline void run_steps(const SimArgs &a0, const PairEntry *s_tab, int 
     __shared__ int s_any;  // a particle moved beyond skin/2 (the block running `last`, or every block)
     // a grid of at most BAR_FLAT_MAX blocks: every block keeps the books of a
     // step (step_barrier_all, finalize_step_all), on rows double-buffered by
-    // step parity, as a block may write the next step's rows while another
-    // still sums this step's
+    // step parity, as a block may write the next step's rows (or the closing
+    // evaluation's) while another still sums this step's
     const bool all = Sync::kGrid && a.bar_all && (int)gridDim.x <= BAR_FLAT_MAX;
     unsigned seq = 0;  // step barriers of this launch
     for (int s = 0; s < nsteps + do_eval; s++) {
@@ -186,8 +186,8 @@ __device__ inline void run_steps(const SimArgs &a0, const PairEntry *s_tab, int 
             if (!ok) return;
         }
         bool ok;
+        double *part = a.partials + (all ? (size_t)(step & 1) * rounds * NQ : 0);
         if (s < nsteps) {
-            double *part = all ? a.partials + (size_t)(step & 1) * rounds * NQ : nullptr;
             const bool moved = phase_step<TP, NT, INTEG, MODE_STEP, false, true>(a, s_tab, nt, cur, step, s_red, g,
                                                                                    &s_ctl, part);
             trace_mark(ctrl, TR_STEP_PHASE);
@@ -198,7 +198,7 @@ __device__ inline void run_steps(const SimArgs &a0, const PairEntry *s_tab, int 
                 ok = sync(
                     ctrl,
                     [&] {
-                        finalize_step<MODE_STEP, INTEG>(a, step, rounds, s_red);
+                        finalize_step<MODE_STEP, INTEG>(a, step, part, rounds, s_red);
                         if (threadIdx.x == 0 && s_any) ctrl->rebuild = 1;
                     },
                     moved, &s_any);
@@ -206,9 +206,9 @@ __device__ inline void run_steps(const SimArgs &a0, const PairEntry *s_tab, int 
             cur ^= 1;
             trace_mark(ctrl, TR_STEP);
         } else {
-            phase_step<TP, NT, INTEG, MODE_EVAL, false, true>(a, s_tab, nt, cur, step, s_red, g, &s_ctl);
+            phase_step<TP, NT, INTEG, MODE_EVAL, false, true>(a, s_tab, nt, cur, step, s_red, g, &s_ctl, part);
             ok = sync(ctrl, [&] {
-                finalize_step<MODE_EVAL>(a, step, rounds, s_red);
+                finalize_step<MODE_EVAL>(a, step, part, rounds, s_red);
                 if (threadIdx.x == 0) ctrl->work[(step + 1) & 1] = 0;
             });
             trace_mark(ctrl, TR_EVAL);
@@ -281,7 +281,7 @@ __global__ void __launch_bounds__(BRICK_THREADS, 2)
             if (!phase_step_bricks<NT, INTEG, MODE_STEP, true>(a, bs, pp, s_tab, tab.nt, cur, step)) return;
             trace_mark(ctrl, TR_STEP_PHASE);
             ok = sync(ctrl, [&] {
-                finalize_step<MODE_STEP>(a, step, nbricks, s_red);
+                finalize_step<MODE_STEP>(a, step, a.partials, nbricks, s_red);
                 if (threadIdx.x == 0 && ctrl->rebuild_next) {
                     ctrl->rebuild = 1;
                     ctrl->rebuild_next = 0;
@@ -292,7 +292,7 @@ __global__ void __launch_bounds__(BRICK_THREADS, 2)
         } else {
             if (!phase_step_bricks<NT, INTEG, MODE_EVAL, true>(a, bs, pp, s_tab, tab.nt, cur, step)) return;
             ok = sync(ctrl, [&] {
-                finalize_step<MODE_EVAL>(a, step, nbricks, s_red);
+                finalize_step<MODE_EVAL>(a, step, a.partials, nbricks, s_red);
                 if (threadIdx.x == 0) ctrl->work[(step + 1) & 1] = 0;
             });
             trace_mark(ctrl, TR_EVAL);
@@ -321,7 +321,7 @@ __global__ void __launch_bounds__(BRICK_THREADS, 2) k_step_bricks(SimArgs a, Pai
     if (threadIdx.x == 0) s_last = atomicAdd(&ctrl->ticket, 1u) == gridDim.x - 1;
     __syncthreads();
     if (!s_last) return;
-    finalize_step<MODE>(a, step, a.nbx * a.nby * a.nbz, s_red);
+    finalize_step<MODE>(a, step, a.partials, a.nbx * a.nby * a.nbz, s_red);
     if (threadIdx.x == 0) ctrl->ticket = 0;
 }
 

@@ -1543,11 +1543,11 @@ __device__ __forceinline__ void write_scalar_row(const SimArgs &a, int step, con
     row[GDB_SCALAR_FSQ] = tot[4];
 }
 
-// Fixed-order float64 sum of `nblocks` partial rows (blocks or rounds) and the
-// bookkeeping of a finished step (NVT.py:113-124, scalar_saver.py:165-179,
+// Fixed-order float64 sum of the `nblocks` partial rows at `part` (blocks or
+// rounds) and the bookkeeping of a finished step (NVT.py:113-124, scalar_saver.py:165-179,
 // momentum_reset.py:64-78).  Run by one whole block.
 template <int MODE, int INTEG = GDB_INTEGRATOR_NVE>
-__device__ inline void finalize_step(const SimArgs &a, int step, int nblocks, double *s_red) {
+__device__ inline void finalize_step(const SimArgs &a, int step, const double *part, int nblocks, double *s_red) {
     DevCtrl *ctrl = a.ctrl;
     const bool rec = MODE == MODE_EVAL || (a.every > 0 && step % a.every == 0);
     const bool reset = MODE == MODE_STEP && a.reset_every > 0 && step % a.reset_every == 0;
@@ -1556,7 +1556,7 @@ __device__ inline void finalize_step(const SimArgs &a, int step, int nblocks, do
     const bool full = rec || reset || npt;
     const bool needk = full || a.omega2 > 0.f;
     double tot[NQ];
-    sum_partial_rows(a.partials, nblocks, full, needk, s_red, tot);
+    sum_partial_rows(part, nblocks, full, needk, s_red, tot);
     if (threadIdx.x == 0) {
         if (MODE == MODE_STEP) {
             const double time = ctrl->time_zero + (double)step * (double)a.dt;

@@ -498,6 +498,36 @@ def test_step_barrier_forms_agree_bit_for_bit(monkeypatch, n, lanes, cap):
         assert np.array_equal(a, b)
 
 
+@pytest.mark.parametrize("ensemble", ["NVT", "NPT"])
+@pytest.mark.parametrize("cells, steps", [(8, 1), (8, 7), (13, 1), (14, 5), (17, 3)])
+def test_odd_blocks_in_both_barrier_forms(monkeypatch, cells, steps, ensemble):
+    """Blocks of an odd number of steps: the closing evaluation writes its rows beside the last step's, which a
+    slower block may still be summing.  Both barrier forms give the same state, scalars and thermostat bit for
+    bit, block after block."""
+    monkeypatch.setenv("GDB_CLUSTER", "0")
+    outs = []
+    for mode in ("1", "0"):
+        monkeypatch.setenv("GDB_STEP_BARRIER", mode)
+        c = workloads.lj_configuration([cells] * 3, 0.754289, 2.0, seed=cells, compute_flags={"Vol": True})
+        c.randomize_velocities(temperature=2.0, seed=cells)
+        pp = gp.PairPotential(gp.apply_shifted_force_cutoff(gp.LJ_12_6_sigma_epsilon), params=[1.0, 1.0, 2.5],
+                              max_num_nbs=300)
+        if ensemble == "NVT":
+            integ = gp.integrators.NVT(2.0, 0.2, 0.004)
+        else:
+            integ = gp.integrators.NPT_Atomic(temperature=2.0, tau=0.4, pressure=4.7, tau_p=20.0, dt=0.004)
+        sim = gp.Simulation(c, pp, integ, [gp.ScalarSaver(1)] if steps > 1 else [], num_timeblocks=12,
+                            steps_per_timeblock=steps,
+                            compute_plan={"pb": 64, "tp": 1, "skin": 0.5, "nblist": "linked lists"}, storage="memory")
+        for _ in sim.run_timeblocks():
+            pass
+        assert sim._sim.last_path() == 1
+        outs.append((c["r"].copy(), c["v"].copy(), integ.thermostat_state.copy(), np.array(c.simbox.lengths),
+                     np.array(sim.output["scalars"]) if steps > 1 else np.zeros(1)))
+    for a, b in zip(*outs):
+        assert np.array_equal(a, b)
+
+
 def test_nve_energy_conservation():
     """tests/test_LJ_nxyz.py:10-111 of the reference: LJ rho 0.8442, T0 1.44,
     shifted force, dt 0.005, 2 x 4096 steps: var(E)/N < 1e-4 and
