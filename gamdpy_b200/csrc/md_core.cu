@@ -485,6 +485,7 @@ static int ensure_partials(gdb_sim *h, int nblocks) {
     if (nblocks > h->partial_cap) {
         if (h->partials) cudaFree(h->partials);
         h->partials = nullptr;
+        h->partial_cap = 0;
         CK(cudaMalloc(&h->partials, (size_t)nblocks * NQ * sizeof(double)));
         h->partial_cap = nblocks;
         free_graphs(h);
@@ -636,9 +637,11 @@ static int step_lanes(const gdb_sim *h) {
     return tp;
 }
 
+static int step_grid(const gdb_sim *h) { return grid_for((long long)h->n * step_lanes(h)); }
+
 static int enqueue_step(gdb_sim *h, int mode) {
     const int tp = step_lanes(h);
-    const int grid = grid_for((long long)h->n * tp);
+    const int grid = step_grid(h);
     int rc = ensure_partials(h, grid);
     if (rc) return rc;
     const SimArgs a = make_args(h);
@@ -1575,7 +1578,9 @@ int gdb_sim_run(gdb_sim *h, double time_zero, int steps, float *ms) {
         free_graphs(h);
     }
     if (rows > 0) CK(cudaMemsetAsync(h->rows, 0, (size_t)rows * GDB_NUM_SCALARS * sizeof(double), h->st));
-    if ((rc = ensure_partials(h, grid_for((long long)h->n * h->tp)))) return rc;
+    // the standalone steps' rows before any capture: build_graph may not
+    // allocate (launch_run reserves the persistent kernel's)
+    if ((rc = ensure_partials(h, step_grid(h)))) return rc;
     CK(cudaMemsetAsync(&h->ctrl->maxcount, 0, sizeof(int), h->st));
     CK(cudaEventRecord(h->ev0, h->st));
     k_block_begin<<<1, 1, 0, h->st>>>(h->ctrl, time_zero);
@@ -1730,8 +1735,7 @@ int gdb_time_step_kernel(gdb_sim *h, int reps, float *ms_per_launch) {
         *ms_per_launch = ms / reps;
         return GDB_OK;
     }
-    const int grid = grid_for((long long)h->n * h->tp);
-    if ((rc = ensure_partials(h, grid))) return rc;
+    if ((rc = ensure_partials(h, step_grid(h)))) return rc;
     // a list for the current positions, then `reps` step kernels alone
     if ((rc = enqueue_rebuild(h))) return rc;
     k_block_begin<<<1, 1, 0, h->st>>>(h->ctrl, 0.0);

@@ -77,3 +77,24 @@ def test_exclusions_on_every_build(oracle, n, kind):
     c1, f1 = sorted_rows(sim.nblist(300))
     c2, f2 = sorted_rows(ref)
     assert np.array_equal(c1, c2) and np.array_equal(f1, f2)
+
+
+@pytest.mark.parametrize("n", [2048, 10007, 37889])
+def test_first_run_through_graphs(oracle, n, monkeypatch):
+    """Without the persistent kernel, the first run of a handle captures its steps into a graph, where nothing can be
+    allocated; sizes whose standalone step has more lanes than the persistent kernel's.  Against that kernel after 32
+    steps: coordinates to 1e-4 (an ulp of a coordinate here is 1e-6 and either path rounds them 32 times)."""
+    conf = workloads.ka_configuration(n, seed=n)
+    L = np.asarray(conf.simbox.lengths, np.float32)
+    monkeypatch.setenv("GDB_CLUSTER", "0")
+    out = []
+    for persistent in ("0", "1"):
+        monkeypatch.setenv("GDB_PERSISTENT", persistent)
+        sim = make_sim(conf["r"], L, conf.ptype, _table(oracle), nblist=_lib.NBLIST_CELLS, skin=SKIN, v=conf["v"])
+        sim.set_nvt(0.005, 0.2, _lib.TFUNC_CONSTANT, [0.45])
+        sim.run(0.0, 32)
+        assert sim.last_path() == int(persistent)
+        out.append(sim.download()["r"])
+    d = out[0] - out[1]
+    d -= L * np.round(d / L)
+    assert np.abs(d).max() < 1e-4
