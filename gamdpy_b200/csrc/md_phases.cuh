@@ -537,8 +537,15 @@ __device__ inline void phase_scatter(const SimArgs &a, Span g = grid_span()) {
 // user indices (the atomics of the assignment rank them arbitrarily; this
 // makes the layout and every sum deterministic).  A particle counts the
 // members of its cell below it, so ordering and moving take one phase.
+// Where the assignment's counts were wrong (phase_scatter has then met a slot
+// past the last one), particles stay in their slots: every slot is written,
+// and the build makes empty lists of them.
+__device__ __forceinline__ bool bad_index(const SimArgs &a) {
+    return (*(volatile unsigned *)&a.ctrl->status & GDB_STATUS_BAD_INDEX) != 0u;
+}
 __device__ inline void phase_place(const SimArgs &a, int cur, Span g = grid_span()) {
     if (g.b == 0 && threadIdx.x == 0) a.ctrl->nbl_work = 0;  // the build follows a barrier later
+    const bool stay = bad_index(a);
     const float4 *pos = cur_pos(a, cur);
     const size_t n = a.n;
     for (int i = g.b * (int)blockDim.x + (int)threadIdx.x; i < a.n; i += g.nb * (int)blockDim.x) {
@@ -548,18 +555,21 @@ __device__ inline void phase_place(const SimArgs &a, int cur, Span g = grid_span
         // K and Fsq travel with the particle; U, W, lapU are rewritten by the
         // next force evaluation
         const float kin = a.pscal[3 * n + i], fsq = a.pscal[4 * n + i];
-        const int lo = a.cell_start[c], hi = a.cell_start[c + 1];
-        int s = lo;
-        for (int x = lo; x < hi; x++) {
-            const int m = a.perm[x];
-            if ((unsigned)m < (unsigned)a.n)
-                s += a.orig[m] < key ? 1 : 0;
-            else
+        int s = i;
+        if (!stay) {
+            const int lo = a.cell_start[c], hi = a.cell_start[c + 1];
+            s = lo;
+            for (int x = lo; x < hi; x++) {
+                const int m = a.perm[x];
+                if ((unsigned)m < (unsigned)a.n)
+                    s += a.orig[m] < key ? 1 : 0;
+                else
+                    atomicOr(&a.ctrl->status, GDB_STATUS_BAD_INDEX);
+            }
+            if ((unsigned)s >= (unsigned)a.n) {
                 atomicOr(&a.ctrl->status, GDB_STATUS_BAD_INDEX);
-        }
-        if ((unsigned)s >= (unsigned)a.n) {
-            atomicOr(&a.ctrl->status, GDB_STATUS_BAD_INDEX);
-            continue;
+                s = i;
+            }
         }
         a.pos_tmp[s] = p;
         a.vel_tmp[s] = v;
@@ -839,7 +849,12 @@ __device__ inline void phase_nbl_cells_lanes(const SimArgs &a, Span g, int LN, u
 
 template <bool FMA>
 __device__ inline void phase_nbl_cells(const SimArgs &a, Span g, unsigned char *rings) {
-    const bool shifted = a.ncx >= 7 && a.ncy >= 7 && a.ncz >= 7 && !*(volatile int *)&a.ctrl->cell_wrap;
+    const bool wrap = *(volatile int *)&a.ctrl->cell_wrap != 0;
+    if (bad_index(a)) {  // the cells' slot ranges cannot be trusted
+        for (int s = g.b * (int)blockDim.x + (int)threadIdx.x; s < a.n; s += g.nb * (int)blockDim.x) a.nbc[s] = 0;
+        return;
+    }
+    const bool shifted = a.ncx >= 7 && a.ncy >= 7 && a.ncz >= 7 && !wrap;
     const long long threads = (long long)g.nb * blockDim.x;
     int lanes = 1;
     while (lanes < 32 && (long long)a.n * lanes * 2 <= threads) lanes *= 2;
