@@ -937,7 +937,9 @@ __device__ __forceinline__ NptStep npt_step_consts(const SimArgs &a, const NptSt
     ns.plus = 1.0f / (float)(1.0 + factor);
     ns.minus = (float)(1.0 - factor);
     ns.rfactor = st.bs0 * a.dt;
-    ns.sf = cbrt(1.0 + (double)a.dt * 3.0 * (double)st.bs0);
+    // (1 + dt D bs0)^(1/3), which is NaN for a runaway barostat's negative base
+    const double sf3 = 1.0 + (double)a.dt * 3.0 * (double)st.bs0;
+    ns.sf = sf3 < 0.0 ? __longlong_as_double(0x7ff8000000000000LL) : cbrt(sf3);
     ns.Lx = (float)((double)st.box[0] * ns.sf);
     ns.Ly = (float)((double)st.box[1] * ns.sf);
     ns.Lz = (float)((double)st.box[2] * ns.sf);

@@ -174,3 +174,16 @@ def test_saved_boxes_of_a_fixed_box():
     boxes = sim.output["sim_box"]
     assert boxes.shape == (2, 6, 3)
     assert np.array_equal(boxes, np.broadcast_to(conf.simbox.lengths, boxes.shape))
+
+
+def test_runaway_barostat_leaves_no_box():
+    """1 + dt D bs0 < 0: scale_box's cube root (integrators/NPT_Atomic.py:168-181) is NaN, so the run ends with an
+    error and the box is NaN, not a box of negative lengths."""
+    conf = workloads.lj_configuration([6, 6, 6], 0.9, 1.5, seed=1)
+    sim, _ = npt_sim(conf, 1.5, 0.4, 2.0, 2.0, 0.004, "N squared", 0.5, 1, 16, 4)
+    ts, bs = sim._sim.npt_state()
+    bs[0] = -1000.0
+    sim._sim.set_npt_state(ts, bs)
+    with pytest.raises(Exception, match="runaway"):
+        sim._sim.run(0.0, 1)
+    assert np.all(np.isnan(sim._sim.box()))
