@@ -458,7 +458,9 @@ struct SweepArgs {
 constexpr int ADJ_RING = 64;
 constexpr size_t ADJ_RING_BYTES = ADJ_RING * sizeof(float4);  // displacement r_j - r_i, and j << 2 | t_j
 
-template <int NT>
+// LONG: columns may hold more than 64 rows (where they cannot, the test of it
+// in every round cost 1.4 % of observables and gradient at KA N 4096).
+template <int NT, bool LONG>
 __global__ void __launch_bounds__(ADJ_WARPS * 32, 1) k_adj_sweep(AdjArgs a, const __grid_constant__ Tables tab,
                                                                  SweepArgs f) {
     __shared__ Tab64 s_tab[ADJ_MAXT * ADJ_MAXT];
@@ -574,10 +576,11 @@ __global__ void __launch_bounds__(ADJ_WARPS * 32, 1) k_adj_sweep(AdjArgs a, cons
                 head += take;
                 __syncwarp();
             };
-            // 64 rows of the columns at a time: first the lanes' hits as bits
-            // (same float32 displacement and cutoff test as the forward), then
-            // round by round every lane's next hit into the ring, so the order
-            // of the sums does not depend on what the list holds beyond the
+            // each lane's hits in its column as bits, 64 rows at a time (same
+            // float32 displacement and cutoff test as the forward), then round
+            // by round every lane's next hit into the ring.  A lane out of hits
+            // looks further down its column within the round, so the order of
+            // the sums does not depend on what the list holds beyond the
             // cutoff, nor on when it was built
             auto pair = [&](int j, float4 p, float &dx, float &dy, float &dz) {
                 dx = mic_rint(p.x - pi.x, a.Lx, iLx);
@@ -585,14 +588,16 @@ __global__ void __launch_bounds__(ADJ_WARPS * 32, 1) k_adj_sweep(AdjArgs a, cons
                 dz = mic_rint(p.z - pi.z, a.Lz, iLz);
                 return dx * dx + dy * dy + dz * dz;
             };
-            for (int c00 = 0; __any_sync(0xffffffffu, c00 < cnt); c00 += 64) {
-                unsigned long long hits = 0ull;
-                const int end = min(cnt, c00 + 64);
-                for (int c0 = c00; c0 < end; c0 += 4) {
+            unsigned long long hits = 0ull;  // of the rows from base to next
+            int base = 0, next = 0;
+            auto look = [&] {
+                base = next;
+                next = min(cnt, base + 64);
+                for (int c0 = base; c0 < next; c0 += 4) {
                     int j[4];
                     float4 p[4];
 #pragma unroll
-                    for (int q = 0; q < 4; q++) j[q] = c0 + q < end ? lst[(c0 + q) * ADJ_LANES] : i;
+                    for (int q = 0; q < 4; q++) j[q] = c0 + q < next ? lst[(c0 + q) * ADJ_LANES] : i;
 #pragma unroll
                     for (int q = 0; q < 4; q++) p[q] = pos[j[q]];
                     unsigned bits = 0;
@@ -600,29 +605,32 @@ __global__ void __launch_bounds__(ADJ_WARPS * 32, 1) k_adj_sweep(AdjArgs a, cons
                     for (int q = 0; q < 4; q++) {
                         float dx, dy, dz;
                         const float d2 = pair(j[q], p[q], dx, dy, dz);
-                        if (c0 + q < end && d2 < s_tab[ti * nt + type_of(p[q])].cut2) bits |= 1u << q;
+                        if (c0 + q < next && d2 < s_tab[ti * nt + type_of(p[q])].cut2) bits |= 1u << q;
                     }
-                    hits |= (unsigned long long)bits << (c0 - c00);
+                    hits |= (unsigned long long)bits << (c0 - base);
                 }
-                while (__any_sync(0xffffffffu, hits != 0ull) || tail > head) {
-                    const bool hit = hits != 0ull;
-                    const unsigned m = __ballot_sync(0xffffffffu, hit);
-                    if (hit) {
-                        const int j = lst[(c00 + __ffsll(hits) - 1) * ADJ_LANES];
-                        hits &= hits - 1ull;
-                        const float4 p = pos[j];
-                        float dx, dy, dz;
-                        pair(j, p, dx, dy, dz);
-                        ring[(tail + __popc(m & below)) & (ADJ_RING - 1)] =
-                            make_float4(dx, dy, dz, __int_as_float((j << 2) | type_of(p)));
-                    }
-                    tail += __popc(m);
-                    // a full round, or after the last hits what is left
-                    if (tail - head >= 32 || (m == 0u && !__any_sync(0xffffffffu, end < cnt)))
-                        drain(min(32, tail - head));
-                    else if (m == 0u)
-                        break;
+            };
+            look();
+            for (;;) {
+                if (LONG)
+                    while (hits == 0ull && next < cnt) look();
+                const bool hit = hits != 0ull;
+                const unsigned m = __ballot_sync(0xffffffffu, hit);
+                if (hit) {
+                    const int j = lst[(base + __ffsll(hits) - 1) * ADJ_LANES];
+                    hits &= hits - 1ull;
+                    const float4 p = pos[j];
+                    float dx, dy, dz;
+                    pair(j, p, dx, dy, dz);
+                    ring[(tail + __popc(m & below)) & (ADJ_RING - 1)] =
+                        make_float4(dx, dy, dz, __int_as_float((j << 2) | type_of(p)));
                 }
+                tail += __popc(m);
+                // a full round, or after the last hits what is left
+                if (tail - head >= 32 || (m == 0u && tail > head))
+                    drain(min(32, tail - head));
+                else if (m == 0u)
+                    break;
             }
             if (rdf && ti == 0) {
                 const double rg_lo = (double)a.r_lo - ADJ_KW * a.width,
@@ -811,10 +819,14 @@ int rdf_copies(const gdb_adj *h) {
     return std::max(1, std::min(8, (int)(96 * 1024 / ((size_t)std::max(h->nbins, 1) * 32 * 8))));
 }
 
+template <bool LONG>
 const void *sweep_kernel(const gdb_adj *h) {
-    return h->nt == 1   ? (const void *)k_adj_sweep<1>
-           : h->nt == 2 ? (const void *)k_adj_sweep<2>
-                        : (const void *)k_adj_sweep<ADJ_MAXT>;
+    return h->nt == 1   ? (const void *)k_adj_sweep<1, LONG>
+           : h->nt == 2 ? (const void *)k_adj_sweep<2, LONG>
+                        : (const void *)k_adj_sweep<ADJ_MAXT, LONG>;
+}
+const void *sweep_kernel(const gdb_adj *h) {
+    return h->maxnb / ADJ_LANES > 64 ? sweep_kernel<true>(h) : sweep_kernel<false>(h);
 }
 
 // One block per SM at most, of as few warps as give every particle one (more
@@ -828,8 +840,11 @@ cudaError_t launch_shape(gdb_adj *h) {
     h->blocks = std::min(sms, (h->n + warps - 1) / warps);
     const int most = 96 * 1024 + ADJ_MAXB * 32 * 8;
     if ((e = cudaFuncSetAttribute(k_adj_forward, cudaFuncAttributeMaxDynamicSharedMemorySize, most))) return e;
-    return cudaFuncSetAttribute(sweep_kernel(h), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)(ADJ_WARPS * ADJ_RING_BYTES));
+    for (const void *fn : {sweep_kernel<false>(h), sweep_kernel<true>(h)})
+        if ((e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)(ADJ_WARPS * ADJ_RING_BYTES))))
+            return e;
+    return cudaSuccess;
 }
 
 // Zero the barrier words and launch one cooperative kernel.

@@ -95,3 +95,21 @@ def test_adjoint_kept_states_equal_checkpoints(monkeypatch, n, every):
         out.append((obs, eng.backward(np.linspace(0.5, 1.5, len(obs))), *eng.final_state()))
     for a, b in zip(*out):
         assert np.isfinite(a).all() and np.array_equal(a, b)
+
+
+def test_adjoint_long_columns_keep_their_order(monkeypatch):
+    """A cutoff near half the box: list columns of more than 64 entries, most lanes' hits and skin entries on both sides
+    of that boundary.  Segments of 11 steps rebuild their lists at other steps than the kept states' sweep; the sums
+    are the same, bit for bit."""
+    conf = workloads.lj_configuration([10, 10, 10], 0.85, 2.0, seed=3)
+    conf.randomize_velocities(temperature=2.0, seed=3)
+    theta = adjoint.theta_from_tables([[1.0]], [[1.0]])
+    out = []
+    for keep in (None, "0"):
+        if keep is not None:
+            monkeypatch.setenv("GDB_ADJ_KEEP_BYTES", keep)
+        eng = adjoint.AdjointNVE(conf, [[8.2]], dt=0.004, steps=60, checkpoint_every=11)
+        obs = eng.forward(theta)
+        out.append((obs, eng.backward(np.array([0.5, 1.0, 1.5])), *eng.final_state()))
+    for a, b in zip(*out):
+        assert np.isfinite(a).all() and np.array_equal(a, b)
