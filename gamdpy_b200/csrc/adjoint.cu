@@ -768,9 +768,11 @@ int aset(gdb_adj *h, int code, const char *fmt, ...) {
 #define ACK(call)                                                                                          \
     do {                                                                                                   \
         cudaError_t e_ = (call);                                                                           \
-        if (e_ != cudaSuccess)                                                                             \
+        if (e_ != cudaSuccess) {                                                                           \
+            (void)cudaGetLastError(); /* reported here, not again by the next launch's check */            \
             return aset(h, GDB_ERR_CUDA, "%s failed: %s (%s:%d)", #call, cudaGetErrorString(e_), __FILE__, \
                         __LINE__);                                                                         \
+        }                                                                                                  \
     } while (0)
 
 void adj_free(gdb_adj *h) {
@@ -1002,6 +1004,7 @@ int gdb_adj_setup(gdb_adj *h, const float box[3], const int32_t *ptype, const fl
         if (!(mass[i] > 0.f)) return aset(h, GDB_ERR_ARG, "gdb_adj_setup: masses must be positive");
     }
     ACK(cudaSetDevice(h->dev));
+    h->setup = h->forward_done = false;  // until everything below is in place
     memcpy(h->box, box, sizeof(h->box));
     h->dt = dt;
     h->steps = steps;
@@ -1039,7 +1042,6 @@ int gdb_adj_setup(gdb_adj *h, const float box[3], const int32_t *ptype, const fl
     }
     ACK(cudaStreamSynchronize(h->st));
     h->setup = true;
-    h->forward_done = false;
     return GDB_OK;
 }
 
@@ -1054,6 +1056,7 @@ int gdb_adj_forward(gdb_adj *h, const double *params, const float *r0, const flo
             return aset(h, GDB_ERR_ARG, "gdb_adj_forward: cut must be below half the box");
     }
     ACK(cudaSetDevice(h->dev));
+    h->forward_done = false;  // the last forward's tables and states are overwritten from here on
     build_tables(h, params);
     const int n = h->n;
     int rc = ensure_list(h);

@@ -186,3 +186,48 @@ def test_bad_arguments_raise():
     with pytest.raises(GdbError) as e:
         adjoint.AdjointNVE(small_ka(), workloads.KA_CUT, dt=-1.0, steps=10)
     assert e.value.args[0] == GDB_ERR_ARG or "bad arguments" in str(e.value)
+
+
+@pytest.mark.gpu
+def test_failed_forward_leaves_nothing_to_differentiate():
+    """A forward whose list overflows has overwritten the states of the one before: backward and final_state refuse, and
+    a good forward brings them back.  An argument that is refused before that leaves the last forward in place."""
+    from gamdpy_b200._lib import GDB_ERR_ARG, GDB_ERR_NBLIST, GDB_ERR_STATE, GdbError
+    conf = workloads.ka_configuration(2048, rho=0.3, temperature=0.6, seed=4)
+    eng = adjoint.AdjointNVE(conf, workloads.KA_CUT, dt=0.004, steps=10)
+    th = ka_theta()
+    obs = eng.forward(th)
+    g = eng.backward(np.ones(3))
+    with pytest.raises(GdbError) as e:
+        eng.forward(-th)
+    assert e.value.code == GDB_ERR_ARG
+    assert np.array_equal(eng.backward(np.ones(3)), g)
+    spread = eng.r0
+    eng.r0 = np.ascontiguousarray(spread * np.float32(0.25))  # 64 times the density: columns outgrow their rows
+    with pytest.raises(GdbError) as e:
+        eng.forward(th)
+    assert e.value.code == GDB_ERR_NBLIST
+    for call in (lambda: eng.backward(np.ones(3)), eng.final_state):
+        with pytest.raises(GdbError) as e:
+            call()
+        assert e.value.code == GDB_ERR_STATE
+    eng.r0 = spread
+    assert np.array_equal(eng.forward(th), obs) and np.array_equal(eng.backward(np.ones(3)), g)
+
+
+@pytest.mark.gpu
+def test_failed_setup_leaves_the_handle_unusable():
+    """Checkpoints of every one of 2e9 steps need terabytes: the setup fails, and the forward refuses."""
+    import ctypes
+
+    from gamdpy_b200 import _lib
+    eng = adjoint.AdjointNVE(small_ka(), workloads.KA_CUT, dt=0.005, steps=10)
+    eng.forward(ka_theta())
+    rc = _lib.lib().gdb_adj_setup(eng.h, _lib.ptr(eng.box), _lib.ptr(eng.ptype), _lib.ptr(eng.mass),
+                                  ctypes.c_float(0.005), 2000000000, 1, 0, ctypes.c_float(0.0), ctypes.c_float(1.0),
+                                  ctypes.c_float(1.0), 0)
+    assert rc == _lib.GDB_ERR_CUDA
+    for call in (lambda: eng.forward(ka_theta()), lambda: eng.backward(np.ones(3)), eng.final_state):
+        with pytest.raises(_lib.GdbError) as e:
+            call()
+        assert e.value.code == _lib.GDB_ERR_STATE
