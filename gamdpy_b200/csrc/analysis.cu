@@ -952,65 +952,125 @@ struct SqRuns {
     std::vector<int4> items;
     std::vector<int> entry;
 };
+
+// One bit per cell of a bounding grid, columns of nz cells along a run axis.
+struct SqGrid {
+    int axis[3], kmin[3], klen[3];
+    std::vector<uint64_t> bits;
+    std::vector<unsigned> cell;  // by q-vector
+    void mark(int nq, const int32_t *nvec, const int lo[3], const int len[3], int run) {
+        axis[0] = run == 0 ? 1 : 0;
+        axis[1] = run == 2 ? 1 : 2;
+        axis[2] = run;
+        for (int d = 0; d < 3; d++) {
+            kmin[d] = lo[axis[d]];
+            klen[d] = len[axis[d]];
+        }
+        bits.assign(((size_t)klen[0] * klen[1] * klen[2] + 63) / 64, 0);
+        cell.resize(nq);
+        const unsigned s1 = klen[2], s0 = klen[1] * s1;  // (modulo 2^32; a cell's number is below 2^31)
+        const unsigned off = kmin[0] * s0 + kmin[1] * s1 + kmin[2];
+        const int32_t *v0 = nvec + axis[0], *v1 = nvec + axis[1], *v2 = nvec + axis[2];
+        for (size_t q = 0; q < (size_t)nq; q++) {
+            const unsigned c = (unsigned)v0[3 * q] * s0 + (unsigned)v1[3 * q] * s1 + (unsigned)v2[3 * q] - off;
+            cell[q] = c;
+            bits[c / 64] |= 1ull << (c % 64);
+        }
+    }
+    // at most as many as there are runs: the marked cells without another
+    // among the seven before them
+    size_t runs_at_least() const {
+        size_t count = 0;
+        uint64_t last = 0;
+        for (const uint64_t m : bits) {
+            if (!m) {
+                last = 0;
+                continue;
+            }
+            unsigned __int128 before = ((unsigned __int128)m << 64 | last) << 1;  // marked 1, then 1 to 7 before
+            before |= before << 1;
+            before |= before << 2;
+            before |= before << 3;
+            count += __builtin_popcountll(m & ~(uint64_t)(before >> 64));
+            last = m;
+        }
+        return count;
+    }
+    // the runs in the order of their cells: f(first cell marked, its column,
+    // start of the run)
+    template <class F>
+    void runs(F f) const {
+        const unsigned nz = klen[2];
+        for (unsigned pos = 0, w = 0; (w = pos / 64) < bits.size();) {
+            const uint64_t m = bits[w] >> (pos % 64);
+            if (!m) {
+                pos = 64 * (w + 1);
+                continue;
+            }
+            pos += __builtin_ctzll(m);
+            const unsigned col = pos / nz, z0 = (pos - col * nz) & ~1u;  // a run starts at an even component
+            f(pos, col, (int)z0);
+            pos = col * nz + std::min(nz, z0 + SQ_Z);
+        }
+    }
+};
+
+// False where k_sq takes the set: runs of less than two q-vectors on average
+// (per particle a run issues 30 instructions and a q-vector of k_sq 23), or a
+// set much sparser than its bounding grid (or wide).  The grid is one bit a
+// cell and its runs are counted before any item is made, so that a set that
+// stays with k_sq costs little: a call of 1000 particles with 1000 scattered
+// q-vectors within 24 of the origin took 834 us with all three axes' items
+// made on a grid of integers and takes 559, with 3778 of them 1246 and 615.
 static bool sq_runs_plan(int nq, const int32_t *nvec, const int kmin[3], const int klen[3], SqRuns &best) {
-    // the plan marks the q-vectors on their bounding grid: sets much sparser
-    // than that (or wide) stay with k_sq
     const double cells = (double)klen[0] * klen[1] * klen[2];
-    if (cells > 64.0 * nq + 65536.0) return false;
-    std::vector<int> at;
+    if (cells > 64.0 * nq + 65536.0 || cells > 2147483648.0) return false;
+    SqGrid g, t;
+    size_t nitems = 0;
     for (int run = 2; run >= 0; run--) {
         // (runs along z that are half full are good enough)
-        if (!best.items.empty() && best.items.size() * SQ_Z <= 2 * (size_t)nq) break;
-        SqRuns s;
-        s.axis[0] = run == 0 ? 1 : 0;
-        s.axis[1] = run == 2 ? 1 : 2;
-        s.axis[2] = run;
-        for (int d = 0; d < 3; d++) {
-            s.kmin[d] = kmin[s.axis[d]];
-            s.klen[d] = klen[s.axis[d]];
-        }
-        const int na = s.klen[0], nb = s.klen[1], nz = s.klen[2];
-        at.assign((size_t)na * nb * nz, -1);
-        for (int q = 0; q < nq; q++) {
-            const int32_t *v = nvec + 3 * (size_t)q;
-            at[((size_t)(v[s.axis[0]] - s.kmin[0]) * nb + (v[s.axis[1]] - s.kmin[1])) * nz + (v[run] - s.kmin[2])] = 0;
-        }
-        // a run starts at the even component at or below its first one
-        for (int x = 0; x < na; x++)
-            for (int y = 0; y < nb; y++) {
-                int *col = &at[((size_t)x * nb + y) * nz];
-                for (int z = 0; z < nz;) {
-                    if (col[z] < 0) {
-                        z++;
-                        continue;
-                    }
-                    const int z0 = z & ~1;
-                    for (z = z0; z < std::min(nz, z0 + SQ_Z); z++)
-                        if (col[z] >= 0) col[z] = (int)s.items.size() * SQ_Z + (z - z0);
-                    s.items.push_back(make_int4(x, y, z0, 0));
-                }
-            }
-        if (!best.items.empty() && best.items.size() <= s.items.size()) continue;
-        // the lanes of a warp share a run (broadcast loads): items in the
-        // order of their run's start
-        std::vector<int> order(s.items.size()), place(s.items.size());
-        for (size_t k = 0; k < order.size(); k++) order[k] = (int)k;
-        std::stable_sort(order.begin(), order.end(), [&](int p, int q) { return s.items[p].z < s.items[q].z; });
-        std::vector<int4> sorted(s.items.size());
-        for (size_t k = 0; k < order.size(); k++) {
-            place[order[k]] = (int)k;
-            sorted[k] = s.items[order[k]];
-        }
-        s.items.swap(sorted);
-        s.entry.resize(nq);
-        const int nitems = (int)s.items.size();
-        for (int q = 0; q < nq; q++) {
-            const int32_t *v = nvec + 3 * (size_t)q;
-            const int e =
-                at[((size_t)(v[s.axis[0]] - s.kmin[0]) * nb + (v[s.axis[1]] - s.kmin[1])) * nz + (v[run] - s.kmin[2])];
-            s.entry[q] = (e % SQ_Z) * nitems + place[e / SQ_Z];
-        }
-        best = std::move(s);
+        if (nitems && nitems * SQ_Z <= 2 * (size_t)nq) break;
+        t.mark(nq, nvec, kmin, klen, run);
+        if (2 * t.runs_at_least() > (size_t)nq) continue;
+        size_t count = 0;
+        t.runs([&](unsigned, unsigned, int) { count++; });
+        if (nitems && nitems <= count) continue;
+        nitems = count;
+        std::swap(g, t);
+    }
+    if (!nitems || 2 * nitems > (size_t)nq) return false;
+    // a q-vector's run is the last one that starts at or before its cell
+    std::vector<uint64_t> first(g.bits.size(), 0);
+    std::vector<int> below(g.bits.size() + 1, 0);  // runs that start in earlier words
+    std::vector<int4> items;
+    std::vector<unsigned> start;  // cell of a run's entry 0
+    items.reserve(nitems);
+    start.reserve(nitems);
+    g.runs([&](unsigned pos, unsigned col, int z0) {
+        first[pos / 64] |= 1ull << (pos % 64);
+        below[pos / 64 + 1]++;
+        items.push_back(make_int4((int)(col / (unsigned)g.klen[1]), (int)(col % (unsigned)g.klen[1]), z0, 0));
+        start.push_back(col * (unsigned)g.klen[2] + z0);
+    });
+    for (size_t w = 1; w < below.size(); w++) below[w] += below[w - 1];
+    // the lanes of a warp share a run (broadcast loads): items in the order
+    // of their run's start
+    std::vector<int> place(nitems), at(g.klen[2] + 1, 0);
+    for (const int4 &i : items) at[i.z + 1]++;
+    for (int z = 0; z < g.klen[2]; z++) at[z + 1] += at[z];
+    for (size_t k = 0; k < nitems; k++) place[k] = at[items[k].z]++;
+    best.entry.resize(nq);
+    for (int q = 0; q < nq; q++) {
+        const unsigned c = g.cell[q];
+        const int k = below[c / 64] + __builtin_popcountll(first[c / 64] << (63 - c % 64)) - 1;
+        best.entry[q] = (int)(c - start[k]) * (int)nitems + place[k];
+    }
+    best.items.resize(nitems);
+    for (size_t k = 0; k < nitems; k++) best.items[place[k]] = items[k];
+    for (int d = 0; d < 3; d++) {
+        best.axis[d] = g.axis[d];
+        best.kmin[d] = g.kmin[d];
+        best.klen[d] = g.klen[d];
     }
     // table columns: the run's section starts at an even column and holds
     // whole runs, so that their 16-byte loads are aligned and inside a row
@@ -1078,10 +1138,8 @@ static int sq_device(gdb_sim *h, cudaStream_t st, const float4 *pos, const int *
     const size_t smem = (size_t)SQ_TILE * row * sizeof(float2);
     if (smem > 200 * 1024) return aset(h, GDB_ERR_ARG, "sq: n_vectors span too wide");
     SqRuns plan;
-    bool runs = sq_runs_plan(nq, nvec_host, a.kmin, a.klen, plan);
-    // per particle a run issues 30 instructions and a q-vector of k_sq 23:
-    // runs where they hold at least two q-vectors on average
-    if (runs) runs = 2 * plan.items.size() <= (size_t)nq && sq_runs_smem(plan.klen, SQ_RUN_THREADS) <= 224 * 1024;
+    const bool runs = sq_runs_plan(nq, nvec_host, a.kmin, a.klen, plan) &&
+                      sq_runs_smem(plan.klen, SQ_RUN_THREADS) <= 224 * 1024;
     const size_t nacc = runs ? plan.items.size() * SQ_Z * 2 : (size_t)nq * 2;
     int *dn = nullptr;  // n-vectors, or the runs' items
     float *dff = nullptr;
