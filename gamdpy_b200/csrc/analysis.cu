@@ -346,8 +346,8 @@ __device__ __forceinline__ int rdf_cell(float r, float L, int nc) {
 }
 
 // Cell search for r_max < L/3: particles sorted by cell, x fastest; cells of
-// edge >= r_max in y and z (at least 3 per side) and >= r_max / 2 in x (at
-// least 6).  A unit of work is 32 consecutive slots of one x-row of cells
+// edge >= r_max in y and z (at least 3 per side) and >= r_max / 2 in x (of
+// half the edge where cells are full, see rdf_device).  A unit of work is 32 consecutive slots of one x-row of cells
 // (unit u: row u / K, slots 32 (u % K) on, K = units of the fullest row; units
 // past a row's end are empty), taken a unit per warp: every lane has a
 // particle, whatever a cell holds.  With [xa, xb] the x-cells of the unit's
@@ -885,10 +885,17 @@ static int rdf_device(gdb_sim *h, cudaStream_t st, const float4 *pos, int n, con
         // coordinate can never separate a pair closer than r_max by two cells
         const double edges = box[k] / (r_max * (1.0 + 1e-4));
         if (edges < 3.0) cells = false;
-        nc[k] = (int)floor(k == 0 ? 2.0 * edges : edges);  // cells of half the edge in x
+        nc[k] = (int)floor(edges);
     }
-    const long long ncell = cells ? (long long)nc[0] * nc[1] * nc[2] : 0;
-    if (ncell > (1LL << 28)) cells = false;  // r_max tiny against L: fall back to all pairs
+    // cells of half the edge in x from 12 particles a whole one on: the search
+    // gains from the narrower windows, the counts' scan loses (a call, us,
+    // whole and half: N 300 000 at 4 a cell 839 and 1030, at 12 804 and 816,
+    // at 24 865 and 830, at 128 1537 and 1240; N 30 000 at 0.01 3510 and 7505)
+    const int ncx2 = cells ? (int)floor(2.0 * (box[0] / (r_max * (1.0 + 1e-4)))) : 0;
+    const long long yz = (long long)nc[1] * nc[2];
+    if (cells && ncx2 * yz > (1LL << 28)) cells = false;  // r_max tiny against L: fall back to all pairs
+    if (cells && 6 * ncx2 * yz <= n) nc[0] = ncx2;
+    const long long ncell = cells ? nc[0] * yz : 0;
     if (!cells) {
         const size_t smem = sizeof(RdfStage<RDF_TILE>) + RDF_WARPS * 1024 * sizeof(float) + hist_bytes;
         const int T = (n + RDF_TILE - 1) / RDF_TILE;

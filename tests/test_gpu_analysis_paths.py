@@ -65,6 +65,25 @@ def test_rdf_rows_of_uneven_occupation(oracle, n, bins, nt):
     assert np.array_equal(got, oracle.rdf(r, pt, L, bins, fma=1, r_max=3.1)) and got.sum() > 0
 
 
+@pytest.mark.parametrize("length", [22.0, 40.0])
+@pytest.mark.parametrize("step", [-1, 0])
+def test_rdf_whole_and_half_cells(oracle, length, step):
+    """The last size of whole cells in x and the first of half ones (six a half cell), every coordinate once on a face;
+    a grid just wide enough for plain differences and a wider one."""
+    L = np.full(3, length, np.float32)
+    edges = float(L[0]) / (3.1 * (1.0 + 1e-4))
+    n = 6 * int(2 * edges) * int(edges) ** 2 + step
+    rng = np.random.default_rng(n)
+    r = ((rng.random((n, 3)) - 0.5) * L).astype(np.float32)
+    h = np.float32(0.5) * L[0]
+    faces = np.array([h, -h, np.nextafter(h, np.float32(0)), np.nextafter(-h, np.float32(0))], np.float32)
+    for axis in range(3):
+        r[100 * axis : 100 * (axis + 1), axis] = np.tile(faces, 25)
+    pt = rng.integers(0, 2, n).astype(np.int32)
+    got = _lib.rdf_compute(r, pt, L, 2, 100, r_max=3.1)
+    assert np.array_equal(got, oracle.rdf(r, pt, L, 100, fma=1, r_max=3.1)) and got.sum() > 0
+
+
 @pytest.mark.parametrize("axis", [0, 1, 2])
 def test_rdf_coordinates_on_the_faces(oracle, axis):
     """Particles on the faces of the box and one float away from them, in a grid that takes plain differences."""
