@@ -83,6 +83,11 @@ constexpr int RDF_THREADS = 256;
 constexpr int RDF_WARPS = RDF_THREADS / 32;
 constexpr int RDF_TILE = RDF_THREADS;     // j positions staged per block (all-pairs path)
 constexpr int RDF_SMEM_MAX_BINS = 12288;  // uint32 entries kept in shared memory
+// Dynamic shared memory that a kernel may be launched with: one value for every
+// call, as calls of several threads set it (a thread that sets less than
+// another is about to launch with would fail that launch).
+constexpr int RDF_HIST_MAX = (2 * RDF_SMEM_MAX_BINS + 1) * (int)sizeof(unsigned);  // histograms and bin edges
+constexpr int SQ_SMEM_MAX = 200 * 1024, SQ_RUN_SMEM_MAX = 224 * 1024;
 
 template <bool B>
 struct RdfTag {
@@ -903,7 +908,8 @@ static int rdf_device(gdb_sim *h, cudaStream_t st, const float4 *pos, int n, con
         ACK(cudaGetDevice(&dev));
         ACK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
         auto kern = fma ? k_rdf_allpairs<true> : k_rdf_allpairs<false>;
-        ACK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        ACK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)(smem - hist_bytes) + RDF_HIST_MAX));
         ACK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, RDF_THREADS, smem));
         // slices of the tile-distance range: about two waves of blocks in all
         const int slots = sms * std::max(per_sm, 1);
@@ -929,7 +935,8 @@ static int rdf_device(gdb_sim *h, cudaStream_t st, const float4 *pos, int n, con
         ACK(cudaGetDevice(&dev));
         ACK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
         auto kern = fma ? k_rdf_cells<true> : k_rdf_cells<false>;
-        ACK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        ACK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)(smem - hist_bytes) + RDF_HIST_MAX));
         ACK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, RDF_THREADS, smem));
         const int grid = sms * std::max(per_sm, 1);  // warps stride over the units
         kern<<<grid, RDF_THREADS, smem, st>>>(a, spos, start, count + ncell, nc[0], nc[1], nc[2]);
@@ -1107,7 +1114,7 @@ static cudaError_t launch_sq_runs(cudaStream_t st, SqRunArgs &r, int n) {
     const size_t smem = sq_runs_smem(r.klen, threads);
     int dev = 0, sms = 0, per_sm = 0;
     cudaError_t e;
-    if ((e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) ||
+    if ((e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, SQ_RUN_SMEM_MAX)) ||
         (e = cudaGetDevice(&dev)) || (e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) ||
         (e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, smem)))
         return e;
@@ -1143,10 +1150,10 @@ static int sq_device(gdb_sim *h, cudaStream_t st, const float4 *pos, const int *
     }
     const int row = a.klen[0] + a.klen[1] + a.klen[2];
     const size_t smem = (size_t)SQ_TILE * row * sizeof(float2);
-    if (smem > 200 * 1024) return aset(h, GDB_ERR_ARG, "sq: n_vectors span too wide");
+    if (smem > SQ_SMEM_MAX) return aset(h, GDB_ERR_ARG, "sq: n_vectors span too wide");
     SqRuns plan;
     const bool runs = sq_runs_plan(nq, nvec_host, a.kmin, a.klen, plan) &&
-                      sq_runs_smem(plan.klen, SQ_RUN_THREADS) <= 224 * 1024;
+                      sq_runs_smem(plan.klen, SQ_RUN_THREADS) <= SQ_RUN_SMEM_MAX;
     const size_t nacc = runs ? plan.items.size() * SQ_Z * 2 : (size_t)nq * 2;
     int *dn = nullptr;  // n-vectors, or the runs' items
     float *dff = nullptr;
@@ -1200,7 +1207,7 @@ static int sq_device(gdb_sim *h, cudaStream_t st, const float4 *pos, const int *
             case 3: fn = a.ff ? (const void *)k_sq<3, true> : (const void *)k_sq<3, false>; break;
             default: fn = a.ff ? (const void *)k_sq<4, true> : (const void *)k_sq<4, false>; break;
         }
-        ACK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        ACK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, SQ_SMEM_MAX));
         switch (qpt) {
             case 1: launch_sq<1>(grid, smem, st, a); break;
             case 2: launch_sq<2>(grid, smem, st, a); break;
@@ -1370,7 +1377,8 @@ int gdb_sq_compute_noalloc(int n, const float *r_dev, const float *ff_dev, const
     cudaStream_t st = (cudaStream_t)stream;
     const int span = 2 * n_max + 1;
     const size_t smem = (size_t)SQ_TILE * 3 * span * sizeof(float2);
-    ACK(cudaFuncSetAttribute(k_sqna, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    constexpr int most = SQ_TILE * 3 * (2 * GDB_SQ_NOALLOC_MAX_N + 1) * (int)sizeof(float2);
+    ACK(cudaFuncSetAttribute(k_sqna, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
     k_sqna_clear<<<(2 * nq + 255) / 256, 256, 0, st>>>(s, nq);
     k_sqna_weight_sum<<<64, 256, 0, st>>>(ff_dev, n, s);
     dim3 grid((nq + SQ_THREADS - 1) / SQ_THREADS, (n + SQ_CHUNK - 1) / SQ_CHUNK);

@@ -132,3 +132,36 @@ def test_adjoint_long_columns_keep_their_order(monkeypatch):
         out.append((obs, eng.backward(np.array([0.5, 1.0, 1.5])), *eng.final_state()))
     for a, b in zip(*out):
         assert np.isfinite(a).all() and np.array_equal(a, b)
+
+
+def test_analyses_from_several_threads():
+    """Threads whose calls need different amounts of shared memory of the same kernels: every call succeeds and gives
+    what it gives alone."""
+    import threading
+    rng = np.random.default_rng(8)
+    L = np.array([10.0, 10.0, 10.0], np.float32)
+    r = ((rng.random((200, 3)) - 0.5) * L).astype(np.float32)
+    pt = np.zeros(200, np.int32)
+    scattered = rng.integers(-20, 21, size=(40, 3))
+    pairs = [(lambda: _lib.sq_compute(r, L, _octant(4)), lambda: _lib.sq_compute(r, L, _octant(16))),
+             (lambda: _lib.sq_compute(r, L, scattered % 7), lambda: _lib.sq_compute(r, L, scattered)),
+             (lambda: _lib.rdf_compute(r, pt, L, 1, 20), lambda: _lib.rdf_compute(r, pt, L, 1, 9000)),
+             (lambda: _lib.rdf_compute(r, pt, L, 1, 20, r_max=2.0), lambda: _lib.rdf_compute(r, pt, L, 1, 9000, r_max=2.0))]
+    for pair in pairs:
+        wrong = []
+
+        def work(f, want):
+            for _ in range(1000):
+                try:
+                    got = f()
+                    if np.abs(got.astype(complex) - want).max() > 1e-9:
+                        wrong.append("other numbers")
+                except Exception as e:
+                    wrong.append(e)
+
+        threads = [threading.Thread(target=work, args=(f, f().astype(complex))) for f in pair for _ in range(2)]
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join()
+        assert not wrong, (len(wrong), wrong[:3])
