@@ -165,6 +165,35 @@ def test_truncated_adjoint_matches_detached_autograd(window, ckpt):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("nt", [1, 2, 3, 4])
+def test_gradient_by_number_of_types(nt):
+    """One, two and more types (an instantiation of the sweep each; three and four types share one): a weighted sum of
+    the observables against torch.autograd through the float64 forward."""
+    import torch
+
+    from oracle import adjoint_torch as R
+    conf = workloads.ka_configuration(256, rho=0.9, temperature=0.6, seed=20 + nt)
+    rng = np.random.default_rng(nt)
+    conf.ptype[:] = rng.permutation(np.arange(256) % nt)
+    sig, eps = np.ones((nt, nt)), np.ones((nt, nt))
+    for a in range(nt):
+        for b in range(nt):
+            sig[a, b] = 1.0 - 0.04 * (a + b)
+            eps[a, b] = 1.0 + 0.1 * (a + b)
+    cut = 2.5 * sig
+    th0 = adjoint.theta_from_tables(sig, eps)
+    eng = adjoint.AdjointNVE(conf, cut, dt=0.005, steps=30, checkpoint_every=10, rdf=RDF)
+    obs = eng.forward(th0)
+    w = np.linspace(1.0, 2.0, len(obs))
+    th = torch.tensor(th0, requires_grad=True)
+    ref = R.observables(th, conf["r"], conf["v"], conf.ptype, conf["m"], conf.simbox.lengths, cut, 0.005, 30, rdf=RDF)
+    (ref * torch.tensor(w)).sum().backward()
+    g, g_ref = eng.backward(w), th.grad.numpy()
+    np.testing.assert_allclose(obs[:3], ref.detach().numpy()[:3], rtol=2e-5)
+    assert np.linalg.norm(g - g_ref) <= GRAD_TOL * np.linalg.norm(g_ref), (g, g_ref)
+
+
+@pytest.mark.gpu
 def test_backward_after_another_forward_reruns_the_forward():
     import torch
     conf = small_ka(seed=9)

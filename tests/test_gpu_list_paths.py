@@ -45,6 +45,27 @@ def test_cell_lists_over_launch_shapes(oracle, n, persistent):
         assert rel_rms(sim.download()["f"], res["f"]) < FORCE_TOL
 
 
+@pytest.mark.parametrize("n,kind", [(2050, _lib.NBLIST_NSQ), (3073, _lib.NBLIST_CELLS), (4737, _lib.NBLIST_CELLS),
+                                    (10007, _lib.NBLIST_CELLS), (37889, _lib.NBLIST_CELLS),
+                                    (75777, _lib.NBLIST_CELLS), (151553, _lib.NBLIST_CELLS)])
+def test_lists_with_rounded_products(oracle, n, kind, monkeypatch):
+    """GDB_NBLIST_FMA=0: the distances' products rounded before they are added (gamdpy's CPU build), over the lanes per
+    particle of the cell build and in the N^2 build."""
+    monkeypatch.setenv("GDB_NBLIST_FMA", "0")
+    monkeypatch.setenv("GDB_CLUSTER", "0")
+    conf = workloads.ka_configuration(n, seed=n, jitter=0.2)
+    L = conf.simbox.lengths
+    sim = make_sim(conf["r"], L, conf.ptype, _table(oracle), nblist=kind, skin=SKIN)
+    sim.run(0.0, 0)
+    if n <= 20011:
+        ref = oracle.nblist_nsq(conf["r"], L, CPS, 300, fma=0)[0]
+    else:
+        ref = oracle.nblist_cells(conf["r"], L, 2.5, SKIN, 300, fma=0)[0]
+    c1, f1 = sorted_rows(sim.nblist(300))
+    c2, f2 = sorted_rows(ref)
+    assert np.array_equal(c1, c2) and np.array_equal(f1, f2)
+
+
 @pytest.mark.parametrize("n", [257, 1024, 1025, 3000])
 @pytest.mark.parametrize("persistent", [True, False])
 def test_nsq_lists_over_mask_edges(oracle, n, persistent, monkeypatch):
