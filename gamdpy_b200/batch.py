@@ -119,8 +119,8 @@ class SimulationBatch:
                 f"Steps : {len(self.timing_blocks)} * {self.steps_per_block}  TPS: {tps:.3e}  "
                 f"atom-steps/s: {tps * self.num_particles:.3e}\n")
 
-    def autotune(self, candidates=(0, 64, 128, 192, 256), clg_candidates=(0, 2048, 4096, 8192),
-                 clg_tps=(1, 2, 4), steps=None, verbose=False):
+    def autotune(self, candidates=(0, 64, 128, 192, 256), clg_candidates=(0, 512, 1024, 2048, 4096, 8192),
+                 clg_tps=(0, 1, 2, 4, 8), steps=None, verbose=False):
         """Pick the batch's shape by timing short batched runs, one axis at a
         time (shared-memory clusters' particles per CTA, then the
         global-memory clusters' particles per CTA, then their lanes per
