@@ -118,9 +118,9 @@ class AdjointNVE:
         """Observables (numpy float64) of the trajectory at parameters theta."""
         obs = np.zeros(self.n_obs, np.float64)
         p = self._params(theta)
+        self.forward_count += 1  # a forward that fails replaces the states of the one before, too
         self._check(_lib.lib().gdb_adj_forward(self.h, _lib.ptr(p), _lib.ptr(self.r0), _lib.ptr(self.v0),
                                                _lib.ptr(obs)), "gdb_adj_forward")
-        self.forward_count += 1
         self._last_theta = np.array(theta, np.float64)
         return obs
 

@@ -245,6 +245,28 @@ def test_failed_forward_leaves_nothing_to_differentiate():
 
 
 @pytest.mark.gpu
+def test_autograd_after_a_failed_forward_reruns_its_own():
+    """Observables whose engine then failed another forward: backward repeats the forward at their parameters."""
+    import torch
+
+    from gamdpy_b200._lib import GdbError
+    conf = workloads.ka_configuration(2048, rho=0.3, temperature=0.6, seed=4)
+    eng = adjoint.AdjointNVE(conf, workloads.KA_CUT, dt=0.004, steps=10)
+    th = torch.tensor(ka_theta(), requires_grad=True)
+    eng.observables(th).sum().backward()
+    want = th.grad.clone()
+    th.grad = None
+    obs = eng.observables(th)
+    spread = eng.r0
+    eng.r0 = np.ascontiguousarray(spread * np.float32(0.25))
+    with pytest.raises(GdbError):
+        eng.forward(ka_theta())
+    eng.r0 = spread
+    obs.sum().backward()
+    assert torch.equal(th.grad, want)
+
+
+@pytest.mark.gpu
 def test_failed_setup_leaves_the_handle_unusable():
     """Checkpoints of every one of 2e9 steps need terabytes: the setup fails, and the forward refuses."""
     import ctypes
