@@ -850,7 +850,9 @@ static float float_at_or_above(double x) {
 static int rdf_device(gdb_sim *h, cudaStream_t st, const float4 *pos, int n, const float *box, int nt, int bins,
                       double r_max, uint64_t *out_host) {
     if (bins < 1 || nt < 1) return aset(h, GDB_ERR_ARG, "rdf: bins and ntypes must be positive");
-    if (nt > 0xffff) return aset(h, GDB_ERR_ARG, "rdf: too many particle types");
+    // the kernels index the nt^2 histograms and the bins' edges by int
+    if ((double)nt * nt * bins > 2147483647.0 || bins > 2147483646)
+        return aset(h, GDB_ERR_ARG, "rdf: more than 2^31 - 1 histogram entries");
     float minL = fminf(box[0], fminf(box[1], box[2]));
     // the reference: min_box_dim float32, (min_box_dim / 2) float64
     const double half = (double)minL / 2.0;

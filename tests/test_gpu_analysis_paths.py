@@ -65,6 +65,15 @@ def test_rdf_rows_of_uneven_occupation(oracle, n, bins, nt):
     assert np.array_equal(got, oracle.rdf(r, pt, L, bins, fma=1, r_max=3.1)) and got.sum() > 0
 
 
+@pytest.mark.parametrize("nt,bins", [(65536, 1), (46341, 1), (2, 1 << 30), (1, 2147483647)])
+def test_rdf_refuses_histograms_beyond_int(nt, bins):
+    r = np.zeros((4, 3), np.float32)
+    with pytest.raises(ValueError, match="rdf"):
+        _lib.check(_lib.lib().gdb_rdf_compute(4, _lib.ptr(r), _lib.ptr(np.zeros(4, np.int32)),
+                                              _lib.ptr(np.ones(3, np.float32)), nt, bins, 0.4,
+                                              _lib.ptr(np.zeros(1, np.uint64))), None, "rdf")
+
+
 @pytest.mark.parametrize("length", [22.0, 40.0])
 @pytest.mark.parametrize("step", [-1, 0])
 def test_rdf_whole_and_half_cells(oracle, length, step):
