@@ -59,7 +59,10 @@ namespace {
 constexpr int ADJ_MAXT = 4;     // particle types
 constexpr int ADJ_MAXB = 128;   // RDF bins
 constexpr int ADJ_LANES = 32;   // lanes per particle: a warp
-constexpr int ADJ_WARPS = 28;   // most warps per block: one block per SM, 4144 particles in flight on 148 SMs
+// Most warps per block (72 registers a thread): one block per SM, 4144 particles
+// in flight on 148 SMs.  One more takes a second turn every step (50 steps,
+// observables and gradient: N 4144 2.22 ms, 4145 2.61, 4200 2.99, 8288 3.84).
+constexpr int ADJ_WARPS = 28;
 constexpr size_t ADJ_KEEP_BYTES = (size_t)1 << 30;  // states kept instead of checkpoints up to this (GDB_ADJ_KEEP_BYTES)
 constexpr int ADJ_NTH = 2 * ADJ_MAXT * ADJ_MAXT;  // d/dsigma, d/depsilon per ordered type pair
 constexpr double ADJ_FIX = 4294967296.0;          // fixed-point scale of the RDF kernel sums
@@ -97,7 +100,6 @@ struct AdjArgs {
     int n, nt;
     float Lx, Ly, Lz;
     float dt;
-    const int *type;
     const float *mass;
     int nbins;
     float r_lo, dr, width;  // bin centres r_lo + (b + 1/2) dr
@@ -221,8 +223,12 @@ __device__ __forceinline__ bool moved_far(const AdjArgs &a, float4 p, float4 q) 
 // Gaussian bins around distance r: calls f(b, x, exp(-x^2 / (2 w^2))) for
 // every bin b within the kernel's support, x = r - centre_b.  From one bin to
 // the next the exponent grows by (2 x dr - dr^2) / (2 w^2): two exponentials
-// for the first bin, two products for each further one (relative error 1e-16
-// per bin); bins wider than four widths take one exponential each.
+// for the first bin, two products for each further one.  The products' errors
+// add up along the bins: against exact values at most 5e-14 of a bin's value
+// over 16 bins, 1.6e-13 over 64 and 5e-13 over the 128 that there can be, where
+// an exponential each has 4e-15 (the forward then rounds a term to 2^-32, and
+// both take r from float32 coordinates).  Bins wider than four widths take one
+// exponential each.
 template <typename F>
 __device__ __forceinline__ void rdf_bins(const AdjArgs &a, double r, F f) {
     const double w = a.width, dr = a.dr, iw2 = 0.5 / (w * w);
@@ -795,7 +801,6 @@ AdjArgs adj_args(const gdb_adj *h) {
     a.Ly = h->box[1];
     a.Lz = h->box[2];
     a.dt = h->dt;
-    a.type = h->d_type;
     a.mass = h->d_mass;
     a.nbins = h->nbins;
     a.r_lo = h->r_lo;

@@ -7,21 +7,29 @@
 // float64, d = sqrt(dist_sq) in float32.  Counts are exact integers (uint64).
 // dist_sq is symmetric bit for bit (the minimum image of -dr is -dr's), so
 // each unordered pair is evaluated once and counted in both orders.
-//   * r_max >= min(L)/3: all pairs, j tiles staged in shared memory.
-//   * smaller r_max: particles sorted into cells of edge >= r_max (counting
-//     sort), home cell and half shell of 13 neighbours.  Same pair set, so
-//     the same counts.
-// Pairs in range are queued per warp and binned 32 at a time.  Per-block
-// histograms live in shared memory (uint32) and are flushed with 64-bit
-// atomics.
+//   * r_max >= min(L)/3 (or more than 2^28 cells): all pairs, j tiles staged
+//     in shared memory.
+//   * smaller r_max: particles sorted into cells (counting sort) of edge >=
+//     r_max in y and z and that or half of it in x; a warp takes 32 slots of
+//     an x-row of cells against its own row and four neighbouring rows.  Same
+//     pair set, so the same counts.
+// A pair in range is binned from an approximate root and one comparison with
+// the bins' edges in dist_sq, which a kernel finds first (k_rdf_edges).
+// Per-block histograms live in shared memory (uint32, each unordered pair
+// once) and are flushed with 64-bit atomics in both orders.
 //
 // S(q) (calculators/calculator_structure_factor.py:131-156, :185-203):
 // rho_q = N_f^-1/2 sum_i f_i exp(i q.r_i) with q = 2 pi n / L.  Because q is
 // on the reciprocal lattice, exp(i q.r) = e_x(nx) e_y(ny) e_z(nz) with
 // e_d(k) = exp(2 pi i k r_d / L_d); each block tabulates e_d(k) for a tile of
-// particles in shared memory (sincospi, float32) and every thread accumulates
-// its q-vectors with complex multiplies, float32 within a tile and float64
-// across tiles.
+// particles in shared memory (sincospi, float32), float32 sums within a tile
+// and float64 across tiles.
+//   * sets that pack into runs along an axis (two q-vectors a run or more): a
+//     thread takes a run of eight and shares the product of the two other
+//     factors among them (k_sq_runs).
+//   * other sets: a thread takes up to four q-vectors, two complex products
+//     each a particle (k_sq).
+// The two differ by float32's rounding (1e-5 of rho_q / N^(1/2)).
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stdio.h>
@@ -644,7 +652,10 @@ __global__ void __launch_bounds__(SQ_THREADS) k_sq(SqArgs a) {
 // the shared memory's rate; 60 % of the issue slots).  Measured on B200 with 1 000 188 particles and 3778 q-vectors in
 // an octant: a call 4.04 ms with k_sq, 1.51 here, 1.34 of it this kernel; with
 // one table and two barriers a tile 1.38, with two items a thread (320
-// threads) 1.57 to 1.85, with two blocks an SM at 48 registers 1.59.
+// threads) 1.57 to 1.85, with two blocks an SM at 48 registers 1.59.  Items
+// beyond SQ_RUN_THREADS take another block that tabulates the particles again:
+// a call of 10^6 particles with 640 items takes 2.35 ms, with 641 2.95, with
+// 1280 3.78.
 constexpr int SQ_Z = 8;
 struct SqRunArgs {
     const float4 *pos;
@@ -1031,9 +1042,12 @@ struct SqGrid {
     }
 };
 
-// False where k_sq takes the set: runs of less than two q-vectors on average
-// (per particle a run issues 30 instructions and a q-vector of k_sq 23), or a
-// set much sparser than its bounding grid (or wide).  The grid is one bit a
+// False where k_sq takes the set: runs of less than two q-vectors on average,
+// so that scattered sets keep k_sq's roundings (those of
+// gdb_sq_compute_noalloc), not because runs are slower there: measured, calls
+// with k_sq and with runs at 1.6 q-vectors a run, N 20 000 and 250 of them 798
+// and 233 us, N 1 000 000 and 600 of them 2425 and 1955 us.  Or a set much
+// sparser than its bounding grid (or wide).  The grid is one bit a
 // cell and its runs are counted before any item is made, so that a set that
 // stays with k_sq costs little: a call of 1000 particles with 1000 scattered
 // q-vectors within 24 of the origin took 834 us with all three axes' items

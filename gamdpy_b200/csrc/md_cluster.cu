@@ -169,8 +169,9 @@ __global__ void __launch_bounds__(CL_THREADS, 1) k_cluster_run(const ClusterJob 
         // build (nblist_linked_lists.py:36-39, :127), orders each cell by
         // index, copies the positions into cell order and builds the lists of
         // its own particles over the 5x5x5 stencil (a warp per particle,
-        // candidates in stencil-row order as the global builds).  Grids with
-        // more than CL_MAX_CELLS cells build N^2.
+        // candidates in stencil-row order; the global builds give the same
+        // sets in another order).  Grids with more than CL_MAX_CELLS cells
+        // build N^2.
         if (rebuild) {
             int lmax = 0;
             if (use_cells) {

@@ -270,12 +270,6 @@ __device__ __forceinline__ bool step_barrier_all(DevCtrl *c, unsigned seq, bool 
 // ---------------------------------------------------------------------------
 // neighbour-list phases
 // ---------------------------------------------------------------------------
-template <bool B>
-struct BoolTag {
-    static constexpr bool value = B;
-};
-
-
 // Hits of a warp's particle i, set bits of the lanes' masks, appended to its
 // list: the lanes' hits follow one another in lane order, bit q of lane L is
 // index(L, q).  Returns the number of hits (all lanes).
@@ -687,8 +681,10 @@ struct NbAppend {
 };
 
 // Build with LN lanes (a power of two) per particle: lane r of a particle
-// takes the stencil rows r, r + LN, ...; the lanes' hits of a round of LN rows
-// follow one another in row order.  LN grows until the lanes fill the
+// takes the stencil rows r, r + LN, ....  Of a round of LN rows, the hits among
+// the first 32 slots of every row come first, lane by lane, then those among
+// the next 32, then those beyond the periodic wrap: a fixed order, but another
+// one for another LN.  LN grows until the lanes fill the
 // threads, up to a warp per particle.  rings: NB_RING_BYTES per warp.
 //
 // What bounds it is instruction issue, with the loads of the candidates behind
