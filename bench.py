@@ -754,7 +754,7 @@ def run_lj_large(args):
 
 def measure_adjoint(local, steps, warmup, seed=77, growth=True):
     """Adjoint workload: KA N=4096, rho 1.2, T 0.6, an NVE trajectory of
-    `steps` steps with checkpoints every 50; loss = squared deviations of
+    `steps` steps; loss = squared deviations of
     <U>/N and P plus the L2 distance of the soft A-A g(r) from targets made at
     eps_AB = 1.45, sigma_AB = 0.82; gradients with respect to the 6 pair
     parameters (wall times of whole gradients through AdjointNVE)."""
@@ -801,7 +801,7 @@ def measure_adjoint(local, steps, warmup, seed=77, growth=True):
     eng.set_window(100)
     loss_w, g_w = gradient()
     eng.set_window(0)
-    out = {"workload": f"KA-LJ NVE N={n} rho=1.2 T=0.6, {steps} steps, checkpoints every 50, "
+    out = {"workload": f"KA-LJ NVE N={n} rho=1.2 T=0.6, {steps} steps, "
                        "loss = (<U>/N, P, soft g_AA(r)) vs targets at eps_AB=1.45 sigma_AB=0.82",
            "n": n, "steps": steps, "rdf": rdf, "gradients_per_s": 1.0 / t_grad, "forward_ms": t_fwd * 1e3,
            "gradient_ms": t_grad * 1e3, "backward_over_forward": (t_grad - t_fwd) / t_fwd, "loss": loss,

@@ -7,8 +7,11 @@ integrators/NVE.py:78-97 with LJ_12_6_sigma_epsilon and
 apply_shifted_force_cutoff) on the GPU and returns time-averaged
 observables; ``TrajectoryObservables`` is the ``torch.autograd.Function``
 whose backward is the library's hand-written discrete adjoint (reverse
-leapfrog sweep with Hessian-vector products of the pair forces, recomputed
-from checkpoints kept every ``checkpoint_every`` steps).
+leapfrog sweep with Hessian-vector products of the pair forces).  An engine
+holds every state of its trajectory (32 bytes a particle and step) while they
+fit 1 GiB (``GDB_ADJ_KEEP_BYTES``), and beyond that checkpoints every
+``checkpoint_every`` steps, from which each segment is recomputed; the numbers
+are the same.
 
 Parameters are the unordered type pairs' (epsilon, sigma), ``theta =
 [eps_00, eps_01, ..., eps_(nt-1)(nt-1), sig_00, sig_01, ...]`` (upper
@@ -163,7 +166,7 @@ def _make_function():
         """obs = TrajectoryObservables.apply(theta, engine); backward runs the
         library's adjoint sweep.  If the engine ran another forward in
         between, the forward at this theta is repeated first (the adjoint
-        needs its checkpoints)."""
+        needs its states)."""
 
         @staticmethod
         def forward(ctx, theta, engine):

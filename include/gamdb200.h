@@ -314,6 +314,10 @@ int gdb_rdf_compute(int n, const float *r, const int32_t *ptype, const float box
                     double r_max, uint64_t *out);
 int gdb_sq_compute(int n, const float *r, const float *ff, const float box[3], int nq, const int32_t *n_vectors,
                    double *rho_re, double *rho_im);
+/* (S(q): sets of q-vectors that pack into runs along an axis and other sets
+ * take different kernels with float32 products within tiles of particles, so
+ * the same q-vector in sets of the two kinds, or in gdb_sq_compute_noalloc,
+ * can differ by float32's rounding, about 1e-5 of N^(1/2) rho_q's scale.) */
 
 /* Trajectory dynamics (tools/calc_dynamics.py:6-75) of ConfigurationSaver
  * frames: frames num_blocks x conf_per_block x 2 x n x 3 float32 (positions,
@@ -374,7 +378,10 @@ int gdb_batch_get_last_error(gdb_batch *b, char *buf, int n);
  * threads) race and must be serialized by the caller.  The first call on a
  * device looks up the array's address and should come before any stream
  * capture; the address is kept for the life of the process, so the device's
- * primary context must not be reset (cudaDeviceReset) between calls. */
+ * primary context must not be reset (cudaDeviceReset) between calls.
+ * It has one kernel, a q-vector a thread, for every set: dense sets take two
+ * to three times gdb_sq_compute's time, and differ from it by float32's
+ * rounding (scattered sets agree to the float64 sums). */
 int gdb_sq_compute_noalloc(int n, const float *r_dev, const float *ff_dev, const float box[3], int nq,
                            const int32_t *n_vectors_dev, int n_max, double *rho_re_dev, double *rho_im_dev,
                            void *stream);
@@ -396,8 +403,13 @@ int gdb_selftest_barrier_timeout(int device, long long cycles, unsigned *status)
  * obs[3 + b] = <g_AA(r_b)>, a Gaussian-kernel radial distribution of type-0
  * pairs on every rdf_every-th step, bin centres r_lo + (b + 1/2)(r_hi - r_lo)/bins.
  * The backward is the discrete adjoint of that forward: a reverse sweep with
- * Hessian-vector products of the pair forces, recomputing each segment from
- * checkpoints kept every checkpoint_every steps. */
+ * Hessian-vector products of the pair forces.  A handle keeps every state of
+ * the trajectory (32 bytes a particle and step) while they fit 1 GiB
+ * (GDB_ADJ_KEEP_BYTES in the environment of gdb_adj_setup) and their memory
+ * can be had; checkpoint_every is then not used.  Otherwise it keeps
+ * checkpoints every checkpoint_every steps and recomputes each segment's
+ * states from them.  Both give the same bits.  The memory is held until the
+ * next gdb_adj_setup or gdb_adj_destroy. */
 typedef struct gdb_adj gdb_adj;
 int gdb_adj_create(int n, int ntypes, int device, gdb_adj **out);
 int gdb_adj_destroy(gdb_adj *h);
