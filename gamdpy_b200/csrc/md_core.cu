@@ -408,8 +408,12 @@ static int choose_tp(const gdb_sim *h) {
     // as many lanes as one block of RUN_THREADS threads per SM gives every
     // particle, at most 16 (measured on B200, KA, us per step: N 4096 12.0 at
     // 16 lanes and 13.8 at 32; N 10 007 15.7 at 8 lanes, 17.3 at 4, and 27.6
-    // at 16, which take two rounds; N 65 536 35.9 at 2, 44.0 at 1, 52.3 at 4)
+    // at 16, which take two rounds; N 65 536 35.9 at 2, 44.0 at 1, 52.3 at 4),
+    // and 32 up to 12 particles per SM (N 1600, 16 and 32 lanes: LJ NVE 8.37
+    // and 7.73, KA NVT 9.00 and 8.72; N 2048: LJ 8.58 and 8.37, KA 9.00 and
+    // 9.36, NPT_Atomic 14.9 and 15.5)
     const long long even = (h->n + h->num_sms - 1) / h->num_sms;
+    if (even <= 12) return 32;
     int tp = 1;
     while (tp < 16 && even * tp * 2 <= RUN_THREADS) tp *= 2;
     return tp;
@@ -665,7 +669,9 @@ static int enqueue_step(gdb_sim *h, int mode) {
 // 15.9 and 25.9 (some blocks had two rounds, others one, and the last of 320
 // to 444 blocks kept the books of all).  Above RUN_THREADS per SM the rounds
 // balance better than even shares taken in turn (N 1 048 576: the force phase
-// 242 us against 320).
+// 242 us against 320).  Particles whose 32 lanes do not fill GDB_BLOCK threads
+// per SM take fewer blocks instead, full ones: the barrier is shorter (LJ NVE
+// N 500, 63 blocks of 8 particles 7.20, 125 of 4 with 16 lanes 7.71).
 struct RunShape {
     int grid, block, per_round;
 };
@@ -675,7 +681,7 @@ static int run_shape(gdb_sim *h, const void *fn, const SimArgs &a, RunShape *s, 
     const int tp = h->tp;
     const int even = (h->n + h->num_sms - 1) / h->num_sms;
     const bool spread = h->grid_cap == 0 && (long long)even * tp <= RUN_THREADS;
-    s->per_round = spread ? even : GDB_BLOCK / tp;
+    s->per_round = spread && even * 32 > GDB_BLOCK ? even : GDB_BLOCK / tp;
     // (the list build's scan wants GDB_BLOCK threads, and its walk uses them)
     s->block = spread ? std::max(GDB_BLOCK, (even * tp + 31) / 32 * 32) : GDB_BLOCK;
     *dsmem = a.nsq_smem ? (size_t)h->n * sizeof(float4)

@@ -100,10 +100,11 @@ def test_exclusions_on_every_build(oracle, n, kind):
     assert np.array_equal(c1, c2) and np.array_equal(f1, f2)
 
 
-@pytest.mark.parametrize("n", [2048, 10007, 37889])
+@pytest.mark.parametrize("n", [300, 1184, 1185, 1776, 1777, 2048, 10007, 37889])
 def test_first_run_through_graphs(oracle, n, monkeypatch):
     """Without the persistent kernel, the first run of a handle captures its steps into a graph, where nothing can be
-    allocated; sizes whose standalone step has more lanes than the persistent kernel's.  Against that kernel after 32
+    allocated; sizes whose standalone step has more lanes than the persistent kernel's, and the lines of that kernel's
+    lanes and blocks at small sizes.  Against that kernel after 32
     steps: coordinates to 1e-4 (an ulp of a coordinate here is 1e-6 and either path rounds them 32 times)."""
     conf = workloads.ka_configuration(n, seed=n)
     L = np.asarray(conf.simbox.lengths, np.float32)
