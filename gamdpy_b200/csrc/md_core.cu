@@ -1975,8 +1975,9 @@ static gdb_batch::Group *batch_group(gdb_batch *b, int kind, int C, int tp) {
     return g;
 }
 
-static cudaError_t launch_run_clusters(const void *fn, const ClusterRunJob *d_jobs, int count, int C, int nsteps,
-                                       int do_eval, cudaStream_t st) {
+// Configuration of a launch of `count` clusters of C CTAs (attr: its storage).
+static cudaError_t run_clusters_config(const void *fn, int count, int C, cudaStream_t st, cudaLaunchAttribute *attr,
+                                       cudaLaunchConfig_t *cfg) {
     constexpr int dsmem = CLG_BLOCK / 32 * NB_RING_BYTES;  // the cell build's rings
     cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, dsmem);
     if (e != cudaSuccess) return e;
@@ -1984,18 +1985,41 @@ static cudaError_t launch_run_clusters(const void *fn, const ClusterRunJob *d_jo
         e = cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
         if (e != cudaSuccess) return e;
     }
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(count * C);
-    cfg.blockDim = dim3(CLG_BLOCK);
-    cfg.dynamicSmemBytes = dsmem;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = C;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    *cfg = {};
+    cfg->gridDim = dim3(count * C);
+    cfg->blockDim = dim3(CLG_BLOCK);
+    cfg->dynamicSmemBytes = dsmem;
+    cfg->stream = st;
+    attr->id = cudaLaunchAttributeClusterDimension;
+    attr->val.clusterDim.x = C;
+    attr->val.clusterDim.y = 1;
+    attr->val.clusterDim.z = 1;
+    cfg->attrs = attr;
+    cfg->numAttrs = 1;
+    return cudaSuccess;
+}
+
+// Clusters of C CTAs that the GPU holds at once, 0 when none fits.  A cluster
+// stays within a group of SMs that share a part of the chip, so they are fewer
+// than SMs / C: on a B200 15 of 7 to 9 CTAs, 11 of ten and 7 of 11 to 16.
+static int clusters_at_once(const void *fn, int C) {
+    cudaLaunchAttribute attr;
+    cudaLaunchConfig_t cfg;
+    int k = 0;
+    if (run_clusters_config(fn, 1, C, nullptr, &attr, &cfg) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&k, fn, &cfg) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return 0;
+    }
+    return k;
+}
+
+static cudaError_t launch_run_clusters(const void *fn, const ClusterRunJob *d_jobs, int count, int C, int nsteps,
+                                       int do_eval, cudaStream_t st) {
+    cudaLaunchAttribute attr;
+    cudaLaunchConfig_t cfg;
+    cudaError_t e = run_clusters_config(fn, count, C, st, &attr, &cfg);
+    if (e != cudaSuccess) return e;
     void *args[] = {(void *)&d_jobs, (void *)&nsteps, (void *)&do_eval};
     return cudaLaunchKernelExC(&cfg, fn, args);
 }
@@ -2087,19 +2111,31 @@ int gdb_batch_create_ex(gdb_sim *const *sims, int count, int particles_per_cta, 
     // particles per CTA of the global-memory clusters: given, or the smallest
     // (from 256, in steps of 1.25x) whose CTAs (one per SM, 1 to 16 a system)
     // fit the SMs left for them by the shared-memory clusters' share of the
-    // particles, so that the launch is one wave
+    // particles, and of whose clusters the GPU holds as many at once as there
+    // are of each size and above, so that the launch is one wave (by the SMs
+    // alone 12 systems of 30 000 particles took clusters of 12 and two waves:
+    // 14.2 ms for 40 steps, 9.3 with clusters of 9; eight of 5000 2.9 ms with
+    // clusters of 16, 1.5 with 10)
     if (clg_particles_per_cta > 0) {
         b->clg_ppc = std::max(256, clg_particles_per_cta);
     } else if (p_glob > 0) {
         const int sms = std::max(1, sims[0]->num_sms);
         const int budget = std::max(1, (int)((double)sms * (double)p_glob / (double)(p_glob + p_smem)));
+        const void *fn = run_clusters_kernel(b->ntypes, 1, b->integ);
+        int at_once[17] = {0};
+        for (int c = 1; c <= 16; c++) at_once[c] = clusters_at_once(fn, c);
         int ppc = 256;
         for (int it = 0; it < 60; it++) {
             long long ctas = 0;
-            for (int k : order)
-                if (!in_smem[k] && sims[k]->n <= CLG_MAX_N)
-                    ctas += std::min(16, (sims[k]->n + ppc - 1) / ppc);
-            if (ctas <= budget || ppc >= CLG_MAX_N) break;
+            int clusters = 0;
+            bool fits = true;
+            for (int k : order)  // largest first: `clusters` counts those of c CTAs and more
+                if (!in_smem[k] && sims[k]->n <= CLG_MAX_N) {
+                    const int c = std::min(16, (sims[k]->n + ppc - 1) / ppc);
+                    ctas += c;
+                    fits = fits && ++clusters <= at_once[c];
+                }
+            if ((fits && ctas <= budget) || ppc >= CLG_MAX_N) break;
             ppc = (int)(ppc * 1.25);
         }
         b->clg_ppc = ppc;

@@ -352,7 +352,7 @@ int gdb_batch_create(gdb_sim *const *sims, int count, int particles_per_cta, gdb
  * (which run the persistent phases on thread-block clusters with state in
  * global memory, one 1024-thread CTA per SM): about clg_particles_per_cta
  * particles per CTA (1 to 16 CTAs a system; 0 = the smallest count from 256
- * up whose CTAs fit the SMs left by the smaller systems' share of the
+ * up whose clusters fit at once into the SMs left by the smaller systems' share of the
  * particles) and clg_tp lanes per particle (1, 2, 4 or 8; 0 = as many as the
  * CTA's threads give every particle).  Tuned by
  * SimulationBatch.autotune. */

@@ -189,6 +189,23 @@ def test_uneven_replica_sweep_matches_individual_runs():
         assert y._sim.status() == 0
 
 
+@pytest.mark.parametrize("count, n", [(1, 5000), (7, 4500), (8, 4500), (12, 9000)])
+def test_equal_large_systems_match_individual_runs(count, n):
+    # as many as the GPU holds clusters of 16 CTAs at once, and more
+    alone, batched = ([ka_sim(n, rho=1.2, temp=0.6, seed=k) for k in range(count)] for _ in range(2))
+    for s in alone:
+        s.configuration.copy_to_device()
+        s._sim.run(0.0, 32)
+    batch = gp.SimulationBatch(batched)
+    for s in batched:
+        s.configuration.copy_to_device()
+    batch.integrate_self(0.0, 32)
+    assert batch.paths() == [3] * count
+    for x, y in zip(alone, batched):
+        assert np.max(np.abs(state(x)["r"] - state(y)["r"])) < 1e-3
+        assert y._sim.status() == 0
+
+
 def test_cluster_lists_survive_other_work_between_blocks():
     # lists live in shared memory during a launch only; the next timeblock
     # takes them from global memory even when other systems ran in between
