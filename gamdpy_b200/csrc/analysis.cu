@@ -132,9 +132,10 @@ __device__ __forceinline__ int rdf_bin(const RdfArgs &a, float d) {
 // exactly those with edge[k] <= d2 < edge[k + 1], where edge[k] is the
 // smallest float32 that is out of range or has a bin >= k.  Non-negative
 // floats are ordered as their bit patterns: 31 halvings find it.  The counting
-// loop then needs neither the exact root nor float64.
-__global__ void k_rdf_edges(RdfArgs a, float *edge) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+// loop then needs neither the exact root nor float64.  (Histograms in global
+// memory need edge[bins] only: `first`.)
+__global__ void k_rdf_edges(RdfArgs a, float *edge, int first) {
+    const int k = first + blockIdx.x * blockDim.x + threadIdx.x;
     if (k > a.bins) return;
     unsigned lo = 0, hi = 0x7f800000u;  // +inf is out of range
     while (lo < hi) {
@@ -150,11 +151,14 @@ __global__ void k_rdf_edges(RdfArgs a, float *edge) {
     edge[k] = __uint_as_float(lo);
 }
 
-// One pair in range (d2 < edge[bins]): a guess of its bin from the
-// approximate root, corrected against the edges, and one count of the
-// unordered pair in (t_i, t_j); rdf_flush gives every pair both orders.  For
-// the histograms that fit shared memory (SH: at most RDF_SMEM_MAX_BINS bins)
-// the guess d / width (1 - 2e-6) is below d / width by more than its rounding
+// One pair in range (d2 < edge[bins]).  In histograms that fit shared memory
+// (SH: at most RDF_SMEM_MAX_BINS bins) one count of the unordered pair in
+// (t_i, t_j), rdf_flush gives every pair both orders; in histograms in global
+// memory both orders at once, one addition where they are the same entry (what
+// bounds those is the additions: N 100 000, 40 000 bins, all pairs, 24 ms, 59 with two additions for every pair and the
+// bins searched among the edges).
+// SH: a guess of the bin from the approximate root, corrected against the
+// edges.  The guess d / width (1 - 2e-6) is below d / width by more than its rounding
 // errors (5e-7 of it) and by less than 0.04, so its floor is the bin or the
 // one before: one edge decides.  The float is truncated to the bin by
 // subtracting a half, adding 1.5 2^23 (whose ulp is 1) and reading the
@@ -162,17 +166,19 @@ __global__ void k_rdf_edges(RdfArgs a, float *edge) {
 template <bool SH>
 __device__ __forceinline__ void rdf_count(const RdfArgs &a, const float *edge, float d2, int row, int col,
                                           unsigned *hist) {
-    float root;
-    asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(root) : "f"(d2));
     if (SH) {
+        float root;
+        asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(root) : "f"(d2));
         const int b = __float_as_int(__fadd_rn(__fmaf_rn(root, a.guess, -0.5f), 12582912.0f)) - 0x4b400000;
         atomicAdd(&hist[row + b + (d2 >= edge[b + 1] ? 1 : 0)], 1u);
     } else {
-        int b = min((int)(root * a.guess), a.bins - 1);
-        while (d2 < edge[b]) b--;
-        while (d2 >= edge[b + 1]) b++;
-        atomicAdd(&a.out[row + b], 1ull);
-        atomicAdd(&a.out[col + b], 1ull);
+        const int b = rdf_bin(a, __fsqrt_rn(d2));
+        if (row == col) {
+            atomicAdd(&a.out[row + b], 2ull);
+        } else {
+            atomicAdd(&a.out[row + b], 1ull);
+            atomicAdd(&a.out[col + b], 1ull);
+        }
     }
 }
 
@@ -224,11 +230,13 @@ struct RdfStage {
 // positions [q0, q0 + 32).  First pass: every candidate's dist_sq goes to
 // the warp's d2s[q][lane] and in-range candidates set bit q of the lane's
 // mask; bits q <= lim are dropped (j at or before i in the same row or tile).
-// Second pass: every lane counts its own hits, one per round.
-template <bool FMA, bool MIC, int N>
+// Second pass: every lane counts its own hits, one per round.  SHARED: the
+// histograms are in shared memory (a kernel each way: with both in one, the
+// other's registers cost a fifth of the time, 1667 us against 1394 below).
+template <bool FMA, bool MIC, bool SHARED, int N>
 __device__ __forceinline__ void rdf_warp_tile(const RdfArgs &a, f32x2 mx, f32x2 my, f32x2 mz, int ti, bool act,
                                               const RdfStage<N> &st, int q0, int lim, float *d2s, int lane,
-                                              const float *edge, float last, unsigned *hist, bool sh) {
+                                              const float *edge, float last, unsigned *hist) {
     unsigned mask = 0;
 #pragma unroll
     for (int q = 0; q < 32; q += 4) {
@@ -254,8 +262,8 @@ __device__ __forceinline__ void rdf_warp_tile(const RdfArgs &a, f32x2 mx, f32x2 
         mask &= ~0u << (lim + 1);
     if (!act) mask = 0;
     // each lane reads back its own column of d2s
-    auto rounds = [&](auto sh_tag, auto one_tag) {
-        constexpr bool SH = decltype(sh_tag)::value, ONE = decltype(one_tag)::value;
+    auto rounds = [&](auto one_tag) {
+        constexpr bool ONE = decltype(one_tag)::value;  // one histogram
         while (mask) {
             const int q = __ffs(mask) - 1;
             mask &= mask - 1u;
@@ -266,23 +274,21 @@ __device__ __forceinline__ void rdf_warp_tile(const RdfArgs &a, f32x2 mx, f32x2 
                 row = (ti * a.nt + tj) * a.bins;
                 col = (tj * a.nt + ti) * a.bins;
             }
-            rdf_count<SH>(a, edge, d2, row, col, hist);
+            rdf_count<SHARED>(a, edge, d2, row, col, hist);
         }
     };
-    if (!sh)
-        rounds(RdfTag<false>{}, RdfTag<false>{});
-    else if (a.nt == 1)
-        rounds(RdfTag<true>{}, RdfTag<true>{});
+    if (a.nt == 1)
+        rounds(RdfTag<true>{});
     else
-        rounds(RdfTag<true>{}, RdfTag<false>{});
+        rounds(RdfTag<false>{});
     __syncwarp();
 }
 
 // Shared memory of a counting block: the warps' d2s, then (when the
 // histograms fit) the bin edges and the histograms.
 __device__ __forceinline__ const float *rdf_begin(const RdfArgs &a, unsigned char *tail, unsigned *&hist, int total,
-                                                  bool sh) {
-    if (!sh) {
+                                                  bool shared) {
+    if (!shared) {
         hist = nullptr;
         return a.edge;
     }
@@ -310,15 +316,14 @@ __device__ __forceinline__ void rdf_flush(const RdfArgs &a, unsigned *hist, int 
 // tile pair at distance T/2 belongs to the lower tile), so every i-tile has
 // the same work; blockIdx.y takes slice y of that k range (small systems still
 // fill the GPU).
-template <bool FMA>
+template <bool FMA, bool SHARED>
 __global__ void __launch_bounds__(RDF_THREADS) k_rdf_allpairs(RdfArgs a, const float4 *pos) {
     extern __shared__ __align__(16) unsigned char smraw[];
     RdfStage<RDF_TILE> &tile = *(RdfStage<RDF_TILE> *)smraw;
     float *d2s = (float *)(smraw + sizeof(RdfStage<RDF_TILE>));  // [RDF_WARPS][32][32]
     unsigned *hist;
     const int total = a.nt * a.nt * a.bins;
-    const bool sh = total <= RDF_SMEM_MAX_BINS;
-    const float *edge = rdf_begin(a, (unsigned char *)(d2s + RDF_WARPS * 1024), hist, total, sh);
+    const float *edge = rdf_begin(a, (unsigned char *)(d2s + RDF_WARPS * 1024), hist, total, SHARED);
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     float *wd2 = d2s + w * 1024;
     const float last = edge[a.bins];  // in range: d2 < last (k_rdf_edges)
@@ -341,10 +346,10 @@ __global__ void __launch_bounds__(RDF_THREADS) k_rdf_allpairs(RdfArgs a, const f
         tile.put(threadIdx.x, valid ? pos[j0 + threadIdx.x] : pi, valid);
         __syncthreads();
         for (int q0 = 0; q0 < jn; q0 += 32)
-            rdf_warp_tile<FMA, true>(a, mx, my, mz, ti, act, tile, q0, k == 0 ? i - (j0 + q0) : -1, wd2, lane, edge,
-                                     last, hist, sh);
+            rdf_warp_tile<FMA, true, SHARED>(a, mx, my, mz, ti, act, tile, q0, k == 0 ? i - (j0 + q0) : -1, wd2, lane, edge,
+                                     last, hist);
     }
-    if (sh) rdf_flush(a, hist, total);
+    if (SHARED) rdf_flush(a, hist, total);
 }
 
 // Cell coordinate of the cell search (the same roundings wherever it is used).
@@ -379,7 +384,7 @@ __device__ __forceinline__ int rdf_cell(float r, float L, int nc) {
 // memory that the two passes go through (59 % of its rate).  Measured on B200, LJ, 1 000 188
 // particles, r_max 5, 1000 bins: a call 3.80 ms with a warp per cell and hits
 // compacted into a ring for a float64 bin, 1.41 ms here.
-template <bool FMA>
+template <bool FMA, bool SHARED>
 __global__ void __launch_bounds__(RDF_THREADS) k_rdf_cells(RdfArgs a, const float4 *spos, const int *start,
                                                            const int *outside, int ncx, int ncy, int ncz) {
     extern __shared__ __align__(16) unsigned char smraw[];
@@ -388,8 +393,7 @@ __global__ void __launch_bounds__(RDF_THREADS) k_rdf_cells(RdfArgs a, const floa
     float *d2s = (float *)(smraw + RDF_WARPS * sizeof(RdfStage<32>));
     unsigned *hist;
     const int total = a.nt * a.nt * a.bins;
-    const bool sh = total <= RDF_SMEM_MAX_BINS;
-    const float *edge = rdf_begin(a, (unsigned char *)(d2s + RDF_WARPS * 1024), hist, total, sh);
+    const float *edge = rdf_begin(a, (unsigned char *)(d2s + RDF_WARPS * 1024), hist, total, SHARED);
     float *wd2 = d2s + w * 1024;
     const float last = edge[a.bins];  // in range: d2 < last (k_rdf_edges)
     const bool inside = *outside == 0;
@@ -442,13 +446,13 @@ __global__ void __launch_bounds__(RDF_THREADS) k_rdf_cells(RdfArgs a, const floa
                 __syncwarp();
                 const int lim = k == 0 ? i - j0 : -1;
                 if (plain)
-                    rdf_warp_tile<FMA, false>(a, mx, my, mz, ti, act, js, 0, lim, wd2, lane, edge, last, hist, sh);
+                    rdf_warp_tile<FMA, false, SHARED>(a, mx, my, mz, ti, act, js, 0, lim, wd2, lane, edge, last, hist);
                 else
-                    rdf_warp_tile<FMA, true>(a, mx, my, mz, ti, act, js, 0, lim, wd2, lane, edge, last, hist, sh);
+                    rdf_warp_tile<FMA, true, SHARED>(a, mx, my, mz, ti, act, js, 0, lim, wd2, lane, edge, last, hist);
             }
         }
     }
-    if (sh) rdf_flush(a, hist, total);
+    if (SHARED) rdf_flush(a, hist, total);
 }
 
 // cell binning for the cell search: a counting sort of the positions;
@@ -885,17 +889,18 @@ static int rdf_device(gdb_sim *h, cudaStream_t st, const float4 *pos, int n, con
     const bool fma = !(fm && fm[0] == '0');
     const size_t total = (size_t)nt * nt * bins;
     ACK(timing_begin(h, st));
-    unsigned long long *dout = nullptr;
-    ACK(pool_alloc(&dout, total * sizeof(unsigned long long), st));
+    unsigned long long *dout = nullptr;  // the counts, then the bins' edges
+    ACK(pool_alloc((unsigned char **)&dout,
+                   total * sizeof(unsigned long long) + ((size_t)bins + 1) * sizeof(float), st));
     ACK(cudaMemsetAsync(dout, 0, total * sizeof(unsigned long long), st));
     a.out = dout;
-    float *dedge = nullptr;
-    ACK(pool_alloc(&dedge, ((size_t)bins + 1) * sizeof(float), st));
+    float *dedge = (float *)(dout + total);
     a.edge = dedge;
-    k_rdf_edges<<<bins / 128 + 1, 128, 0, st>>>(a, dedge);
     // histograms and bin edges in shared memory
-    const size_t hist_bytes =
-        total <= (size_t)RDF_SMEM_MAX_BINS ? total * sizeof(unsigned) + ((size_t)bins + 1) * sizeof(float) : 0;
+    const bool shared = total <= (size_t)RDF_SMEM_MAX_BINS;
+    const size_t hist_bytes = shared ? total * sizeof(unsigned) + ((size_t)bins + 1) * sizeof(float) : 0;
+    const int first = shared ? 0 : bins;
+    k_rdf_edges<<<(bins - first) / 128 + 1, 128, 0, st>>>(a, dedge, first);
     int nc[3];
     bool cells = true;
     for (int k = 0; k < 3; k++) {
@@ -920,7 +925,8 @@ static int rdf_device(gdb_sim *h, cudaStream_t st, const float4 *pos, int n, con
         int dev = 0, sms = 0, per_sm = 0;
         ACK(cudaGetDevice(&dev));
         ACK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-        auto kern = fma ? k_rdf_allpairs<true> : k_rdf_allpairs<false>;
+        auto kern = shared ? (fma ? k_rdf_allpairs<true, true> : k_rdf_allpairs<false, true>)
+                           : (fma ? k_rdf_allpairs<true, false> : k_rdf_allpairs<false, false>);
         ACK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)(smem - hist_bytes) + RDF_HIST_MAX));
         ACK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, RDF_THREADS, smem));
@@ -947,7 +953,8 @@ static int rdf_device(gdb_sim *h, cudaStream_t st, const float4 *pos, int n, con
         int dev = 0, sms = 0, per_sm = 0;
         ACK(cudaGetDevice(&dev));
         ACK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-        auto kern = fma ? k_rdf_cells<true> : k_rdf_cells<false>;
+        auto kern = shared ? (fma ? k_rdf_cells<true, true> : k_rdf_cells<false, true>)
+                           : (fma ? k_rdf_cells<true, false> : k_rdf_cells<false, false>);
         ACK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)(smem - hist_bytes) + RDF_HIST_MAX));
         ACK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, RDF_THREADS, smem));
@@ -964,7 +971,6 @@ static int rdf_device(gdb_sim *h, cudaStream_t st, const float4 *pos, int n, con
     ACK(timing_end(h, st));
     ACK(cudaMemcpyAsync(tmp.data(), dout, total * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
     ACK(cudaFreeAsync(dout, st));
-    ACK(cudaFreeAsync(dedge, st));
     ACK(cudaStreamSynchronize(st));
     timing_store(h);
     for (size_t k = 0; k < total; k++) out_host[k] += tmp[k];
