@@ -155,7 +155,7 @@ __global__ void k_rdf_edges(RdfArgs a, float *edge, int first) {
 // (SH: at most RDF_SMEM_MAX_BINS bins) one count of the unordered pair in
 // (t_i, t_j), rdf_flush gives every pair both orders; in histograms in global
 // memory both orders at once, one addition where they are the same entry (what
-// bounds those is the additions: N 100 000, 40 000 bins, all pairs, 24 ms, 59 with two additions for every pair and the
+// bounds those is the additions: N 100 000, 40 000 bins, all pairs, 23.6 ms, 58.6 with two additions for every pair and the
 // bins searched among the edges).
 // SH: a guess of the bin from the approximate root, corrected against the
 // edges.  The guess d / width (1 - 2e-6) is below d / width by more than its rounding
@@ -232,7 +232,7 @@ struct RdfStage {
 // mask; bits q <= lim are dropped (j at or before i in the same row or tile).
 // Second pass: every lane counts its own hits, one per round.  SHARED: the
 // histograms are in shared memory (a kernel each way: with both in one, the
-// other's registers cost a fifth of the time, 1667 us against 1394 below).
+// loops are scheduled worse: LJ below 1.39 to 1.67 ms against 1.23).
 template <bool FMA, bool MIC, bool SHARED, int N>
 __device__ __forceinline__ void rdf_warp_tile(const RdfArgs &a, f32x2 mx, f32x2 my, f32x2 mz, int ti, bool act,
                                               const RdfStage<N> &st, int q0, int lim, float *d2s, int lane,
@@ -383,7 +383,7 @@ __device__ __forceinline__ int rdf_cell(float r, float L, int nc) {
 // What bounds it is instruction issue (69 % of the slots), then the shared
 // memory that the two passes go through (59 % of its rate).  Measured on B200, LJ, 1 000 188
 // particles, r_max 5, 1000 bins: a call 3.80 ms with a warp per cell and hits
-// compacted into a ring for a float64 bin, 1.41 ms here.
+// compacted into a ring for a float64 bin, 1.23 ms here.
 template <bool FMA, bool SHARED>
 __global__ void __launch_bounds__(RDF_THREADS) k_rdf_cells(RdfArgs a, const float4 *spos, const int *start,
                                                            const int *outside, int ncx, int ncy, int ncz) {
@@ -738,7 +738,7 @@ __global__ void __launch_bounds__(SQ_RUN_THREADS, 1) k_sq_runs(SqRunArgs a) {
     // sums, from the positions loaded a tile before
     for (int t = 0; t < tiles; t++) {
         if (loader) fetch(t + 2, p, w);
-        tabulate(t + 1);
+        if (t + 1 < tiles) tabulate(t + 1);
         const int np = min(SQ_TILE, p_end - p_begin - t * SQ_TILE);
         const float2 *tab = rtab + (t & 1) * SQ_TILE * row;
         // sums of x_re (z_re, z_im) and x_im (z_re, z_im), x = e_a e_b
