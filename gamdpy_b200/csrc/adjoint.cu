@@ -54,6 +54,8 @@
 #include "../../include/gamdb200.h"
 #include "gdb_internal.cuh"
 
+using namespace gdb;
+
 namespace {
 
 constexpr int ADJ_MAXT = 4;     // particle types
@@ -61,7 +63,7 @@ constexpr int ADJ_MAXB = 128;   // RDF bins
 constexpr int ADJ_LANES = 32;   // lanes per particle: a warp
 // Most warps per block (72 registers a thread): one block per SM, 4144 particles
 // in flight on 148 SMs.  One more takes a second turn every step (50 steps,
-// observables and gradient: N 4144 2.22 ms, 4145 2.61, 4200 2.99, 8288 3.84).
+// observables and gradient: N 4144 1.90 ms, 4145 2.11, 4200 2.51, 8288 3.01).
 constexpr int ADJ_WARPS = 28;
 constexpr size_t ADJ_KEEP_BYTES = (size_t)1 << 30;  // states kept instead of checkpoints up to this (GDB_ADJ_KEEP_BYTES)
 constexpr int ADJ_NTH = 2 * ADJ_MAXT * ADJ_MAXT;  // d/dsigma, d/depsilon per ordered type pair
@@ -114,6 +116,7 @@ struct AdjArgs {
     int *nbl, *nbc;
     int maxnb;
     float far2;     // (RDF reach + skin)^2, 0 without RDF bins
+    float any2;     // the largest of the reaches + skin, squared
     float move2;    // (skin / 2 - margin)^2
     float4 *rref;   // positions at the last build
     AdjBar *bar;
@@ -181,28 +184,49 @@ __device__ __forceinline__ bool adj_barrier(const AdjArgs &a, unsigned seq, bool
 __device__ __forceinline__ int type_of(float4 p) { return __float_as_int(p.w); }
 
 // The warp's list of particle i at positions pos (AdjArgs::nbl); lane L tests
-// j = L, L + 32, ... and writes its own column, which only it reads.
+// j = L, L + 32, ... and writes its own column, which only it reads.  Four
+// candidates' loads in flight, the minimum image without the rounding
+// instruction (an eighth of an add's rate), and one compare for the candidates
+// beyond every reach; the type pair's cutoff only for the others.  With a
+// rintf a component and a look at the cutoffs for every candidate the forward
+// of N 60 000 took 37.0 ms for 40 steps (20.8 with builds as kernels of their
+// own) and takes 17.3; N 4096 0.62 and 0.52.
 __device__ __forceinline__ void build_list(const AdjArgs &a, const Tab64 *tab, int nt, const float4 *pos, int i,
                                            float4 pi, int lane) {
-    const float iLx = 1.0f / a.Lx, iLy = 1.0f / a.Ly, iLz = 1.0f / a.Lz;
-    const int rows = a.maxnb / ADJ_LANES, ti = type_of(pi);
+    constexpr float RINT = 12582912.0f;  // 1.5 2^23: rint by adding and subtracting it
+    const f32x2 mxy = pack2(-pi.x, -pi.y), ilxy = pack2(1.0f / a.Lx, 1.0f / a.Ly), nlxy = pack2(-a.Lx, -a.Ly);
+    const float ilz = 1.0f / a.Lz;
+    const int n = a.n, rows = a.maxnb / ADJ_LANES, ti = type_of(pi);
+    const float any2 = a.any2, far2 = ti == 0 ? a.far2 : 0.f;
     int *col = a.nbl + (size_t)i * a.maxnb + lane;
     int near = 0, far = 0;
-#pragma unroll 4
-    for (int j = lane; j < a.n; j += ADJ_LANES) {
-        const float4 pj = pos[j];
-        const float dx = mic_rint(pj.x - pi.x, a.Lx, iLx);
-        const float dy = mic_rint(pj.y - pi.y, a.Ly, iLy);
-        const float dz = mic_rint(pj.z - pi.z, a.Lz, iLz);
-        const float d2 = dx * dx + dy * dy + dz * dz;
-        const int tj = type_of(pj);
-        if (j == i) continue;
-        if (d2 < tab[ti * nt + tj].reach2) {
-            if (near + far < rows) col[near * ADJ_LANES] = j;
-            near++;
-        } else if (d2 < a.far2 && ti == 0 && tj == 0) {
-            if (near + far < rows) col[(rows - 1 - far) * ADJ_LANES] = j;
-            far++;
+    for (int j0 = lane; j0 < n; j0 += 4 * ADJ_LANES) {
+        float4 p[4];
+#pragma unroll
+        for (int q = 0; q < 4; q++) p[q] = pos[min(j0 + q * ADJ_LANES, n - 1)];
+        float d2[4];
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            f32x2 dxy = add2(pack2(p[q].x, p[q].y), mxy);
+            float dz = p[q].z - pi.z;
+            dxy = fma2(add2(fma2(dxy, ilxy, pack2(RINT, RINT)), pack2(-RINT, -RINT)), nlxy, dxy);
+            dz = __fmaf_rn(__fsub_rn(__fmaf_rn(dz, ilz, RINT), RINT), -a.Lz, dz);
+            float dx, dy;
+            unpack2(dxy, dx, dy);
+            d2[q] = dx * dx + dy * dy + dz * dz;
+        }
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            const int j = j0 + q * ADJ_LANES;
+            if (!(d2[q] < any2) || j >= n || j == i) continue;
+            const int tj = type_of(p[q]);
+            if (d2[q] < tab[ti * nt + tj].reach2) {
+                if (near + far < rows) col[near * ADJ_LANES] = j;
+                near++;
+            } else if (tj == 0 && d2[q] < far2) {
+                if (near + far < rows) col[(rows - 1 - far) * ADJ_LANES] = j;
+                far++;
+            }
         }
     }
     if (near + far > rows) {
@@ -269,8 +293,8 @@ struct States {
 //
 // A step is a serial chain: list chunk, position gathers, warp sums, the new
 // position, the grid barrier.  Measured on B200, KA N 4096, 50 steps with 40
-// RDF bins sampled every 10: 1.0 ms, and observables and gradient together
-// 2.23 ms, against 7.35 ms with eight launches a step (gated N^2 rebuild
+// RDF bins sampled every 10: 0.8 ms, and observables and gradient together
+// 1.96 ms, against 7.35 ms with eight launches a step (gated N^2 rebuild
 // kernels, segments recomputed from checkpoints).
 struct ForwardArgs {
     States st;
@@ -460,7 +484,7 @@ struct SweepArgs {
 // the float64 derivatives run with every lane busy (a column holds about 1.5
 // pairs beyond the cutoff for each inside it, and the columns' lengths differ).
 // A warp's ring takes a round's hits beside 31 pending ones.  Measured on
-// B200, KA N 4096, 50 steps: the sweep takes 1.19 ms.
+// B200, KA N 4096, 50 steps: the sweep takes 1.0 ms.
 constexpr int ADJ_RING = 64;
 constexpr size_t ADJ_RING_BYTES = ADJ_RING * sizeof(float4);  // displacement r_j - r_i, and j << 2 | t_j
 
@@ -813,6 +837,7 @@ AdjArgs adj_args(const gdb_adj *h) {
     a.step_ratio = exp(-ratio * ratio);
     const float far = (float)((double)h->r_hi + ADJ_KW * h->width) + ADJ_SKIN;
     a.far2 = h->nbins > 0 ? far * far : 0.f;
+    a.any2 = h->rl * h->rl;
     const float mv = 0.5f * ADJ_SKIN - 0.01f;
     a.move2 = mv * mv;
     a.rref = h->d_rref;
