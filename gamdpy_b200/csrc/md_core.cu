@@ -671,7 +671,8 @@ static int enqueue_step(gdb_sim *h, int mode) {
 // balance better than even shares taken in turn (N 1 048 576: the force phase
 // 242 us against 320).  Particles whose 32 lanes do not fill GDB_BLOCK threads
 // per SM take fewer blocks instead, full ones: the barrier is shorter (LJ NVE
-// N 500, 63 blocks of 8 particles 7.20, 125 of 4 with 16 lanes 7.71).
+// N 500, 63 blocks of 8 particles 7.20, 125 of 4 with 16 lanes 7.71; with one
+// lane, if that is asked for, even shares are better: KA N 1000 22.1 and 26.7).
 struct RunShape {
     int grid, block, per_round;
 };
@@ -681,7 +682,7 @@ static int run_shape(gdb_sim *h, const void *fn, const SimArgs &a, RunShape *s, 
     const int tp = h->tp;
     const int even = (h->n + h->num_sms - 1) / h->num_sms;
     const bool spread = h->grid_cap == 0 && (long long)even * tp <= RUN_THREADS;
-    s->per_round = spread && even * 32 > GDB_BLOCK ? even : GDB_BLOCK / tp;
+    s->per_round = spread && (even * 32 > GDB_BLOCK || tp < 16) ? even : GDB_BLOCK / tp;
     // (the list build's scan wants GDB_BLOCK threads, and its walk uses them)
     s->block = spread ? std::max(GDB_BLOCK, (even * tp + 31) / 32 * 32) : GDB_BLOCK;
     *dsmem = a.nsq_smem ? (size_t)h->n * sizeof(float4)
